@@ -123,60 +123,43 @@ KR_HD void interface_tangents(double p, int iface, const LayerP& up, const Layer
   }
 }
 
-// Reverse of kennett_step, differentiating its symmetric adjugate form.  States and their
-// adjoints are symmetric: the adjoint of an off-diagonal entry is that of the one value both
-// positions share (ob.b; ob.c is not read and rbar.c is 0).  Inputs: the step's input state
-// r, the phase factors, the interface, and ob = dR/d(step output).  Outputs:
-// rbar = dR/d(step input), dR/dea, dR/deb and the 10 coefficient adjoints cbar (same order
-// as ScatTan).  Forward, with P = ea^2, Q = eb^2, S = ea eb:
-//   m = (P r11, S r12, Q r22),  dm = m11 m22 - m12^2,  dru = ru11 ru22 - ru12^2,
-//   D = 1 - ru11 m11 - 2 ru12 m12 - ru22 m22 + dru dm,
-//   A = (m11 - ru22 dm, m12 + ru12 dm, m22 - ru11 dm),  X = A / D,
-//   out = Rd + Td^T X Td = Rd + q(Td) . X.
-KR_HD void kennett_step_reverse(const M2& r, cd ea, cd eb, const Iface& f, const M2& ob,
-                                M2& rbar, cd& eabar, cd& ebbar, cd cbar[10]) {
-  // forward quantities, formed exactly as in kennett_step
-  const cd P = ea * ea, Q = eb * eb, S = ea * eb;
-  const cd m11 = P * r.a, m12 = S * r.b, m22 = Q * r.d;
-  const cd dm = cdot2(m11, m22, -m12, m12);
-  const cd one = mk(1.0, 0.0);
-  const cd idet = recip(cmac(cmac(cmac(cmac(one, -f.ru11, m11), -f.ru12x2, m12), -f.ru22, m22),
-                             f.dru, dm));
-  const cd a11 = cmac(m11, -f.ru22, dm), a12 = cmac(m12, f.ru12, dm),
-           a22 = cmac(m22, -f.ru11, dm);
-  const cd x11 = a11 * idet, x12 = a12 * idet, x22 = a22 * idet;
-  const cd o11 = ob.a, o12 = ob.b, o22 = ob.d;
-  // out = Rd + q . X: adjoints of X, and of Td through the quadratic forms (W = X Td)
-  const cd xb11 = cmac(cmac(f.q[0] * o11, f.q[3], o12), f.q[6], o22);
-  const cd xb12 = cmac(cmac(f.q[1] * o11, f.q[4], o12), f.q[7], o22);
-  const cd xb22 = cmac(cmac(f.q[2] * o11, f.q[5], o12), f.q[8], o22);
-  const cd w1 = cdot2(f.td11, x11, f.td21, x12), w2 = cdot2(f.td11, x12, f.td21, x22);
-  const cd w3 = cdot2(f.td12, x11, f.td22, x12), w4 = cdot2(f.td12, x12, f.td22, x22);
-  const cd o11x2 = 2.0 * o11, o22x2 = 2.0 * o22;
-  cbar[0] = o11;
-  cbar[1] = o12;
-  cbar[2] = o22;
-  cbar[6] = cdot2(o11x2, w1, o12, w3);  // td11
-  cbar[7] = cdot2(o12, w1, o22x2, w3);  // td12
-  cbar[8] = cdot2(o11x2, w2, o12, w4);  // td21
-  cbar[9] = cdot2(o12, w2, o22x2, w4);  // td22
-  // X = A / D
-  const cd ab11 = xb11 * idet, ab12 = xb12 * idet, ab22 = xb22 * idet;
-  const cd Db = -(cmac(cdot2(xb11, a11, xb12, a12), xb22, a22) * (idet * idet));
-  // A and D from m, dm and Ru
-  const cd dmb = cmac(cmac(cmac(f.dru * Db, -f.ru22, ab11), f.ru12, ab12), -f.ru11, ab22);
-  const cd mb11 = cmac(cmac(ab11, -f.ru11, Db), m22, dmb);
-  const cd mb22 = cmac(cmac(ab22, -f.ru22, Db), m11, dmb);
-  const cd mb12 = cmac(cmac(ab12, -f.ru12x2, Db), -2.0 * m12, dmb);
-  const cd dDb = Db * dm;  // adjoint of dru
-  cbar[3] = cmac(cmac(-(m11 * Db), f.ru22, dDb), -ab22, dm);                 // ru11
-  cbar[4] = cmac(cmac(-2.0 * (m12 * Db), -f.ru12x2, dDb), ab12, dm);         // ru12
-  cbar[5] = cmac(cmac(-(m22 * Db), f.ru11, dDb), -ab11, dm);                 // ru22
-  // m = (P r11, S r12, Q r22)
-  rbar = m2(mb11 * P, mb12 * S, mk(0.0, 0.0), mb22 * Q);
-  const cd Sb = r.b * mb12;
-  eabar = cmac(eb * Sb, 2.0 * ea, r.a * mb11);
-  ebbar = cmac(ea * Sb, 2.0 * eb, r.d * mb22);
+// The reverse sweep along a ray.  R reads one entry of the topmost state, so the adjoint of
+// every state has rank one: with a scalar seed, the adjoint of state i (a symmetric 2x2
+// matrix, its off-diagonal shared by both positions) is g g^T for a complex 2-vector g, and
+// the sweep carries g alone.  For the step out = Rd + Td^T X Td, X = M (I - Ru M)^-1,
+// M = E r E, with
+//     y = Td g,   x = X y,   z = y + Ru x  (= (I - Ru M)^-1 y, since M z = x),   g' = E z
+// the first variation of g^T out g is
+//     g^T dRd g + 2 x^T dTd g + x^T dRu x + 2 sum_a z_a x_a dlog(e_a) + g'^T dr g',
+// so g' is the next step's vector, every coefficient adjoint is a product of two components
+// of (g, x), and the phases' are 2 z_a x_a (times omega: the phases are exp(omega c)).  X is
+// all the step must keep from the forward sweep: 64 FP64 operations per step for (g, x, z, g')
+// where differentiating the step's arithmetic entry by entry took ~300.
+struct Ray {
+  cd a, b;
+};
+
+KR_HD void ray_step(const S3& X, const IfaceT<cd>& f, const Ray& g, Ray& x, Ray& z) {
+  const cd y1 = cdot2(f.td11, g.a, f.td12, g.b), y2 = cdot2(f.td21, g.a, f.td22, g.b);
+  x.a = cdot2(X.a, y1, X.b, y2);
+  x.b = cdot2(X.b, y1, X.d, y2);
+  z.a = cmac(cmac(y1, f.ru11, x.a), f.ru12, x.b);
+  z.b = cmac(cmac(y2, f.ru12, x.a), f.ru22, x.b);
+}
+
+// The 10 coefficient adjoints of a step (order of ScatTan) from its (g, x).
+KR_HD void ray_adjoints(const Ray& g, const Ray& x, cd cbar[10]) {
+  const Ray g2 = {2.0 * g.a, 2.0 * g.b};
+  cbar[0] = g.a * g.a;
+  cbar[1] = g2.a * g.b;
+  cbar[2] = g.b * g.b;
+  cbar[3] = x.a * x.a;
+  cbar[4] = (2.0 * x.a) * x.b;
+  cbar[5] = x.b * x.b;
+  cbar[6] = x.a * g2.a;  // td11
+  cbar[7] = x.a * g2.b;  // td12
+  cbar[8] = x.b * g2.a;  // td21
+  cbar[9] = x.b * g2.b;  // td22
 }
 
 // Bytes of one slowness's derivative data in shared memory (layer terms, layer derivative
@@ -226,9 +209,9 @@ KR_HD void contract(const ScatTan& t, const cd cbar[10], AccT& up, AccT& lo) {
   lo.r = lo.r + s[5];
 }
 
-// Tape of one (omega, p) pair, in local memory: up to kSegMax steps of inputs (the three
-// entries of the symmetric state) and phase factors (80 B per step; 48 B where the phases
-// come from a table) plus kCpMax checkpoints.  64 steps hold every model of up to 66 layers
+// Tape of one (omega, p) pair, in local memory: up to kSegMax steps of X (the three entries of
+// the step's symmetric matrix, ray_step) and phase factors (80 B per step; 48 B where the
+// phases come from a table) plus kCpMax checkpoints of the state.  64 steps hold every model of up to 66 layers
 // outright, so those run without any recomputation; measured on an uneven batch of 3-64-layer
 // models with the per-step contraction, the larger per-thread stack (~7 KB) cost far less
 // than recomputing segments did (24 steps: 1080 ms, 40: 1049 ms, 64: 963 ms per batch).
@@ -252,7 +235,7 @@ KR_HD int checkpoint_spacing(int nsteps) {
 // reflectivity(R) returns the seed of the reverse sweep (1 for dR/dtheta itself,
 // 2 conj(R - R_obs) for the misfit gradient) and its AccT picks complex or real
 // accumulation.  Forward sweep storing the state every `seg` steps (and recording the top
-// segment's step inputs and phases outright), then the reverse sweep top-down, every other
+// segment's X and phases outright), then the reverse sweep top-down (ray_step), every other
 // segment recomputed from its checkpoint (no recomputation at all when the steps fit one
 // segment).  sink.reflectivity(R) is called once before the reverse pass, sink.layer(l, acc)
 // once per layer l (in order 0, 1, ..., L-1) with the finished dR/d(alpha_l, beta_l, rho_l,
@@ -279,31 +262,32 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
     if (s % seg == 0) cp[s / seg] = s3(r);
     const int i = I - 2 - s;
     const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
+    S3 x;
+    r = kennett_step_keep(r, ea, eb, coef[i], x.a, x.b, x.d);
     if (s >= top0) {  // the top segment is recorded now and never recomputed
-      sg[s - top0] = s3(r);
+      sg[s - top0] = x;
       if (keep_ph) {
         sea[s - top0] = ea;
         seb[s - top0] = eb;
       }
     }
-    r = kennett_step(r, ea, eb, coef[i]);
   }
   typedef typename Sink::AccT AccT;
   const cd e0 = ph.a(0);
   const cd seed = sink.reflectivity(pp_surface(r.a, e0, free_surface));
   // top: R = E0^2 RRd_00, or y / (1 + y) with y = E0^2 RRd_00
-  cd g = mk(1.0, 0.0);
+  cd dy = mk(1.0, 0.0);
   if (free_surface) {
     cd q = recip(1.0 + (e0 * e0) * r.a);
-    g = q * q;
+    dy = q * q;
   }
-  cd ob0 = (e0 * e0) * g;
-  cd f0 = 2.0 * (e0 * r.a) * g * e0 * w;
+  cd ob0 = (e0 * e0) * dy;
+  cd f0 = 2.0 * (e0 * r.a) * dy * e0 * w;
   if (Sink::kSeeded) {
     ob0 = ob0 * seed;
     f0 = f0 * seed;
   }
-  M2 ob = m2(ob0, mk(0.0, 0.0), mk(0.0, 0.0), mk(0.0, 0.0));
+  Ray g = {csqrt(ob0), mk(0.0, 0.0)};
   AccT cur, nxt;
   acc_zero(cur);
   acc_zero(nxt);
@@ -318,24 +302,27 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
       for (int s = s0; s < s1; ++s) {
         const int i = I - 2 - s;
         const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
-        sg[s - s0] = s3(x);
+        S3 X;
+        x = kennett_step_keep(x, ea, eb, coef[i], X.a, X.b, X.d);
+        sg[s - s0] = X;
         if (keep_ph) {
           sea[s - s0] = ea;
           seb[s - s0] = eb;
         }
-        if (s + 1 < s1) x = kennett_step(x, ea, eb, coef[i]);
       }
     }
     for (int s = s1 - 1; s >= s0; --s) {
       const int i = I - 2 - s;  // interface i, lower layer i + 1
       const cd ea = keep_ph ? sea[s - s0] : ph.a(i + 1);
       const cd eb = keep_ph ? seb[s - s0] : ph.b(i + 1);
-      M2 rb;
-      cd eab, ebb, cbar[10];
-      kennett_step_reverse(m2(sg[s - s0]), ea, eb, coef[i], ob, rb, eab, ebb, cbar);
+      Ray x, z;
+      ray_step(sg[s - s0], coef[i], g, x, z);
+      cd cbar[10];
+      ray_adjoints(g, x, cbar);
       contract(tan[i], cbar, cur, nxt);
       const LayerD& d = dlay[i + 1];
-      const cd fa = eab * ea * w, fb = ebb * eb * w;
+      const cd w2 = 2.0 * w;
+      const cd fa = (z.a * x.a) * w2, fb = (z.b * x.b) * w2;
       acc_add(nxt.a, fa, d.ca_alpha);
       acc_add(nxt.b, fb, d.cb_beta);
       acc_add(nxt.h, fa, d.ca_h);
@@ -343,14 +330,15 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
       sink.layer(i, cur);
       cur = nxt;
       acc_zero(nxt);
-      ob = rb;
+      g.a = ea * z.a;
+      g.b = eb * z.b;
     }
   }
-  // bottom interface I-1 initialises RRd = Rd (ob.b: the symmetric off-diagonal's adjoint)
+  // bottom interface I-1 initialises RRd = Rd
   cd cbar[10];
-  cbar[0] = ob.a;
-  cbar[1] = ob.b;
-  cbar[2] = ob.d;
+  cbar[0] = g.a * g.a;
+  cbar[1] = (2.0 * g.a) * g.b;
+  cbar[2] = g.b * g.b;
   for (int k = 3; k < 10; ++k) cbar[k] = mk(0.0, 0.0);
   contract(tan[I - 1], cbar, cur, nxt);
   sink.layer(I - 1, cur);
@@ -379,14 +367,17 @@ constexpr int kSumVals = 12;  // per step: 10 coefficient adjoints, fa, fb
 // layer i + 1 (slots 10, 11); row I holds the top phase term of layer 0 (slot 10).
 KR_HD size_t sum_rows(int L) { return (size_t)L; }
 
-// One (omega, p) pair: forward sweep with the tape of jacobian_pair, seed, reverse sweep; per
-// step sink.step(i, cbar, fa, fb), once sink.top(f0) (the ocean phase term of layer 0).
+// One (omega, p) pair: forward sweep with the tape of jacobian_pair, seed, reverse sweep.  The
+// sink gets once top(f0) (the ocean phase term of layer 0) and per step
+// ray(i, g, x, wz): g and x of ray_step at interface i and omega z, whose products are the 12
+// adjoints (the 10 of ray_adjoints; fa = 2 wz_a x_a, fb = 2 wz_b x_b); the bottom interface
+// comes with x = wz = 0.
 #ifdef __CUDACC__
 #pragma nv_exec_check_disable
 #endif
 template <class Sink, class Ph>
-KR_HD void adjoint_pair_sums(int L, cd w, bool free_surface, int seg, const Iface* coef,
-                             const Ph& ph, Sink& sink) {
+KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* coef, const Ph& ph,
+                        Sink& sink) {
   const int I = L - 1;
   const int nsteps = I - 1;  // step s applies interface i = I - 2 - s
   const int ncp = nsteps > 0 ? (nsteps + seg - 1) / seg : 0;
@@ -402,26 +393,27 @@ KR_HD void adjoint_pair_sums(int L, cd w, bool free_surface, int seg, const Ifac
     if (s % seg == 0) cp[s / seg] = s3(r);
     const int i = I - 2 - s;
     const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
+    S3 x;
+    r = kennett_step_keep(r, ea, eb, coef[i], x.a, x.b, x.d);
     if (s >= top0) {
-      sg[s - top0] = s3(r);
+      sg[s - top0] = x;
       if (keep_ph) {
         sea[s - top0] = ea;
         seb[s - top0] = eb;
       }
     }
-    r = kennett_step(r, ea, eb, coef[i]);
   }
   const cd e0 = ph.a(0);
   const cd seed = sink.reflectivity(pp_surface(r.a, e0, free_surface));
-  cd g = mk(1.0, 0.0);
+  cd dy = mk(1.0, 0.0);
   if (free_surface) {
     cd q = recip(1.0 + (e0 * e0) * r.a);
-    g = q * q;
+    dy = q * q;
   }
-  const cd ob0 = ((e0 * e0) * g) * seed;
-  const cd f0 = (2.0 * (e0 * r.a) * g * e0 * w) * seed;
+  const cd ob0 = ((e0 * e0) * dy) * seed;
+  const cd f0 = (2.0 * (e0 * r.a) * dy * e0 * w) * seed;
   sink.top(f0);
-  M2 ob = m2(ob0, mk(0.0, 0.0), mk(0.0, 0.0), mk(0.0, 0.0));
+  Ray g = {csqrt(ob0), mk(0.0, 0.0)};
   for (int q = ncp - 1; q >= 0; --q) {
     const int s0 = q * seg;
     const int s1 = s0 + seg < nsteps ? s0 + seg : nsteps;
@@ -430,32 +422,52 @@ KR_HD void adjoint_pair_sums(int L, cd w, bool free_surface, int seg, const Ifac
       for (int s = s0; s < s1; ++s) {
         const int i = I - 2 - s;
         const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
-        sg[s - s0] = s3(x);
+        S3 X;
+        x = kennett_step_keep(x, ea, eb, coef[i], X.a, X.b, X.d);
+        sg[s - s0] = X;
         if (keep_ph) {
           sea[s - s0] = ea;
           seb[s - s0] = eb;
         }
-        if (s + 1 < s1) x = kennett_step(x, ea, eb, coef[i]);
       }
     }
     for (int s = s1 - 1; s >= s0; --s) {
       const int i = I - 2 - s;
       const cd ea = keep_ph ? sea[s - s0] : ph.a(i + 1);
       const cd eb = keep_ph ? seb[s - s0] : ph.b(i + 1);
-      M2 rb;
-      cd eab, ebb, cbar[10];
-      kennett_step_reverse(m2(sg[s - s0]), ea, eb, coef[i], ob, rb, eab, ebb, cbar);
-      sink.step(i, cbar, eab * ea * w, ebb * eb * w);
-      ob = rb;
+      Ray x, z;
+      ray_step(sg[s - s0], coef[i], g, x, z);
+      const Ray wz = {w * z.a, w * z.b};
+      sink.ray(i, g, x, wz);
+      g.a = ea * z.a;
+      g.b = eb * z.b;
     }
   }
-  // bottom interface I-1 initialises RRd = Rd (ob.b: the symmetric off-diagonal's adjoint)
-  cd cbar[10];
-  cbar[0] = ob.a;
-  cbar[1] = ob.b;
-  cbar[2] = ob.d;
-  for (int k = 3; k < 10; ++k) cbar[k] = mk(0.0, 0.0);
-  sink.step(I - 1, cbar, mk(0.0, 0.0), mk(0.0, 0.0));
+  const Ray none = {mk(0.0, 0.0), mk(0.0, 0.0)};
+  sink.ray(I - 1, g, none, none);  // bottom interface I-1 initialises RRd = Rd
+}
+
+// The same with the products formed: per step sink.step(i, cbar, fa, fb).
+template <class Sink>
+struct RayProducts {
+  Sink& sink;
+  KR_HD cd reflectivity(cd R) { return sink.reflectivity(R); }
+  KR_HD void top(cd f0) { sink.top(f0); }
+  KR_HD void ray(int i, const Ray& g, const Ray& x, const Ray& wz) {
+    cd cbar[10];
+    ray_adjoints(g, x, cbar);
+    sink.step(i, cbar, 2.0 * (wz.a * x.a), 2.0 * (wz.b * x.b));
+  }
+};
+
+#ifdef __CUDACC__
+#pragma nv_exec_check_disable
+#endif
+template <class Sink, class Ph>
+KR_HD void adjoint_pair_sums(int L, cd w, bool free_surface, int seg, const Iface* coef,
+                             const Ph& ph, Sink& sink) {
+  RayProducts<Sink> rp{sink};
+  adjoint_rays(L, w, free_surface, seg, coef, ph, rp);
 }
 
 // The contraction of the summed rows for layer l: out[0..3] = Re of the alpha, beta, rho, h

@@ -361,10 +361,9 @@ deriv_sum_kernel(int L, int n_p, const double2* __restrict__ omega, int n_w, int
   const int iw = tile * kDerThreads + threadIdx.x;
   const bool valid = iw < n_w;
   const int warp = threadIdx.x >> 5;
-  constexpr int RS = 1;  // one staging round: registers, not shared memory, bound residency
-  cd* acc = reinterpret_cast<cd*>(s_raw);
-  cd* stage = acc + (size_t)W * sum_rows(L) * kSumVals;
-  unsigned char* b = reinterpret_cast<unsigned char*>(stage + W * 32 * stage_stride<RS>());
+  double* acc = s_raw;
+  cd* stage = reinterpret_cast<cd*>(acc + (size_t)W * sum_rows(L) * kRayRow);
+  unsigned char* b = reinterpret_cast<unsigned char*>(stage + W * kRayStage);
   Iface* sc = reinterpret_cast<Iface*>(b);
   LayerP* sl = reinterpret_cast<LayerP*>(b + sizeof(Iface) * I);
   cd* s_ph = reinterpret_cast<cd*>(b + sizeof(Iface) * I + sizeof(LayerP) * L);
@@ -384,15 +383,15 @@ deriv_sum_kernel(int L, int n_p, const double2* __restrict__ omega, int n_w, int
   const PhaseAuto ph{use_tab, phase_at(s_ph, kPhHead + 1, valid ? iw : tile * kDerThreads, tile),
                      PhaseDirect{w, sl}};
   const size_t e = (size_t)ip * n_w + (valid ? iw : 0);
-  SumSink<RS> sink;
+  RaySumSink sink;
   sink.valid = valid;
   sink.vjp = vjp != 0;
   sink.obs = obs + e;
   sink.R_out = R_out ? R_out + e : nullptr;
-  sink.acc = acc + (size_t)warp * sum_rows(L) * kSumVals;
-  sink.stage = stage + warp * 32 * stage_stride<RS>();
+  sink.acc = acc + (size_t)warp * sum_rows(L) * kRayRow;
+  sink.stage = stage + warp * kRayStage;
   sink.I = I;
-  adjoint_pair_sums(L, w, free_surface != 0, seg, sc, ph, sink);
+  adjoint_rays(L, w, free_surface != 0, seg, sc, ph, sink);
   double c2 = valid ? (sink.res.x * sink.res.x + sink.res.y * sink.res.y) : 0.0;
   for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);
   if ((threadIdx.x & 31) == 0) s_chi[warp] = c2;
@@ -413,9 +412,8 @@ deriv_sum_kernel(int L, int n_p, const double2* __restrict__ omega, int n_w, int
 constexpr size_t kStageSmemMax = 160 * 1024;
 
 // Register budget of the sweep kernels: blocks of 128 threads per SM (2 -> up to 255
-// registers, 3 -> 168).  KR_DERIV_MINB or kr_set_deriv_variant; default 2.  (The
-// frequency-sum kernel fits 168 registers without spills, but three of its blocks leave too
-// little L1 for the tape: 0.154 ms vs 0.138 ms per 64 x 1024 gradient.)
+// registers, 3 -> 168).  KR_DERIV_MINB or kr_set_deriv_variant; default 2 (the frequency-sum
+// kernel needs 164 registers either way: 80.6 us per 64 x 1024 gradient at both settings).
 static int g_deriv_minb = -1;
 
 static int deriv_minb_setting() {
@@ -464,7 +462,7 @@ static kr_status launch_sweep(int minb, unsigned blocks, size_t smem, cudaStream
 
 // Dynamic smem of deriv_sum_kernel for a model of L layers (0 if it does not fit).
 static size_t sum_kernel_smem(int L, int table) {
-  const size_t smem = adjsum_smem_bytes(L, kDerThreads / 32, 1) + prologue_smem_bytes(L) +
+  const size_t smem = raysum_smem_bytes(L, kDerThreads / 32) + prologue_smem_bytes(L) +
                       (table ? phase_table_bytes(L, 1) : 0);
   return smem <= kStageSmemMax ? smem : 0;
 }

@@ -340,6 +340,18 @@ KR_HD M2 kennett_step(const M2& r, cd ea, cd eb, const Iface& f) {
   return o;
 }
 
+// kennett_step that also hands out X (entries 11, 12, 22), from which the reverse sweep of the
+// derivatives needs nothing else of the step (kr_adjoint.cuh).  Same arithmetic, same bits.
+KR_HD M2 kennett_step_keep(const M2& r, cd ea, cd eb, const Iface& f, cd& x11, cd& x12, cd& x22) {
+  step_x(r, ea, eb, f, x11, x12, x22);
+  M2 o;
+  o.a = cmac(cmac(cmac(f.rd11, f.q[0], x11), f.q[1], x12), f.q[2], x22);
+  o.b = cmac(cmac(cmac(f.rd12, f.q[3], x11), f.q[4], x12), f.q[5], x22);
+  o.d = cmac(cmac(cmac(f.rd22, f.q[6], x11), f.q[7], x12), f.q[8], x22);
+  o.c = o.b;
+  return o;
+}
+
 // The last (ocean-bottom) step, returning only RRd_00 (the same arithmetic as kennett_step's
 // first entry; that interface's Td has one column, so only q[0..2] are non-zero).
 KR_HD cd kennett_last_step_pp(const M2& r, cd ea, cd eb, const Iface& f) {
