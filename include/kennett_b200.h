@@ -65,6 +65,10 @@ int32_t kr_version(void);
  */
 kr_status kr_validate_layers(const double* layers_host, int32_t n_layers);
 
+/* kr_validate_layers of n_tables consecutive tables [n_tables][6][n_layers] (host); the status
+ * and error detail of the first invalid one. */
+kr_status kr_validate_tables(const double* tables_host, int32_t n_tables, int32_t n_layers);
+
 /*
  * Plane-wave PP reflectivity R(p, omega) for one model on a slowness x frequency grid.
  * Replaces kennett_reflectivity (Kennett_Reflectivity/kennett_reflectivity.py:73-78) and

@@ -51,6 +51,7 @@ _SIGNATURES = {
     "kr_last_error": (ctypes.c_char_p, []),
     "kr_version": (_i32, []),
     "kr_validate_layers": (_i32, [_vp, _i32]),
+    "kr_validate_tables": (_i32, [_vp, _i32, _i32]),
     "kr_reflectivity": (_i32, [_vp, _i32, _vp, _i32, _vp, _i32, _u32, _vp, _vp]),
     "kr_gmm_reflectivity": (_i32, [_vp, _i32, _vp, _i32, _vp, _i32, _u32, _vp, _vp]),
     "kr_jacobian_workspace_bytes": (_size_t, [_i32, _i32, _i32]),

@@ -198,8 +198,7 @@ class ModelBatch:
         n, six, L = tables.shape
         if six != 6:
             raise ValueError("tables must have shape [n, 6, n_layers]")
-        for b in range(n):
-            D.validate_table(tables[b])
+        D.validate_tables(tables)
         p = np.ascontiguousarray(p, dtype=np.float64).reshape(-1)
         w = np.ascontiguousarray(omega, dtype=np.complex128).reshape(-1)
         self = cls.__new__(cls)

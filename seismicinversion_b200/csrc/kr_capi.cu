@@ -67,3 +67,12 @@ extern "C" kr_status kr_validate_layers(const double* tab, int32_t n) {
   }
   return KR_OK;
 }
+
+extern "C" kr_status kr_validate_tables(const double* tabs, int32_t n_tables, int32_t n) {
+  if (n_tables < 0 || (n_tables > 0 && !tabs)) return KR_ERR_INVALID_ARGUMENT;
+  for (int32_t b = 0; b < n_tables; ++b) {
+    const kr_status s = kr_validate_layers(tabs + (size_t)b * 6 * (n > 0 ? n : 0), n);
+    if (s != KR_OK) return s;
+  }
+  return KR_OK;
+}

@@ -1,0 +1,271 @@
+// The forward sweep of one slowness over a uniform frequency grid, warp by warp, shared by the
+// per-model and the batched forward kernels (so that both give the same bits).
+//
+// What bounds it is the FP64 pipe: ~115 FP64 instructions per (omega, p, interface) in
+// kennett_step_x when the squared and mixed phase factors P = ea^2, Q = eb^2, S = ea eb come
+// from a table.  The table holds, per phase exponent c (2 i eta h, 2 i neta h, i (eta + neta) h
+// of every layer above the half-space), lo[j] = exp(j delta c), j < 16, and
+// mid[m] = exp(16 m delta c), m < 8; a warp forms hi = exp(omega_{128 u} c) of its tile u times
+// the mid entries of its own frequencies once per pass (hm), so a lookup is one complex product
+// of two shared-memory reads.  Models too deep for three phases per layer in shared memory
+// tabulate ea and eb alone (two lookups and three more products per step); models deeper still
+// evaluate exponentials directly, as do tiles that are off the grid's line (kr_phase.cuh).
+//
+// A lane sweeps F frequencies at once (the kernels use 1; 2 halves the reads of the 17
+// coefficients per step but costs more registers than it gains, kr_forward.cu).
+#pragma once
+
+#include "kr_phase.cuh"
+
+namespace kr {
+
+// Phases per layer of a tabulating model: 3 (P, Q, S) up to kPqsLayers layers, where a block of
+// four warps (56 KB at 30 layers) fits four times on an SM; 2 (ea, eb) up to kPairLayers, where
+// a block of eight warps (113 KB at 66) fits twice: 193 x 1501 of a 64-layer model takes 253 us
+// against 348 with direct exponentials; 0 beyond.  Every forward kernel applies this rule to
+// the model, so a model's phases round alike everywhere.
+constexpr int kPqsLayers = 30;
+constexpr int kPairLayers = 66;
+__host__ __device__ inline int sweep_phases(int n_layers) {
+  return n_layers <= kPqsLayers ? 3 : n_layers <= kPairLayers ? 2 : 0;
+}
+
+// Shared memory of one slowness (layer terms and roots, interface coefficients, lo / mid
+// entries) and of
+// one warp (its hm products) for NPH phases per layer and F frequencies per lane.
+__host__ __device__ inline size_t sweep_slowness_bytes(int n_layers, int nph) {
+  return prologue_smem_bytes(n_layers) + sizeof(LayerRoots) * n_layers +
+         sizeof(cd) * kPhHead * nph * (size_t)(n_layers - 1);
+}
+__host__ __device__ inline size_t sweep_warp_bytes(int n_layers, int nph, int F) {
+  return sizeof(cd) * 2 * F * nph * (size_t)(n_layers - 1);
+}
+
+// Exponent `id` (NPH l + k) of a model.
+template <int NPH>
+__device__ __forceinline__ cd sweep_exponent(const LayerP* lay, int id) {
+  const LayerP& lp = lay[id / NPH];
+  const int k = id % NPH;
+  if (NPH == 2) return k ? lp.cb : lp.ca;
+  return k == 0 ? 2.0 * lp.ca : k == 1 ? 2.0 * lp.cb : lp.ca + lp.cb;
+}
+
+__device__ __forceinline__ bool phase_usable(cd v) {
+  return fabs(v.x) <= kPhMaxMag && fabs(v.y) <= kPhMaxMag;
+}
+
+// Entry e (id kPhHead + j) of a slowness's lo / mid table; returns whether it is usable.
+template <int NPH>
+__device__ __forceinline__ bool sweep_table_entry(const GridLine& g, const LayerP* lay, int e,
+                                                  cd* tab) {
+  const int id = e / kPhHead, j = e - id * kPhHead;
+  const cd z = (double)(j < kPhLo ? j : (j - kPhLo) * kPhLo) * g.d;
+  const cd v = cexp_(z * sweep_exponent<NPH>(lay, id));
+  tab[e] = v;
+  return phase_usable(v);
+}
+
+// The prologue's two stages out of line: one compiled body per kernel file, called by every
+// kernel that must agree bit for bit, and no register pressure on the sweep around it.  Stage 1,
+// a thread per (layer, P or S): terms and square root; stage 2, a thread per interface: the
+// coefficients, a chain of complex products once the roots are there.
+static __device__ __noinline__ void layer_store(const double* tab, int L, int l, int half,
+                                                double p, LayerP* lay, LayerRoots* roots) {
+  if (half == 0) {
+    layer_terms_p(tab, L, l, p, *lay);
+    roots->eta = csqrt(lay->eta);
+  } else {
+    layer_terms_s(tab, L, l, p, *lay);
+    roots->neta = csqrt(lay->neta);
+  }
+}
+static __device__ __noinline__ void interface_store(double p, int i, const LayerP* lay,
+                                                    const LayerRoots* roots, Iface* out) {
+  *out = interface_coeffs(p, i, lay[i], lay[i + 1], roots[i], roots[i + 1]);
+}
+
+// Phase factors of F frequencies of one lane from the table.
+template <int NPH, int F>
+struct SweepTable {
+  const cd* lo;  // the lane's lo entry of phase 0
+  const cd* hm;  // the lane's first hm product of phase 0 (frequency f: + 2 f)
+  __device__ __forceinline__ void pqs(int l, cd P[F], cd Q[F], cd S[F]) const {
+    const cd* a = lo + (size_t)(NPH * l) * kPhHead;
+    const cd* b = hm + (size_t)(NPH * l) * 2 * F;
+    const cd l0 = a[0], l1 = a[kPhHead];
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      const cd u = b[2 * f] * l0, v = b[2 * F + 2 * f] * l1;
+      if (NPH == 3) {
+        P[f] = u;
+        Q[f] = v;
+        S[f] = b[4 * F + 2 * f] * a[2 * kPhHead];
+      } else {
+        P[f] = u * u;
+        Q[f] = v * v;
+        S[f] = u * v;
+      }
+    }
+  }
+  __device__ __forceinline__ void ocean(cd E[F]) const {  // e0^2
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      const cd u = hm[2 * f] * lo[0];
+      E[f] = NPH == 3 ? u : u * u;
+    }
+  }
+};
+
+// Direct exponentials of one frequency.
+struct SweepDirect {
+  cd w;
+  const LayerP* lay;
+  __device__ __forceinline__ void pqs(int l, cd P[1], cd Q[1], cd S[1]) const {
+    const cd a = cexp_(w * lay[l].ca), b = cexp_(w * lay[l].cb);
+    P[0] = a * a;
+    Q[0] = b * b;
+    S[0] = a * b;
+  }
+  __device__ __forceinline__ void ocean(cd E[1]) const {
+    const cd a = cexp_(w * lay[0].ca);
+    E[0] = a * a;
+  }
+};
+
+// The upward sweep of F frequencies: R at the surface.
+template <int F, class Ph>
+__device__ __forceinline__ void sweep_frequencies(int n_layers, const Iface* coef, const Ph& ph,
+                                                  bool fs, cd R[F]) {
+  const int I = n_layers - 1;
+  M2 r[F];
+#pragma unroll
+  for (int f = 0; f < F; ++f) {
+    r[f].a = coef[I - 1].rd11;
+    r[f].b = coef[I - 1].rd12;
+    r[f].d = coef[I - 1].rd22;
+  }
+  cd P[F], Q[F], S[F], rpp[F], E[F];
+#pragma unroll 1
+  for (int i = I - 2; i >= 1; --i) {
+    ph.pqs(i + 1, P, Q, S);
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      cd x11, x12, x22;
+      r[f] = kennett_step_x(r[f], P[f], Q[f], S[f], coef[i], x11, x12, x22);
+    }
+  }
+  if (I > 1) ph.pqs(1, P, Q, S);
+  ph.ocean(E);
+#pragma unroll
+  for (int f = 0; f < F; ++f) {
+    rpp[f] = I > 1 ? kennett_last_step_pp(r[f], P[f], Q[f], S[f], coef[0]) : r[f].a;
+    R[f] = pp_surface2(rpp[f], E[f], fs);
+  }
+}
+
+// The two kinds of sweep out of line, so that the hot loop's registers are its own: inlined
+// next to the exponentials and the task bookkeeping it spilled inside the loop.
+template <int F>
+struct SweepOut {
+  cd R[F];
+};
+template <int NPH, int F>
+__device__ __noinline__ SweepOut<F> sweep_table(int n_layers, const Iface* coef, const cd* lo,
+                                                const cd* hm, bool fs) {
+  SweepOut<F> o;
+  sweep_frequencies<F>(n_layers, coef, SweepTable<NPH, F>{lo, hm}, fs, o.R);
+  return o;
+}
+static __device__ __noinline__ cd sweep_direct(int n_layers, const Iface* coef, const LayerP* lay,
+                                               cd w, bool fs) {
+  cd R[1];
+  sweep_frequencies<1>(n_layers, coef, SweepDirect{w, lay}, fs, R);
+  return R[0];
+}
+
+// Tiles whose start and verdict a block keeps in shared memory at once.
+constexpr int kSweepTiles = 66;
+struct SweepTiles {
+  double2 w0[kSweepTiles];        // the tile's first frequency
+  unsigned char off[kSweepTiles]; // 1: the tile leaves the grid's line
+};
+
+// Block-cooperative: starts and verdicts of tiles [u0, u0 + n).  The caller synchronises before
+// (off[] cleared by sweep_tiles_clear) and after.
+__device__ __forceinline__ void sweep_tiles_clear(SweepTiles& t, int n) {
+  for (int e = threadIdx.x; e < n; e += blockDim.x) t.off[e] = 0;
+}
+__device__ __forceinline__ void sweep_tiles_check(const double2* __restrict__ omega, int n_w,
+                                                  const GridLine& g, int u0, int n,
+                                                  SweepTiles& t) {
+  const int k_end = min(n_w, (u0 + n) * kPhTile);
+  for (int k = u0 * kPhTile + threadIdx.x; k < k_end; k += blockDim.x) {
+    const double2 w = omega[k];
+    const double m = (double)k;
+    if (k % kPhTile == 0) t.w0[k / kPhTile - u0] = w;
+    if (!(fabs(w.x - fma(m, g.d.x, g.w0.x)) <= g.tol && fabs(w.y - fma(m, g.d.y, g.w0.y)) <= g.tol))
+      t.off[k / kPhTile - u0] = 1;
+  }
+}
+
+// One warp: passes [pass0, pass1) of tile u (pass q: the 32 F consecutive frequencies from
+// 128 u + 32 F q), frequencies outside [k_lo, k_hi) skipped.  `w0`: the tile's first frequency;
+// `use`: whether the tile and the slowness's lo / mid entries `tab` may be used (NPH > 0); hm:
+// the warp's scratch.  The tile's hi entries are evaluated once and stay in registers.
+template <int NPH, int F>
+__device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, double2 w0, int u,
+                                           int pass0, int pass1, int k_lo, int k_hi, int n_layers,
+                                           const LayerP* lay, const Iface* coef, const cd* tab,
+                                           bool use, cd* hm, bool fs, double2* __restrict__ Rp) {
+  const int lane = threadIdx.x & 31;
+  constexpr int N = NPH > 0 ? NPH : 1;
+  constexpr int kHi = NPH == 3 ? (3 * (kPqsLayers - 1) + 31) / 32 : (2 * (kPairLayers - 1) + 31) / 32;
+  const int n_phase = N * (n_layers - 1);
+  cd hi[kHi];
+  if (NPH > 0 && use) {
+    bool bad = false;
+#pragma unroll
+    for (int r = 0; r < kHi; ++r) {
+      const int id = 32 * r + lane;
+      if (id < n_phase) {
+        hi[r] = cexp_(mk(w0.x, w0.y) * sweep_exponent<N>(lay, id));
+        bad |= !phase_usable(hi[r]);
+      }
+    }
+    use = !__any_sync(0xffffffffu, bad);
+  }
+  for (int pass = pass0; pass < pass1; ++pass) {
+    const int kb = u * kPhTile + pass * 32 * F;
+    if (kb >= k_hi || kb + 32 * F <= k_lo) continue;
+    if (NPH > 0 && use) {
+#pragma unroll
+      for (int r = 0; r < kHi; ++r) {
+        const int id = 32 * r + lane;
+        if (id < n_phase) {
+          const cd* mid = tab + id * kPhHead + kPhLo + pass * 2 * F;
+#pragma unroll
+          for (int m = 0; m < 2 * F; ++m) hm[id * 2 * F + m] = hi[r] * mid[m];
+        }
+      }
+      __syncwarp();
+      const SweepOut<F> o = sweep_table<N, F>(n_layers, coef, tab + (lane & (kPhLo - 1)),
+                                              hm + (lane >> 4), fs);
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const int k = kb + 32 * f + lane;
+        if (k >= k_lo && k < k_hi) Rp[k] = make_double2(o.R[f].x, o.R[f].y);
+      }
+      __syncwarp();  // hm is read before the next pass overwrites it
+      continue;
+    }
+    for (int f = 0; f < F; ++f) {
+      const int k = kb + 32 * f + lane;
+      if (k < k_lo || k >= k_hi) continue;
+      const double2 wv = omega[k];
+      const cd R = sweep_direct(n_layers, coef, lay, mk(wv.x, wv.y), fs);
+      Rp[k] = make_double2(R.x, R.y);
+    }
+  }
+}
+
+}  // namespace kr

@@ -56,6 +56,13 @@ def validate_table(tab: np.ndarray) -> None:
     _lib.check(_lib.lib().kr_validate_layers(tab.ctypes.data, tab.shape[1]), "layer model")
 
 
+def validate_tables(tabs: np.ndarray) -> None:
+    """``validate_table`` of every table of a C-contiguous float64 [n, 6, n_layers] array, in one
+    call (the first invalid table's error)."""
+    _lib.check(_lib.lib().kr_validate_tables(tabs.ctypes.data, tabs.shape[0], tabs.shape[2]),
+               "layer model")
+
+
 def layer_table(model: LayerModel, device=None) -> torch.Tensor:
     """Validated float64 ``[6, n_layers]`` layer table on the device."""
     dev = require_cuda(device)
