@@ -220,7 +220,11 @@ class ModelBatch:
         self.graph = None
         self.schedule = None
         self.plan = None
-        self.set_schedule(schedule or (128, 128))
+        # short grids leave a wide block's warps without frequencies: 12 x 64 of 4096 5-layer
+        # models take 361 us with one warp per item, 401 with two and 530 with four; of 1500
+        # 12-layer models (12 x 50) 395, 321 and 392, their table being larger than their sweep
+        few = 128 if len(w) > 256 else 64 if L > 8 or len(w) > 128 else 32
+        self.set_schedule(schedule or (few, 128))
         return self
 
     # -- planning ------------------------------------------------------------------------

@@ -263,7 +263,7 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
     const int i = I - 2 - s;
     const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
     S3 x;
-    r = kennett_step_keep(r, ea, eb, coef[i], x.a, x.b, x.d);
+    r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
     if (s >= top0) {  // the top segment is recorded now and never recomputed
       sg[s - top0] = x;
       if (keep_ph) {
@@ -303,7 +303,7 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
         const int i = I - 2 - s;
         const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
         S3 X;
-        x = kennett_step_keep(x, ea, eb, coef[i], X.a, X.b, X.d);
+        x = kennett_step_x(x, ea * ea, eb * eb, ea * eb, coef[i], X.a, X.b, X.d);
         sg[s - s0] = X;
         if (keep_ph) {
           sea[s - s0] = ea;
@@ -394,7 +394,7 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
     const int i = I - 2 - s;
     const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
     S3 x;
-    r = kennett_step_keep(r, ea, eb, coef[i], x.a, x.b, x.d);
+    r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
     if (s >= top0) {
       sg[s - top0] = x;
       if (keep_ph) {
@@ -423,7 +423,7 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
         const int i = I - 2 - s;
         const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
         S3 X;
-        x = kennett_step_keep(x, ea, eb, coef[i], X.a, X.b, X.d);
+        x = kennett_step_x(x, ea * ea, eb * eb, ea * eb, coef[i], X.a, X.b, X.d);
         sg[s - s0] = X;
         if (keep_ph) {
           sea[s - s0] = ea;

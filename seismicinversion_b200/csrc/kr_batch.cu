@@ -6,17 +6,19 @@
 //   * a pair table: one entry per (model, slowness) with the offset of its coefficient block
 //     in the plan buffer;
 //   * two work lists (forward items, gradient items), item = (pair, first frequency, count),
-//     sorted by descending cost (layers x frequencies, x4 for gradients) so the dynamic
-//     scheduler hands out the longest items first (LPT);
+//     models of more than 30 layers first, each class sorted by descending cost (layers x
+//     frequencies, x4 for gradients) so the dynamic scheduler hands out the longest items
+//     first (LPT);
 // and uploads them into the caller's plan buffer.  kr_batch_launch (device only, capturable
 // in a CUDA graph) then runs:
-//   1. batch_prep_kernel: one block per pair -> layer terms and interface coefficients (and,
-//      for gradient models, layer derivative factors) into the plan;
+//   1. batch_prep_kernel: a group of threads per pair -> layer terms and interface coefficients
+//      (and, for gradient models, layer derivative factors) into the plan;
 //   2. batch_tan_kernel: the gradient models' coefficient tangents, one thread per interface
 //      and tangent column, alongside the forward kernel (its programmatic dependent);
-//   3. batch_forward_kernel and batch_grad_sums_kernel (batch_gradient_kernel where a model's
-//      frequency sums exceed shared memory): persistent grids (resident blocks only) that
-//      pull items with an atomic counter until the list is exhausted.
+//   3. batch_forward_kernel (a launch for each depth class) and batch_grad_sums_kernel
+//      (batch_gradient_kernel where a model's frequency sums exceed shared memory): persistent
+//      grids (resident blocks only) that pull items with an atomic counter until the list is
+//      exhausted.  Without observed data there are no gradient models and no launches for them.
 // Gradient items reduce their contributions per block in a fixed order and add them to the
 // model's chi_grad with FP64 atomics (the order of those additions across blocks is not
 // fixed: results agree to rounding, ~1e-16 relative, run to run).
@@ -29,7 +31,7 @@
 #include "kr_adjoint.cuh"
 #include "kr_adjsum.cuh"
 #include "kr_internal.cuh"
-#include "kr_phase.cuh"
+#include "kr_sweep.cuh"
 
 namespace kr {
 
@@ -50,7 +52,8 @@ struct PlanHeader {
   int32_t n_models, n_pairs, n_fwd, n_grad;
   int32_t threads, tile_w, grid_fwd, grid_grad;
   int64_t off_models, off_pairs, off_fwd, off_grad, total_bytes;
-  int32_t counters[4];  // [0] forward item counter, [1] gradient item counter
+  int32_t n_fwd_deep, n_grad_deep;  // the lists' leading items, of models deeper than kPqsLayers
+  int32_t counters[4];  // item counters: forward deep / shallow, gradient [2]
 };
 
 __host__ __device__ inline size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -84,32 +87,49 @@ __device__ __forceinline__ PairView pair_view(const unsigned char* plan, const P
   return v;
 }
 
-__global__ void batch_prep_kernel(unsigned char* plan, const double* __restrict__ layers,
-                                  const double* __restrict__ p_all) {
+// Layer terms, derivative factors (gradient models) and interface coefficients of every pair.
+// A group of GS threads takes a pair: GS is the power of two that covers the deepest model's
+// layers (4 to 64), so a batch of 5-layer models keeps all of a warp's lanes busy (eight
+// threads a pair) where a block a pair left 59 of 64 threads idle (49152 pairs of 5 layers:
+// 360 us).  A pair's threads meet at a warp or (GS = 64) block barrier between the layer terms
+// and the coefficients that read them back; every group of a block runs the same number of
+// rounds.
+constexpr int kPrepBlock = 64;
+
+__global__ void __launch_bounds__(kPrepBlock)
+batch_prep_kernel(unsigned char* plan, const double* __restrict__ layers,
+                  const double* __restrict__ p_all, int gs) {
+  __shared__ LayerRoots s_roots[kMaxLayers];  // kMaxLayers / groups per group, at least gs
   const PlanHeader* h = reinterpret_cast<const PlanHeader*>(plan);
   const kr_model_desc* models = reinterpret_cast<const kr_model_desc*>(plan + h->off_models);
   const PairRec* pairs = reinterpret_cast<const PairRec*>(plan + h->off_pairs);
-  for (int q = blockIdx.x; q < h->n_pairs; q += gridDim.x) {
-    const PairRec pr = pairs[q];
+  const int groups = kPrepBlock / gs, mine = threadIdx.x / gs, t0 = threadIdx.x % gs;
+  const int stride = gridDim.x * groups;
+  for (int q0 = blockIdx.x * groups; q0 < h->n_pairs; q0 += stride) {
+    const int q = q0 + mine;
+    const bool have = q < h->n_pairs;
+    const PairRec pr = pairs[have ? q : q0];
     const kr_model_desc d = models[pr.model];
-    const int L = d.n_layers, I = L - 1;
+    const int L = have ? d.n_layers : 0, I = L - 1;
     const double* tab = layers + d.layers_off;
     const double pj = p_all[d.p_off + pr.j];
     unsigned char* b = plan + pr.coef_off;
     LayerP* lay = reinterpret_cast<LayerP*>(b);
-    b += a256(sizeof(LayerP) * L);
+    b += a256(sizeof(LayerP) * d.n_layers);
     Iface* coef = reinterpret_cast<Iface*>(b);
-    b += a256(sizeof(Iface) * I);
+    b += a256(sizeof(Iface) * (d.n_layers - 1));
     LayerD* dlay = reinterpret_cast<LayerD*>(b);
     const bool grad = (d.flags & KR_BATCH_GRADIENT) != 0;
-    for (int l = threadIdx.x; l < L; l += blockDim.x) {
-      lay[l] = layer_terms(tab, L, l, pj);
-      if (grad) dlay[l] = layer_derivs(tab, L, l, pj, lay[l]);
+    LayerRoots* roots = s_roots + mine * (kMaxLayers / kPrepBlock) * gs;
+    for (int t = t0; t < 2 * L; t += gs) {
+      const int half = t >= L ? 1 : 0, l = t - half * L;
+      layer_store(tab, L, l, half, pj, lay + l, roots + l);
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < I; i += blockDim.x)
-      coef[i] = interface_coeffs(pj, i, lay[i], lay[i + 1]);
-    __syncthreads();
+    if (gs > 32) __syncthreads(); else __syncwarp();
+    for (int i = t0; i < I; i += gs) interface_store(pj, i, lay, roots, coef + i);
+    if (grad)
+      for (int l = t0; l < L; l += gs) dlay[l] = layer_derivs(tab, L, l, pj, lay[l]);
+    if (gs > 32) __syncthreads(); else __syncwarp();  // the roots are read before the next pair's
   }
 }
 
@@ -157,71 +177,109 @@ __global__ void batch_reset_kernel(unsigned char* plan, double* chi_grad) {
   }
 }
 
-__device__ __forceinline__ int next_item(int* counter) {
-  __shared__ int s_item;
+// The block's work items from a shared counter.  The next item's number is fetched while the
+// current one is processed, so the atomic's latency does not sit between short items.
+struct ItemFeed {
+  int* counter;
+  int* slot;  // one shared word
+  int ahead;  // thread 0: the number fetched ahead
+  __device__ __forceinline__ ItemFeed(int* c, int* s) : counter(c), slot(s), ahead(0) {
+    if (threadIdx.x == 0) ahead = atomicAdd(counter, 1);
+  }
+  // Contains block barriers: every thread is done with the previous item.
+  __device__ __forceinline__ int next() {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      *slot = ahead;
+      ahead = atomicAdd(counter, 1);
+    }
+    __syncthreads();
+    return *slot;
+  }
+};
+
+// Forward items: one (model, slowness) pair and a frequency range [w0, w0 + nw).  The block
+// copies the pair's layer terms and coefficients from the plan, builds its phase table and its
+// warps take the passes of the range in turn (kr_sweep.cuh: the code of kr_reflectivity, so the
+// results are bit-identical to a per-model call).  DEEP selects the class of the work list:
+// models of up to kPqsLayers layers, whose blocks are small, or deeper ones; each class is one
+// persistent launch with the shared memory and registers of its own models, so that a batch's
+// shallow models do not run at the occupancy of its deepest.
+template <int NPH, int F, int THREADS>
+__device__ __forceinline__ void forward_item(const ItemRec& item, const kr_model_desc& d, int j,
+                                             const PairView& v, const double2* om, double2* Rp,
+                                             unsigned char* smem, SweepTiles& tiles) {
+  constexpr int N = NPH > 0 ? NPH : 1;
+  const int L = d.n_layers, I = L - 1;
+  LayerP* lay = reinterpret_cast<LayerP*>(smem);
+  Iface* coef = reinterpret_cast<Iface*>(lay + L);
+  cd* tab = reinterpret_cast<cd*>(coef + I);
+  cd* hm = tab + (size_t)NPH * I * kPhHead + (size_t)(threadIdx.x >> 5) * 2 * F * NPH * I;
+  const int u0 = item.w0 / kPhTile, n_tiles = (item.w0 + item.nw - 1) / kPhTile - u0 + 1;
+  copy16(lay, v.lay, sizeof(LayerP) * L);
+  copy16(coef, v.coef, sizeof(Iface) * I);
+  if (NPH > 0) sweep_tiles_clear(tiles, n_tiles);
   __syncthreads();
-  if (threadIdx.x == 0) s_item = atomicAdd(counter, 1);
-  __syncthreads();
-  return s_item;
+  bool bad = false;
+  if (NPH > 0) {
+    const GridLine g = grid_line(om, d.n_w);
+    sweep_tiles_check(om, d.n_w, g, u0, n_tiles, tiles);
+    // an item within one tile needs only the mid entries of its own frequencies
+    const int m0 = n_tiles > 1 ? 0 : (item.w0 % kPhTile) / kPhLo;
+    const int m1 = n_tiles > 1 ? kPhMid : ((item.w0 + item.nw - 1) % kPhTile) / kPhLo + 1;
+    const int per = kPhLo + m1 - m0;
+    for (int e = threadIdx.x; e < NPH * I * per; e += THREADS) {
+      const int id = e / per, j = e - id * per;
+      bad |= !sweep_table_entry<N>(g, lay, id, j < kPhLo ? j : j + m0, tab);
+    }
+  }
+  const bool ok = __syncthreads_or(bad) == 0;
+  constexpr int kPasses = kPhTile / (32 * F);
+  // a warp takes whole tiles, or single passes of short items
+  const int passes = n_tiles >= 2 * (THREADS / 32) ? kPasses : 1, parts = kPasses / passes;
+  for (int t = threadIdx.x >> 5; t < n_tiles * parts; t += THREADS / 32) {
+    const int q = t / parts, pass = (t - q * parts) * passes;
+    sweep_tile<NPH, F>(om, NPH > 0 ? tiles.w0[q] : make_double2(0.0, 0.0), u0 + q, pass,
+                       pass + passes, item.w0, item.w0 + item.nw, L, lay, coef, tab,
+                       NPH > 0 && ok && tiles.off[q] == 0, hm, (d.flags & KR_FREE_SURFACE) != 0,
+                       Rp);
+  }
 }
 
-// Forward items: one (model, slowness) pair and a frequency range [w0, w0 + nw).  With
-// tab_entries > 0 (kPhHead + 2: lo, mid and two hi slots) models that tabulate take their
-// phase factors from a table holding one tile's hi entry at a time (kr_phase.cuh; same
-// entries and decisions as kr_reflectivity, so the results are bit-identical to a per-model
-// call): ~37 KB of shared memory for the deepest such model, six blocks per SM.
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS)
+template <int THREADS, bool DEEP>
+__global__ void __launch_bounds__(THREADS, (DEEP ? 256 : 512) / THREADS)
 batch_forward_kernel(unsigned char* plan, const double2* __restrict__ omega_all,
-                     double2* __restrict__ R_all, int tab_entries) {
-  extern __shared__ __align__(16) unsigned char s_pair[];  // layer terms + coefficients + table
+                     double2* __restrict__ R_all) {
+  // the next launch on the stream that allows it may fill in as this one's blocks finish
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ __align__(16) unsigned char s_pair[];
+  __shared__ SweepTiles s_tiles;
   PlanHeader* h = reinterpret_cast<PlanHeader*>(plan);
   const kr_model_desc* models = reinterpret_cast<const kr_model_desc*>(plan + h->off_models);
   const PairRec* pairs = reinterpret_cast<const PairRec*>(plan + h->off_pairs);
-  const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_fwd);
-  const int n_items = h->n_fwd;
+  const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_fwd) +
+                         (DEEP ? 0 : h->n_fwd_deep);
+  const int n_items = DEEP ? h->n_fwd_deep : h->n_fwd - h->n_fwd_deep;
+  __shared__ int s_item;
+  ItemFeed feed(&h->counters[DEEP ? 0 : 1], &s_item);
   for (;;) {
-    const int it = next_item(&h->counters[0]);
+    const int it = feed.next();
     if (it >= n_items) break;
     const ItemRec item = items[it];
     const PairRec pr = pairs[item.pair];
     const kr_model_desc d = models[pr.model];
     const PairView v = pair_view(plan, pr, d);
-    const bool fs = (d.flags & KR_FREE_SURFACE) != 0;
-    LayerP* lay = reinterpret_cast<LayerP*>(s_pair);
-    Iface* coef = reinterpret_cast<Iface*>(s_pair + sizeof(LayerP) * d.n_layers);
-    cd* s_ph = reinterpret_cast<cd*>(s_pair + prologue_smem_bytes(d.n_layers));
-    copy16(lay, v.lay, sizeof(LayerP) * d.n_layers);
-    copy16(coef, v.coef, sizeof(Iface) * (d.n_layers - 1));
-    __syncthreads();
     const double2* om = omega_all + d.omega_off;
-    const GridLine g = grid_line(om, d.n_w);
-    // block-uniform conditions: every thread takes the same branches through the barriers
-    const bool tab = tab_entries > 0 && phase_table_model(d.n_layers);
-    const bool lomid = tab && build_phase_lomid(g, tab_entries, d.n_layers, lay, s_ph);
-    const int u_end = (item.w0 + item.nw - 1) / kPhTile;
-    for (int u = item.w0 / kPhTile; u <= u_end; ++u) {
-      // tile u's hi entry goes to slot u & 1, last read by tile u - 2, whose readers passed
-      // the barrier inside phase_hi_tile for tile u - 1
-      const bool tile_tab =
-          lomid && phase_hi_tile(om, d.n_w, g, u, u & 1, tab_entries, d.n_layers, lay, s_ph);
-      const int k_lo = max(item.w0, u * kPhTile);
-      const int k_hi = min(item.w0 + item.nw, (u + 1) * kPhTile);
-      for (int iw = k_lo + threadIdx.x; iw < k_hi; iw += THREADS) {
-        cd e0, rpp;
-        if (tile_tab) {
-          rpp = sweep_ph(d.n_layers, coef, phase_at(s_ph, tab_entries, iw, u - (u & 1)), &e0);
-        } else {
-          const double2 wv = om[iw];
-          rpp = sweep(mk(wv.x, wv.y), d.n_layers, lay, coef, &e0);
-        }
-        const cd out = pp_surface(rpp, e0, fs);
-        R_all[d.R_off + (size_t)pr.j * d.n_w + iw] = make_double2(out.x, out.y);
-      }
-    }
+    double2* Rp = R_all + d.R_off + (size_t)pr.j * d.n_w;
+    if (!DEEP)
+      forward_item<3, 1, THREADS>(item, d, pr.j, v, om, Rp, s_pair, s_tiles);
+    else if (sweep_phases(d.n_layers) == 2)
+      forward_item<2, 1, THREADS>(item, d, pr.j, v, om, Rp, s_pair, s_tiles);
+    else
+      forward_item<0, 1, THREADS>(item, d, pr.j, v, om, Rp, s_pair, s_tiles);
   }
-  // launched as batch_tan_kernel's programmatic dependent: this grid completes only after
-  // that one has, so the gradient kernel launched after it reads finished tangents
+  // launched as its predecessor's programmatic dependent: this grid completes only after that
+  // one has, so the gradient kernel launched after it reads finished tangents
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
@@ -275,8 +333,10 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
   const PairRec* pairs = reinterpret_cast<const PairRec*>(plan + h->off_pairs);
   const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_grad);
   const int n_items = h->n_grad;
+  __shared__ int s_item;
+  ItemFeed feed(&h->counters[2], &s_item);
   for (;;) {
-    const int it = next_item(&h->counters[1]);
+    const int it = feed.next();
     if (it >= n_items) break;
     const ItemRec item = items[it];
     const PairRec pr = pairs[item.pair];
@@ -373,8 +433,10 @@ batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_al
   // the item's [4L] result reuses the staging rows once the sweeps are done
   double* s_out = reinterpret_cast<double*>(stage);
   unsigned char* area = reinterpret_cast<unsigned char*>(stage + W * kRayStage);
+  __shared__ int s_item;
+  ItemFeed feed(&h->counters[2], &s_item);
   for (;;) {
-    const int it = next_item(&h->counters[1]);
+    const int it = feed.next();
     if (it >= n_items) break;
     const ItemRec item = items[it];
     const PairRec pr = pairs[item.pair];
@@ -463,7 +525,7 @@ static kr_status layout(const kr_model_desc* descs, int n_models, const kr_batch
   h.n_models = n_models;
   h.threads = cfg->threads;
   h.tile_w = cfg->tile_w;
-  long long n_pairs = 0, n_fwd = 0, n_grad = 0;
+  long long n_pairs = 0, n_fwd = 0, n_grad = 0, n_fwd_deep = 0, n_grad_deep = 0;
   size_t coef = 0;
   for (int b = 0; b < n_models; ++b) {
     const kr_model_desc& d = descs[b];
@@ -474,7 +536,9 @@ static kr_status layout(const kr_model_desc* descs, int n_models, const kr_batch
       return KR_ERR_INVALID_ARGUMENT;
     const bool gr = (d.flags & KR_BATCH_GRADIENT) != 0;
     n_pairs += d.n_p;
-    (gr ? n_grad : n_fwd) += (long long)d.n_p * ((d.n_w + cfg->tile_w - 1) / cfg->tile_w);
+    const long long items = (long long)d.n_p * ((d.n_w + cfg->tile_w - 1) / cfg->tile_w);
+    (gr ? n_grad : n_fwd) += items;
+    if (d.n_layers > kPqsLayers) (gr ? n_grad_deep : n_fwd_deep) += items;
     coef += pair_bytes(d) * (size_t)d.n_p;
   }
   if (n_pairs > 0x7fffffffLL || n_fwd > 0x7fffffffLL || n_grad > 0x7fffffffLL)
@@ -482,6 +546,8 @@ static kr_status layout(const kr_model_desc* descs, int n_models, const kr_batch
   h.n_pairs = (int)n_pairs;
   h.n_fwd = (int)n_fwd;
   h.n_grad = (int)n_grad;
+  h.n_fwd_deep = (int)n_fwd_deep;
+  h.n_grad_deep = (int)n_grad_deep;
   size_t off = a256(sizeof(PlanHeader));
   h.off_models = (int64_t)off;
   off = a256(off + sizeof(kr_model_desc) * (size_t)n_models);
@@ -500,8 +566,16 @@ static kr_status layout(const kr_model_desc* descs, int n_models, const kr_batch
 
 constexpr size_t kBatchStageMax = 160 * 1024;
 
-static size_t fwd_smem(int max_layers) {
-  return sizeof(LayerP) * (size_t)max_layers + sizeof(Iface) * (size_t)(max_layers - 1);
+// Shared memory of the forward kernel's two classes for models of up to max_layers.
+static size_t fwd_smem(int threads, int max_layers, bool deep) {
+  const int w = threads / 32;
+  if (!deep) {
+    const int L = std::min(max_layers, kPqsLayers);
+    return sweep_slowness_bytes(L, 3) + w * sweep_warp_bytes(L, 3, 1);
+  }
+  const int L = std::min(max_layers, kPairLayers);
+  return std::max(sweep_slowness_bytes(L, 2) + w * sweep_warp_bytes(L, 2, 1),
+                  prologue_smem_bytes(max_layers));
 }
 
 // Phase-table entries per phase for items of tile_w frequencies (0: direct exponentials for
@@ -562,15 +636,8 @@ static bool batch_sums_enabled() {
 }
 
 template <int THREADS>
-static kr_status grids(PlanHeader& h, int max_layers, int tab_entries, int ftab, size_t* fsm,
-                       size_t* gsm, int* stage, int* gtab, bool* sums) {
-  const int lt = std::min(max_layers, phase_table_max_layers());
-  // a model's table sits right after its own layer terms and coefficients, so the block needs
-  // the larger of the deepest model's prologue and the deepest tabulating model's prologue
-  // plus table (not their sum: 51 instead of 66 KB for 64- and 30-layer models, four blocks
-  // per SM instead of three)
-  *fsm = std::max(fwd_smem(max_layers),
-                  fwd_smem(lt) + (ftab ? sizeof(cd) * (size_t)ftab * 2 * (size_t)(lt - 1) : 0));
+static kr_status grids(PlanHeader& h, int max_layers, int tab_entries, size_t* gsm, int* stage,
+                       int* gtab, bool* sums) {
   int stab = 0;
   const size_t ssm = batch_sums_enabled() ? sums_smem(THREADS, max_layers, tab_entries, &stab) : 0;
   *sums = ssm > 0;
@@ -583,16 +650,12 @@ static kr_status grids(PlanHeader& h, int max_layers, int tab_entries, int ftab,
   }
   // limits only ever rise (raise_smem_limit), so batches of different shapes launched from
   // several host threads at once never find a kernel's limit lowered under them
-  static SmemLimit flim, slim, glim;
-  if (*fsm > 48 * 1024 && raise_smem_limit((const void*)batch_forward_kernel<THREADS>, *fsm, flim,
-                                           "kr_batch_launch: forward smem") != KR_OK)
-    return KR_ERR_CUDA;
+  static SmemLimit slim, glim;
   const void* gk = *sums ? (const void*)batch_grad_sums_kernel<THREADS>
                         : (const void*)batch_gradient_kernel<THREADS>;
   if (*gsm > 48 * 1024 && raise_smem_limit(gk, *gsm, *sums ? slim : glim,
                                            "kr_batch_launch: gradient smem") != KR_OK)
     return KR_ERR_CUDA;
-  h.grid_fwd = occupancy_grid((const void*)batch_forward_kernel<THREADS>, THREADS, *fsm);
   h.grid_grad = occupancy_grid(gk, THREADS, *gsm);
   return KR_OK;
 }
@@ -616,7 +679,7 @@ static size_t meta_bytes(const PlanLayout& lay) {
 // Fills the plan's metadata image (header, model table, pair table, work lists) of
 // meta_bytes(lay) bytes.  Host only: no CUDA call.  Items of one model differ in cost only
 // between its full frequency ranges and its last, shorter one, so the lists are sorted as
-// groups (model, full or last range) by descending cost and then written out: planning 4096
+// groups (model, full or last range), deep models first, by descending cost and then written out: planning 4096
 // models of 12 slownesses took four passes of 1.4 to 3.9 ms, two of them sorting 49152 items.
 static void plan_image(const kr_model_desc* descs, int n_models, const kr_batch_config* cfg,
                        const PlanLayout& lay, unsigned char* img) {
@@ -645,8 +708,11 @@ static void plan_image(const kr_model_desc* descs, int n_models, const kr_batch_
     for (int j = 0; j < d.n_p; ++j, ++q, off += pb) pairs[q] = PairRec{b, j, off};
   }
   auto write = [&](std::vector<Group>& list, ItemRec* it) {
-    std::stable_sort(list.begin(), list.end(),
-                     [](const Group& a, const Group& b) { return a.cost > b.cost; });
+    std::stable_sort(list.begin(), list.end(), [&](const Group& a, const Group& b) {
+      const bool da = descs[a.model].n_layers > kPqsLayers;
+      const bool db = descs[b.model].n_layers > kPqsLayers;
+      return da != db ? da : a.cost > b.cost;
+    });
     for (const Group& g : list) {
       const kr_model_desc& d = descs[g.model];
       const int full = d.n_w / cfg->tile_w;
@@ -706,6 +772,35 @@ extern "C" kr_status kr_batch_plan(const kr_model_desc* descs, int32_t n_models,
 
 namespace kr {
 
+// One class of the forward items on a resident grid.  `after`: as the programmatic dependent of
+// the launch before it (the tangents, or the deep class).
+template <int THREADS, bool DEEP>
+static kr_status launch_batch_forward(unsigned char* pl, int max_layers, const double2* w,
+                                      double2* R, bool after, cudaStream_t st) {
+  const void* fn = (const void*)batch_forward_kernel<THREADS, DEEP>;
+  const size_t smem = fwd_smem(THREADS, max_layers, DEEP);
+  static SmemLimit lim;
+  if (smem > 46 * 1024 &&  // with the static arrays above the 48 KB default
+      raise_smem_limit(fn, smem, lim, "kr_batch_launch: forward smem") != KR_OK)
+    return KR_ERR_CUDA;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(occupancy_grid(fn, THREADS, smem));
+  lc.blockDim = dim3(THREADS);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = after ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&lc, batch_forward_kernel<THREADS, DEEP>, pl, w, R);
+  if (e != cudaSuccess) {
+    set_last_error("kr_batch_launch: forward", e);
+    return KR_ERR_CUDA;
+  }
+  return KR_OK;
+}
+
 // One batch launch for a block size of THREADS (32: one warp per work item, i.e. per
 // (model, slowness) pair and frequency range; 64 / 128: two / four warps per item).
 template <int THREADS>
@@ -715,14 +810,12 @@ static kr_status launch_batch(unsigned char* pl, const kr_batch_config* cfg, int
                               cudaStream_t st) {
   // Grid sizes from an occupancy query (host-side, capture-safe).
   PlanHeader h{};
-  size_t fsm = 0, gsm = 0;
+  size_t gsm = 0;
   int stage = 0;
   const int tab = fwd_table_entries(cfg->tile_w);
-  // the forward kernel holds lo / mid and two tiles' hi entries per phase (kPhHead + 2)
-  const int ftab = kPhHead + 2;
   int gtab = 0;
   bool sums = false;
-  kr_status s = grids<THREADS>(h, max_layers, tab, ftab, &fsm, &gsm, &stage, &gtab, &sums);
+  kr_status s = grids<THREADS>(h, max_layers, tab, &gsm, &stage, &gtab, &sums);
   if (s != KR_OK) {
     set_last_error_msg("kr_batch_launch: shared-memory attribute");
     return s;
@@ -730,33 +823,29 @@ static kr_status launch_batch(unsigned char* pl, const kr_batch_config* cfg, int
   batch_reset_kernel<<<148, 128, 0, st>>>(pl, chi_grad);
   s = check_launch("kr_batch_launch: reset");
   if (s != KR_OK) return s;
-  batch_prep_kernel<<<148 * 16, 64, 0, st>>>(pl, layers, p);
+  int gs = 4;
+  while (gs < max_layers && gs < kPrepBlock) gs *= 2;
+  batch_prep_kernel<<<148 * 16, kPrepBlock, 0, st>>>(pl, layers, p, gs);
   s = check_launch("kr_batch_launch: prep");
   if (s != KR_OK) return s;
-  // tangents on a resident-sized grid (every block starts at once and releases the forward
-  // kernel), the forward kernel as its programmatic dependent
-  batch_tan_kernel<<<148 * 4, 64, 0, st>>>(pl, p);
-  s = check_launch("kr_batch_launch: tangents");
-  if (s != KR_OK) return s;
-  const double2* w = reinterpret_cast<const double2*>(omega);
-  {
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3(h.grid_fwd);
-    lc.blockDim = dim3(THREADS);
-    lc.dynamicSmemBytes = fsm;
-    lc.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&lc, batch_forward_kernel<THREADS>, pl, w,
-                                             reinterpret_cast<double2*>(R), ftab);
-    if (e != cudaSuccess) {
-      set_last_error("kr_batch_launch: forward", e);
-      return KR_ERR_CUDA;
-    }
+  // a batch without observed data has no gradient models: no tangents, no gradient kernel
+  const bool grads = R_obs != nullptr;
+  if (grads) {
+    // tangents on a resident-sized grid: every block starts at once and releases the forward
+    // kernel, its programmatic dependent
+    batch_tan_kernel<<<148 * 4, 64, 0, st>>>(pl, p);
+    s = check_launch("kr_batch_launch: tangents");
+    if (s != KR_OK) return s;
   }
+  const double2* w = reinterpret_cast<const double2*>(omega);
+  double2* R2 = reinterpret_cast<double2*>(R);
+  if (max_layers > kPqsLayers) {
+    s = launch_batch_forward<THREADS, true>(pl, max_layers, w, R2, grads, st);
+    if (s != KR_OK) return s;
+  }
+  s = launch_batch_forward<THREADS, false>(pl, max_layers, w, R2, grads || max_layers > kPqsLayers,
+                                           st);
+  if (s != KR_OK || !grads) return s;
   if (sums)
     batch_grad_sums_kernel<THREADS><<<h.grid_grad, THREADS, gsm, st>>>(
         pl, w, reinterpret_cast<const double2*>(R_obs), reinterpret_cast<double2*>(R), chi_grad,

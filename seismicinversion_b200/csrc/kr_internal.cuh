@@ -76,53 +76,6 @@ inline kr_status check_launch(const char* where) {
   return KR_OK;
 }
 
-// Computes the layer terms and interface coefficients of one slowness into shared memory
-// (threads of the block cooperate: one layer / one interface per thread).  Ends with a
-// block barrier.
-__device__ __forceinline__ void block_prologue(const double* __restrict__ tab, int n_layers,
-                                               double p, LayerP* s_layer, Iface* s_iface) {
-  for (int l = threadIdx.x; l < n_layers; l += blockDim.x) s_layer[l] = layer_terms(tab, n_layers, l, p);
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_layers - 1; i += blockDim.x)
-    s_iface[i] = interface_coeffs(p, i, s_layer[i], s_layer[i + 1]);
-  __syncthreads();
-}
-
-// The full upward sweep for one (omega, p) with coefficients in shared memory; `ph` supplies
-// the layer phase factors (PhaseDirect, or a tabulated source with the same a(l) / b(l)).
-// Returns RRd_PP below the ocean and the ocean phase factor e0.  The phase factors of the
-// next layer are fetched one step ahead, so their latency overlaps the current step's
-// algebra; the last (ocean-bottom) step forms only RRd_00.
-template <class Ph>
-__device__ __forceinline__ cd sweep_ph(int n_layers, const Iface* s_iface, const Ph& ph,
-                                       cd* e0_out) {
-  const int I = n_layers - 1;
-  // Bottom interface: RRd below it is 0, so RRd = Rd.
-  M2 r;
-  r.a = s_iface[I - 1].rd11;
-  r.b = s_iface[I - 1].rd12;
-  r.c = s_iface[I - 1].rd12;
-  r.d = s_iface[I - 1].rd22;
-  if (I == 1) {
-    *e0_out = ph.a(0);
-    return r.a;
-  }
-  cd ea = ph.a(I - 1), eb = ph.b(I - 1);
-  for (int i = I - 2; i >= 1; --i) {
-    const cd ea_n = ph.a(i), eb_n = ph.b(i);
-    r = kennett_step(r, ea, eb, s_iface[i]);
-    ea = ea_n;
-    eb = eb_n;
-  }
-  *e0_out = ph.a(0);
-  return kennett_last_step_pp(r, ea, eb, s_iface[0]);
-}
-
-__device__ __forceinline__ cd sweep(cd w, int n_layers, const LayerP* s_layer,
-                                    const Iface* s_iface, cd* e0_out) {
-  return sweep_ph(n_layers, s_iface, PhaseDirect{w, s_layer}, e0_out);
-}
-
 // Block-cooperative copy of n bytes (multiple of 16, 16-byte aligned) into shared memory.
 __device__ __forceinline__ void copy16(void* dst, const void* src, size_t n) {
   double2* d = reinterpret_cast<double2*>(dst);

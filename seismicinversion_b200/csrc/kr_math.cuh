@@ -66,6 +66,27 @@ KR_HD cd recip(cd z) {
   double inv = 1.0 / fma(zx, zx, zy * zy);
   return mk(zx * inv * s, -zy * inv * s);
 }
+
+// 1/z of a step determinant (|z| near 1 in practice).  recip() spends ~20 FP64 instructions,
+// most of them on range scaling and the correctly rounded division; here the range is tested
+// on the exponent bits of |z|^2 (integer work) and 1/|z|^2 comes from the hardware's
+// reciprocal estimate y (relative error e < 2^-19) refined once by the cubically convergent
+// iteration y (1 + e + e^2), e = 1 - n y (Householder's method for 1/n: the new error is
+// e^3 < 2^-57, then one rounding): 8 FP64 instructions, within 2 ulp of the quotient.
+KR_HD cd recip_near(cd z) {
+#ifdef __CUDA_ARCH__
+  const double n = fma(z.x, z.x, z.y * z.y);
+  // 2^-800 <= n < 2^800: neither n nor its estimate is near the ends of the range
+  if ((unsigned)(__double2hiint(n) - (223 << 20)) < (unsigned)(1600 << 20)) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(n));
+    const double e = fma(-n, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
+    return mk(z.x * y, -z.y * y);
+  }
+#endif
+  return recip(z);
+}
 KR_HD cd operator/(cd a, cd b) { return a * recip(b); }
 KR_HD cd operator/(cd a, double s) { return mk(a.x / s, a.y / s); }
 
@@ -136,30 +157,36 @@ struct PhaseDirect {
 
 // Layer table layout (device or host): 6 rows of n_layers doubles:
 // alpha, beta, rho, thickness, Q_alpha, Q_beta.
-KR_HD LayerP layer_terms(const double* tab, int n_layers, int l, double p) {
-  const double alpha = tab[l];
-  const double beta = tab[n_layers + l];
-  const double rho = tab[2 * n_layers + l];
+//
+// The P and the S half of a layer's terms are independent chains (two divisions, a complex
+// root), so a block's prologue gives each its own thread.
+KR_HD void layer_terms_p(const double* tab, int n_layers, int l, double p, LayerP& o) {
   const double h = tab[3 * n_layers + l];
-  const double qa = tab[4 * n_layers + l];
-  const double qb = tab[5 * n_layers + l];
-  LayerP o;
-  cd sp = complex_slowness(alpha, qa);
-  cd ss = beta > 0.0 ? complex_slowness(beta, qb) : mk(0.0, 0.0);
-  o.betac = (ss.x != 0.0 || ss.y != 0.0) ? recip(ss) : mk(0.0, 0.0);
-  o.eta = vertical_slowness(sp, p);
-  o.neta = (l == 0) ? mk(0.0, 0.0) : vertical_slowness(ss, p);
-  if (is_half_space(h)) {
-    o.ca = mk(0.0, 0.0);
-    o.cb = mk(0.0, 0.0);
-  } else {
-    o.ca = mk(-o.eta.y * h, o.eta.x * h);
-    o.cb = mk(-o.neta.y * h, o.neta.x * h);
-  }
-  o.rho = rho;
+  o.eta = vertical_slowness(complex_slowness(tab[l], tab[4 * n_layers + l]), p);
+  o.ca = is_half_space(h) ? mk(0.0, 0.0) : mk(-o.eta.y * h, o.eta.x * h);
+  o.rho = tab[2 * n_layers + l];
   o.pad = 0.0;
+}
+KR_HD void layer_terms_s(const double* tab, int n_layers, int l, double p, LayerP& o) {
+  const double beta = tab[n_layers + l];
+  const double h = tab[3 * n_layers + l];
+  const cd ss = beta > 0.0 ? complex_slowness(beta, tab[5 * n_layers + l]) : mk(0.0, 0.0);
+  o.betac = (ss.x != 0.0 || ss.y != 0.0) ? recip(ss) : mk(0.0, 0.0);
+  o.neta = (l == 0) ? mk(0.0, 0.0) : vertical_slowness(ss, p);
+  o.cb = is_half_space(h) ? mk(0.0, 0.0) : mk(-o.neta.y * h, o.neta.x * h);
+}
+KR_HD LayerP layer_terms(const double* tab, int n_layers, int l, double p) {
+  LayerP o;
+  layer_terms_p(tab, n_layers, l, p, o);
+  layer_terms_s(tab, n_layers, l, p, o);
   return o;
 }
+
+// Square roots of a layer that its two interfaces' coefficients share: formed once per layer
+// (four complex roots, ~150 instructions each, leave the coefficients' serial chain).
+struct LayerRoots {
+  cd eta, neta;  // sqrt(eta), sqrt(neta)
+};
 
 // ---------------------------------------------------------------------------------------
 // Interface coefficients: Rd, Ru symmetric (3 entries each), Td full (Tu = Td^T).
@@ -183,10 +210,8 @@ struct Iface : IfaceT<cd> {
 // (T = a dual number).  rho enters as T so its tangent can be seeded.
 template <class T>
 KR_HD void solid_solid(double p, T eta1, T neta1, T rho1, T beta1, T eta2, T neta2, T rho2,
-                       T beta2, IfaceT<T>& o) {
-  T rteta1 = csqrt(eta1), rteta2 = csqrt(eta2);
-  T rtneta1 = csqrt(neta1), rtneta2 = csqrt(neta2);
-  T rtrho1 = csqrt(rho1), rtrho2 = csqrt(rho2);
+                       T beta2, T rteta1, T rtneta1, T rtrho1, T rteta2, T rtneta2, T rtrho2,
+                       IfaceT<T>& o) {
   T rtza1 = rteta1 * rtrho1, rtza2 = rteta2 * rtrho2;
   T rtzb1 = rtneta1 * rtrho1, rtzb2 = rtneta2 * rtrho2;
   const double psq = p * p;
@@ -226,10 +251,8 @@ KR_HD void solid_solid(double p, T eta1, T neta1, T rho1, T beta1, T eta2, T net
 }
 
 template <class T>
-KR_HD void ocean_bottom(double p, T eta1, T rho1, T eta2, T neta2, T rho2, T beta2,
-                        IfaceT<T>& o) {
-  T rteta1 = csqrt(eta1), rteta2 = csqrt(eta2), rtneta2 = csqrt(neta2);
-  T rtrho1 = csqrt(rho1), rtrho2 = csqrt(rho2);
+KR_HD void ocean_bottom(double p, T eta1, T rho1, T eta2, T neta2, T rho2, T beta2, T rteta1,
+                        T rtrho1, T rteta2, T rtneta2, T rtrho2, IfaceT<T>& o) {
   T rtza1 = rtrho1 * rteta1, rtza2 = rtrho2 * rteta2, rtzb2 = rtrho2 * rtneta2;
   const double psq = p * p;
   T d = 2.0 * (rho2 * beta2 * beta2);
@@ -266,16 +289,33 @@ KR_HD void ocean_bottom(double p, T eta1, T rho1, T eta2, T neta2, T rho2, T bet
   o.td22 = zero;
 }
 
+template <class T>
+KR_HD void solid_solid(double p, T eta1, T neta1, T rho1, T beta1, T eta2, T neta2, T rho2,
+                       T beta2, IfaceT<T>& o) {
+  solid_solid(p, eta1, neta1, rho1, beta1, eta2, neta2, rho2, beta2, csqrt(eta1), csqrt(neta1),
+              csqrt(rho1), csqrt(eta2), csqrt(neta2), csqrt(rho2), o);
+}
+template <class T>
+KR_HD void ocean_bottom(double p, T eta1, T rho1, T eta2, T neta2, T rho2, T beta2,
+                        IfaceT<T>& o) {
+  ocean_bottom(p, eta1, rho1, eta2, neta2, rho2, beta2, csqrt(eta1), csqrt(rho1), csqrt(eta2),
+               csqrt(neta2), csqrt(rho2), o);
+}
+
 KR_HD cd to_c(double r) { return mk(r, 0.0); }
 
-// Coefficients of interface `iface` (between layers iface and iface+1) from layer terms.
-KR_HD Iface interface_coeffs(double p, int iface, const LayerP& up, const LayerP& lo) {
+// Coefficients of interface `iface` (between layers iface and iface+1) from layer terms and
+// their square roots (the root of a real density is real).
+KR_HD Iface interface_coeffs(double p, int iface, const LayerP& up, const LayerP& lo,
+                             const LayerRoots& rup, const LayerRoots& rlo) {
   Iface o;
+  const cd r1 = to_c(sqrt(up.rho)), r2 = to_c(sqrt(lo.rho));
   if (iface == 0)
-    ocean_bottom<cd>(p, up.eta, to_c(up.rho), lo.eta, lo.neta, to_c(lo.rho), lo.betac, o);
+    ocean_bottom<cd>(p, up.eta, to_c(up.rho), lo.eta, lo.neta, to_c(lo.rho), lo.betac, rup.eta,
+                     r1, rlo.eta, rlo.neta, r2, o);
   else
     solid_solid<cd>(p, up.eta, up.neta, to_c(up.rho), up.betac, lo.eta, lo.neta, to_c(lo.rho),
-                    lo.betac, o);
+                    lo.betac, rup.eta, rup.neta, r1, rlo.eta, rlo.neta, r2, o);
   const cd t11 = o.td11, t12 = o.td12, t21 = o.td21, t22 = o.td22;
   o.ru12x2 = 2.0 * o.ru12;
   o.dru = cdot2(o.ru11, o.ru22, -o.ru12, o.ru12);
@@ -289,6 +329,11 @@ KR_HD Iface interface_coeffs(double p, int iface, const LayerP& up, const LayerP
   o.q[7] = 2.0 * (t12 * t22);
   o.q[8] = t22 * t22;
   return o;
+}
+
+KR_HD Iface interface_coeffs(double p, int iface, const LayerP& up, const LayerP& lo) {
+  return interface_coeffs(p, iface, up, lo, LayerRoots{csqrt(up.eta), csqrt(up.neta)},
+                          LayerRoots{csqrt(lo.eta), csqrt(lo.neta)});
 }
 
 // ---------------------------------------------------------------------------------------
@@ -316,55 +361,54 @@ struct M2 {
   cd a, b, c, d;
 };
 
-// X = MT (I - Ru MT)^-1 of the step (entries 11, 12, 22).
-KR_HD void step_x(const M2& r, cd ea, cd eb, const Iface& f, cd& x11, cd& x12, cd& x22) {
-  cd eaea = ea * ea, ebeb = eb * eb, eaeb = ea * eb;
-  cd m11 = eaea * r.a, m12 = eaeb * r.b, m22 = ebeb * r.d;
-  cd dm = cdot2(m11, m22, -m12, m12);
+// X = MT (I - Ru MT)^-1 of the step (entries 11, 12, 22) from the squared and mixed phase
+// factors P = ea^2, Q = eb^2, S = ea eb.
+KR_HD void step_x(const M2& r, cd P, cd Q, cd S, const Iface& f, cd& x11, cd& x12, cd& x22) {
+  const cd m11 = P * r.a, m12 = S * r.b, m22 = Q * r.d;
+  const cd dm = cdot2(m11, m22, -m12, m12);
   const cd one = mk(1.0, 0.0);
-  cd idet = recip(cmac(cmac(cmac(cmac(one, -f.ru11, m11), -f.ru12x2, m12), -f.ru22, m22),
-                       f.dru, dm));
+  const cd idet = recip_near(
+      cmac(cmac(cmac(cmac(one, -f.ru11, m11), -f.ru12x2, m12), -f.ru22, m22), f.dru, dm));
   x11 = cmac(m11, -f.ru22, dm) * idet;
   x12 = cmac(m12, f.ru12, dm) * idet;
   x22 = cmac(m22, -f.ru11, dm) * idet;
 }
 
+// The step, which also hands out X: the reverse sweep of the derivatives needs nothing else of
+// it (kr_adjoint.cuh).
+KR_HD M2 kennett_step_x(const M2& r, cd P, cd Q, cd S, const Iface& f, cd& x11, cd& x12,
+                        cd& x22) {
+  step_x(r, P, Q, S, f, x11, x12, x22);
+  M2 o;
+  o.a = cmac(cmac(cmac(f.rd11, f.q[0], x11), f.q[1], x12), f.q[2], x22);
+  o.b = cmac(cmac(cmac(f.rd12, f.q[3], x11), f.q[4], x12), f.q[5], x22);
+  o.d = cmac(cmac(cmac(f.rd22, f.q[6], x11), f.q[7], x12), f.q[8], x22);
+  o.c = o.b;
+  return o;
+}
+
 KR_HD M2 kennett_step(const M2& r, cd ea, cd eb, const Iface& f) {
   cd x11, x12, x22;
-  step_x(r, ea, eb, f, x11, x12, x22);
-  M2 o;
-  o.a = cmac(cmac(cmac(f.rd11, f.q[0], x11), f.q[1], x12), f.q[2], x22);
-  o.b = cmac(cmac(cmac(f.rd12, f.q[3], x11), f.q[4], x12), f.q[5], x22);
-  o.d = cmac(cmac(cmac(f.rd22, f.q[6], x11), f.q[7], x12), f.q[8], x22);
-  o.c = o.b;
-  return o;
+  return kennett_step_x(r, ea * ea, eb * eb, ea * eb, f, x11, x12, x22);
 }
 
-// kennett_step that also hands out X (entries 11, 12, 22), from which the reverse sweep of the
-// derivatives needs nothing else of the step (kr_adjoint.cuh).  Same arithmetic, same bits.
-KR_HD M2 kennett_step_keep(const M2& r, cd ea, cd eb, const Iface& f, cd& x11, cd& x12, cd& x22) {
-  step_x(r, ea, eb, f, x11, x12, x22);
-  M2 o;
-  o.a = cmac(cmac(cmac(f.rd11, f.q[0], x11), f.q[1], x12), f.q[2], x22);
-  o.b = cmac(cmac(cmac(f.rd12, f.q[3], x11), f.q[4], x12), f.q[5], x22);
-  o.d = cmac(cmac(cmac(f.rd22, f.q[6], x11), f.q[7], x12), f.q[8], x22);
-  o.c = o.b;
-  return o;
-}
-
-// The last (ocean-bottom) step, returning only RRd_00 (the same arithmetic as kennett_step's
-// first entry; that interface's Td has one column, so only q[0..2] are non-zero).
-KR_HD cd kennett_last_step_pp(const M2& r, cd ea, cd eb, const Iface& f) {
+// The last (ocean-bottom) step, returning only RRd_00 (that interface's Td has one column, so
+// only q[0..2] are non-zero).
+KR_HD cd kennett_last_step_pp(const M2& r, cd P, cd Q, cd S, const Iface& f) {
   cd x11, x12, x22;
-  step_x(r, ea, eb, f, x11, x12, x22);
+  step_x(r, P, Q, S, f, x11, x12, x22);
   return cmac(cmac(cmac(f.rd11, f.q[0], x11), f.q[1], x12), f.q[2], x22);
 }
 
-// PP reflectivity at the surface from RRd_PP below the ocean and the ocean phase e0.
-KR_HD cd pp_surface(cd rpp, cd e0, bool free_surface) {
-  cd y = (e0 * e0) * rpp;
+// PP reflectivity at the surface from RRd_PP below the ocean and the squared ocean phase, or
+// the ocean phase e0 itself.
+KR_HD cd pp_surface2(cd rpp, cd e0e0, bool free_surface) {
+  cd y = e0e0 * rpp;
   if (!free_surface) return y;
   return y * recip(1.0 + y);
+}
+KR_HD cd pp_surface(cd rpp, cd e0, bool free_surface) {
+  return pp_surface2(rpp, e0 * e0, free_surface);
 }
 
 }  // namespace kr

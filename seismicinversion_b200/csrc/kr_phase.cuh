@@ -13,7 +13,8 @@
 // shared-memory reads replace an exp and a sincos per layer, phase and frequency.  A tile
 // whose frequencies leave the line, or whose entries exceed 1e100 in magnitude (so that no
 // product can overflow), evaluates its phases directly.  The per-tile decision depends only
-// on the grid, so every kernel that uses this table gives bit-identical results.
+// on the grid, so the derivative kernels, which use this table, agree bit for bit; the forward
+// kernels tabulate by the same rules in the form their warps read (kr_sweep.cuh).
 #pragma once
 
 #include "kr_internal.cuh"
@@ -34,9 +35,9 @@ __host__ __device__ inline size_t phase_table_bytes(int n_layers, int tiles) {
   return sizeof(cd) * (size_t)phase_entries(tiles) * 2 * (size_t)(n_layers - 1);
 }
 
-// Which models tabulate: those whose forward-kernel block (prologue + a table of 16 tiles)
-// stays within 50 KB of shared memory, i.e. up to 30 layers.  Every kernel applies the same
-// per-model rule, so a model's phases come from the same source everywhere.
+// Which models tabulate in these kernels: those whose layer terms, coefficients and a table of
+// 16 tiles stay within 50 KB of shared memory, i.e. up to 30 layers.  Every kernel applies the
+// same per-model rule, so a model's phases come from the same source everywhere.
 constexpr int kFwdTabTiles = 16;
 constexpr size_t kFwdTabSmemMax = 50 * 1024;
 __host__ __device__ inline bool phase_table_model(int n_layers) {
@@ -86,32 +87,6 @@ struct PhaseAuto {
   __device__ __forceinline__ cd b(int l) const { return tab ? t.b(l) : d.b(l); }
   __device__ __forceinline__ bool cheap() const { return tab; }
 };
-
-// The same factors with the per-tile products hi[u] * mid[m] formed once per tile
-// (phase_hm_warp): one complex product per lookup instead of two, the same roundings in the
-// same order, so the values are bit-identical to PhaseTable's.  A warp's 32 consecutive
-// frequencies use two mid entries, so each warp forms its own products (no block barrier).
-struct PhaseTableHM {
-  const cd* tab;
-  const cd* hm;  // [2 (L - 1)][2] products of the warp's current tile
-  int entries, lo, m;  // m: which of the warp's two mid entries
-  __device__ __forceinline__ cd at(int id) const {
-    return hm[2 * id + m] * tab[id * entries + lo];
-  }
-  __device__ __forceinline__ cd a(int l) const { return at(2 * l); }
-  __device__ __forceinline__ cd b(int l) const { return at(2 * l + 1); }
-};
-
-// Warp-cooperative: s_hm[2 id + k] = hi[hi_entry] * mid[m0 + k] (k = 0, 1) for the n_phase
-// phases, followed by __syncwarp.
-__device__ __forceinline__ void phase_hm_warp(const cd* s_ph, int entries, int n_phase,
-                                              int hi_entry, int m0, cd* s_hm) {
-  for (int e = threadIdx.x & 31; e < 2 * n_phase; e += 32) {
-    const cd* q = s_ph + (e >> 1) * entries;
-    s_hm[e] = q[hi_entry] * q[kPhLo + m0 + (e & 1)];
-  }
-  __syncwarp();
-}
 
 __device__ __forceinline__ PhaseTable phase_at(const cd* s_ph, int entries, int k, int u0) {
   const int t = k & (kPhTile - 1);
@@ -168,53 +143,6 @@ __device__ inline unsigned build_phase_table(const double2* __restrict__ omega, 
   __syncthreads();
   const unsigned b = *s_bad;
   return (b >> 31) ? 0u : ~b;
-}
-
-// The same table built in two block-cooperative pieces, for kernels that hold the hi entries
-// of one or two tiles at a time (kPhHead + slots entries per phase): build_phase_lomid fills
-// the lo and mid entries of every phase and returns whether all of them are usable;
-// phase_hi_tile fills tile u's hi entry in hi slot `slot` and returns whether tile u uses
-// the table.  Every entry and every decision is formed exactly as build_phase_table forms it,
-// so the phase factors are bit-identical to it.  Each contains a block barrier and reads
-// omega / lay only; all threads must call them.
-__device__ inline bool build_phase_lomid(const GridLine& g, int entries, int n_layers,
-                                         const LayerP* lay, cd* s_ph) {
-  bool bad = false;
-  const int n_phase = 2 * (n_layers - 1);
-  for (int e = threadIdx.x; e < n_phase * kPhHead; e += blockDim.x) {
-    const int id = e / kPhHead, j = e - id * kPhHead;
-    const LayerP& lp = lay[id >> 1];
-    const cd c = (id & 1) ? lp.cb : lp.ca;
-    const cd z = j < kPhLo ? (double)j * g.d : (double)((j - kPhLo) * kPhLo) * g.d;
-    const cd v = cexp_(z * c);
-    if (!(fabs(v.x) <= kPhMaxMag && fabs(v.y) <= kPhMaxMag)) bad = true;
-    s_ph[id * entries + j] = v;
-  }
-  return __syncthreads_or(bad) == 0;
-}
-
-__device__ inline bool phase_hi_tile(const double2* __restrict__ omega, int n_w,
-                                     const GridLine& g, int u, int slot, int entries,
-                                     int n_layers, const LayerP* lay, cd* s_ph) {
-  bool bad = false;
-  const int k_end = min(n_w, (u + 1) * kPhTile);
-  for (int k = u * kPhTile + threadIdx.x; k < k_end; k += blockDim.x) {
-    const double2 w = omega[k];
-    const double m = (double)k;
-    const bool ok = fabs(w.x - fma(m, g.d.x, g.w0.x)) <= g.tol &&
-                    fabs(w.y - fma(m, g.d.y, g.w0.y)) <= g.tol;
-    if (!ok) bad = true;
-  }
-  const int n_phase = 2 * (n_layers - 1);
-  const double2 ws = omega[u * kPhTile];
-  for (int id = threadIdx.x; id < n_phase; id += blockDim.x) {
-    const LayerP& lp = lay[id >> 1];
-    const cd c = (id & 1) ? lp.cb : lp.ca;
-    const cd v = cexp_(mk(ws.x, ws.y) * c);
-    if (!(fabs(v.x) <= kPhMaxMag && fabs(v.y) <= kPhMaxMag)) bad = true;
-    s_ph[id * entries + kPhHead + slot] = v;
-  }
-  return __syncthreads_or(bad) == 0;
 }
 
 }  // namespace kr

@@ -54,14 +54,13 @@ __device__ __forceinline__ bool phase_usable(cd v) {
   return fabs(v.x) <= kPhMaxMag && fabs(v.y) <= kPhMaxMag;
 }
 
-// Entry e (id kPhHead + j) of a slowness's lo / mid table; returns whether it is usable.
+// Entry j (lo, then mid) of phase `id` of a slowness's table; returns whether it is usable.
 template <int NPH>
-__device__ __forceinline__ bool sweep_table_entry(const GridLine& g, const LayerP* lay, int e,
-                                                  cd* tab) {
-  const int id = e / kPhHead, j = e - id * kPhHead;
+__device__ __forceinline__ bool sweep_table_entry(const GridLine& g, const LayerP* lay, int id,
+                                                  int j, cd* tab) {
   const cd z = (double)(j < kPhLo ? j : (j - kPhLo) * kPhLo) * g.d;
   const cd v = cexp_(z * sweep_exponent<NPH>(lay, id));
-  tab[e] = v;
+  tab[id * kPhHead + j] = v;
   return phase_usable(v);
 }
 
