@@ -15,7 +15,7 @@
  *
  * Stream capture: the launch entry points (kr_reflectivity, kr_gmm_reflectivity,
  * kr_bessel_sum[_noalloc], kr_traces, kr_jacobian, kr_misfit_gradient, kr_vjp,
- * kr_misfit_hvp, kr_jacobian_dot, kr_batch_launch) make
+ * kr_misfit_hvp, kr_misfit_hessian, kr_jacobian_dot, kr_batch_launch) make
  * no CUDA runtime call besides their launches once they have been called on that device with
  * the same sizes (the first call raises kernel shared-memory limits, creates the cuFFT plan
  * or looks up static scratch), so later calls can be recorded into a CUDA graph.
@@ -156,6 +156,25 @@ size_t kr_vjp_workspace_bytes(int32_t n_layers, int32_t n_p, int32_t n_w);
 kr_status kr_vjp(const double* layers, int32_t n_layers, const double* p, int32_t n_p,
                  const double* omega, int32_t n_w, uint32_t flags, const double* gR, double* R,
                  double* grad, void* workspace, size_t workspace_bytes, void* stream);
+
+/* Bytes of device workspace kr_misfit_hessian needs; 0 for models it does not take (deeper than
+ * a block's shared memory holds, 50 layers), for which kr_misfit_hvp gives the Hessian. */
+size_t kr_misfit_hessian_workspace_bytes(int32_t n_layers, int32_t n_p, int32_t n_w);
+
+/*
+ * Exact Hessian of the misfit chi = sum_{p, w} |R - R_obs|^2 over the parameters of the layers
+ * below the ocean: H[k*N + l-1][k'*N + l'-1] = d^2 chi / d theta d theta', N = n_layers - 1,
+ * k = alpha, beta, rho, h of layer l = 1 .. N (the half-space's h row and column are zero).
+ * The same second derivatives as kr_misfit_hvp along every axis (taup_inversion.py:177,
+ * kennett_torch.py:644-684), formed pair by pair from one forward and one reverse sweep per
+ * (p, w); block partials reduced in a fixed order (deterministic).
+ *   R_obs : device complex [n_p][n_w];  H : device float64 [4N][4N] output
+ *   workspace : >= kr_misfit_hessian_workspace_bytes(n_layers, n_p, n_w) bytes
+ */
+kr_status kr_misfit_hessian(const double* layers, int32_t n_layers, const double* p, int32_t n_p,
+                            const double* omega, int32_t n_w, uint32_t flags,
+                            const double* R_obs, double* H, void* workspace,
+                            size_t workspace_bytes, void* stream);
 
 /* Bytes of device workspace kr_misfit_hvp needs for n_dir directions. */
 size_t kr_misfit_hvp_workspace_bytes(int32_t n_layers, int32_t n_p, int32_t n_w, int32_t n_dir);

@@ -64,6 +64,9 @@ _SIGNATURES = {
     "kr_misfit_hvp_workspace_bytes": (_size_t, [_i32, _i32, _i32, _i32]),
     "kr_misfit_hvp": (_i32, [_vp, _i32, _vp, _i32, _vp, _i32, _u32, _vp, _vp, _i32, _vp, _vp,
                              _size_t, _vp]),
+    "kr_misfit_hessian_workspace_bytes": (_size_t, [_i32, _i32, _i32]),
+    "kr_misfit_hessian": (_i32, [_vp, _i32, _vp, _i32, _vp, _i32, _u32, _vp, _vp, _vp, _size_t,
+                                 _vp]),
     "kr_jacobian_dot_workspace_bytes": (_size_t, [_i32, _i32, _i32, _i32]),
     "kr_jacobian_dot": (_i32, [_vp, _i32, _vp, _i32, _vp, _i32, _u32, _vp, _i32, _vp, _vp,
                                _size_t, _vp]),

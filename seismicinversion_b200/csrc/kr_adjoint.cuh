@@ -369,9 +369,9 @@ KR_HD size_t sum_rows(int L) { return (size_t)L; }
 
 // One (omega, p) pair: forward sweep with the tape of jacobian_pair, seed, reverse sweep.  The
 // sink gets once top(f0) (the ocean phase term of layer 0) and per step
-// ray(i, g, x, wz): g and x of ray_step at interface i and omega z, whose products are the 12
-// adjoints (the 10 of ray_adjoints; fa = 2 wz_a x_a, fb = 2 wz_b x_b); the bottom interface
-// comes with x = wz = 0.
+// ray(i, g, x, wz, X, ea, eb): g and x of ray_step at interface i and omega z, whose products
+// are the 12 adjoints (the 10 of ray_adjoints; fa = 2 wz_a x_a, fb = 2 wz_b x_b), and the step's
+// X and phases; the bottom interface comes with everything but g zero.
 #ifdef __CUDACC__
 #pragma nv_exec_check_disable
 #endif
@@ -438,13 +438,14 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
       Ray x, z;
       ray_step(sg[s - s0], coef[i], g, x, z);
       const Ray wz = {w * z.a, w * z.b};
-      sink.ray(i, g, x, wz);
+      sink.ray(i, g, x, wz, sg[s - s0], ea, eb);
       g.a = ea * z.a;
       g.b = eb * z.b;
     }
   }
-  const Ray none = {mk(0.0, 0.0), mk(0.0, 0.0)};
-  sink.ray(I - 1, g, none, none);  // bottom interface I-1 initialises RRd = Rd
+  const cd zero = mk(0.0, 0.0);
+  const Ray none = {zero, zero};
+  sink.ray(I - 1, g, none, none, S3{zero, zero, zero}, zero, zero);  // bottom interface I-1 initialises RRd = Rd
 }
 
 // The same with the products formed: per step sink.step(i, cbar, fa, fb).
@@ -453,7 +454,7 @@ struct RayProducts {
   Sink& sink;
   KR_HD cd reflectivity(cd R) { return sink.reflectivity(R); }
   KR_HD void top(cd f0) { sink.top(f0); }
-  KR_HD void ray(int i, const Ray& g, const Ray& x, const Ray& wz) {
+  KR_HD void ray(int i, const Ray& g, const Ray& x, const Ray& wz, const S3&, cd, cd) {
     cd cbar[10];
     ray_adjoints(g, x, cbar);
     sink.step(i, cbar, 2.0 * (wz.a * x.a), 2.0 * (wz.b * x.b));

@@ -168,7 +168,7 @@ struct RaySumSink {
       acc[(size_t)I * kRayRow + 1] += f0.y;
     }
   }
-  __device__ void ray(int i, Ray g, Ray x, Ray wz) {
+  __device__ void ray(int i, Ray g, Ray x, Ray wz, const S3&, cd, cd) {
     if (!valid) g = x = wz = Ray{mk(0.0, 0.0), mk(0.0, 0.0)};  // a lane without a frequency
     ray_add(g, x, wz, stage, acc + (size_t)i * kRayRow);
   }

@@ -28,6 +28,7 @@
 #include "kr_adjsum.cuh"
 #include "kr_internal.cuh"
 #include "kr_phase.cuh"
+#include "kr_prep.cuh"
 
 namespace kr {
 
@@ -63,55 +64,6 @@ static DerivWs deriv_ws(void* base, int L, int n_p, size_t n_blocks) {
   off = a256(off + sizeof(double) * n_blocks * (size_t)(4 * L + 1));
   w.bytes = off;
   return w;
-}
-
-// One block per (slowness, chunk of kPrepThreads interface items): the layer terms and
-// derivative factors of the chunk's layers go to shared memory, then one thread per
-// (interface, item): items 0..5 form one tangent column each, item 6 the interface's
-// coefficients and the workspace copy of its upper layer (and of the half-space, for the last
-// interface), so no lane of a warp waits on another's extra work.  The coefficients read the
-// layer terms back from shared memory after a barrier, as the forward kernel's prologue
-// does, so they round exactly as there (R bit-identical across entry points).
-constexpr int kPrepThreads = 128;
-constexpr int kPrepItems = 7;                                  // per interface
-constexpr int kPrepLayers = kPrepThreads / kPrepItems + 3;     // layers one chunk touches
-
-__global__ void __launch_bounds__(kPrepThreads)
-deriv_prep_kernel(const double* __restrict__ tab, int L, const double* __restrict__ p,
-                  int n_chunks, LayerP* lay, LayerD* dlay, Iface* coef, ScatTan* tan) {
-  __shared__ LayerP s_lp[kPrepLayers];
-  __shared__ LayerD s_ld[kPrepLayers];
-  const int I = L - 1;
-  const int j = blockIdx.x / n_chunks;
-  const int t0 = (blockIdx.x % n_chunks) * kPrepThreads;
-  const int t1 = min(t0 + kPrepThreads, kPrepItems * I);
-  const int l0 = t0 / kPrepItems, l1 = (t1 - 1) / kPrepItems + 1;  // the chunk's layers
-  const double pj = p[j];
-  for (int l = l0 + threadIdx.x; l <= l1; l += blockDim.x) {
-    const LayerP lp = layer_terms(tab, L, l, pj);
-    s_lp[l - l0] = lp;
-    s_ld[l - l0] = layer_derivs(tab, L, l, pj, lp);
-  }
-  __syncthreads();
-  const int t = t0 + threadIdx.x;
-  if (t >= t1) return;
-  const int i = t / kPrepItems, item = t % kPrepItems;
-  const size_t idx = (size_t)j * I + i, e = (size_t)j * L + i;
-  const LayerP& up = s_lp[i - l0];
-  const LayerP& lo = s_lp[i + 1 - l0];
-  if (item == 6) {
-    lay[e] = up;
-    dlay[e] = s_ld[i - l0];
-    if (i == I - 1) {
-      lay[e + 1] = lo;
-      dlay[e + 1] = s_ld[i + 1 - l0];
-    }
-    coef[idx] = interface_coeffs(pj, i, up, lo);
-    return;
-  }
-  cd c[10];
-  interface_tangent_col(pj, i, up, s_ld[i - l0], lo, s_ld[i + 1 - l0], item, c);
-  for (int k = 0; k < 10; ++k) tan[idx].t[k][item] = c[k];
 }
 
 // The same preparation in two kernels, for the frequency-sum sweep, which needs the

@@ -24,6 +24,7 @@ __all__ = [
     "misfit_gradient",
     "vjp",
     "misfit_hvp",
+    "misfit_hessian",
     "jacobian_dot",
     "table_from_tensors",
     "stream_handle",
@@ -288,6 +289,36 @@ def misfit_hvp(layers: torch.Tensor, p, omega, R_obs, V, free_surface: bool = Fa
                              ws.data_ptr(), ws_bytes, stream_handle(dev))
         _lib.check(st, "kr_misfit_hvp")
     return out
+
+
+def misfit_hessian(layers: torch.Tensor, p, omega, R_obs, free_surface: bool = False):
+    """Exact Hessian of chi = sum |R - R_obs|^2 over the packed sub-ocean parameters
+    [4N - 1, 4N - 1] (alpha, beta, rho of layers 1..N, h of layers 1..N-1), float64 on the
+    device: ``kr_misfit_hessian``, or ``kr_misfit_hvp`` along every axis for models too deep for
+    it."""
+    dev = layers.device
+    L = layers.shape[1]
+    n = 4 * (L - 1)
+    p_t = _dev_f64(p, dev).reshape(-1)
+    w_t = _dev_c128(omega, dev).reshape(-1)
+    n_p, n_w = p_t.numel(), w_t.numel()
+    Ro = _dev_c128(R_obs, dev).reshape(n_p, n_w).contiguous()
+    h = _lib.lib()
+    ws_bytes = h.kr_misfit_hessian_workspace_bytes(L, n_p, n_w)
+    if ws_bytes == 0 and n_p > 0 and n_w > 0:
+        idx = torch.as_tensor([k * L + l for k in range(4) for l in range(1, L)][:n - 1], device=dev)
+        V = torch.zeros((n - 1, 4 * L), dtype=torch.float64, device=dev)
+        V[torch.arange(n - 1, device=dev), idx] = 1.0
+        H = misfit_hvp(layers, p_t, w_t, Ro, V, free_surface)[:, idx]
+        return 0.5 * (H + H.T)
+    ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
+    H = torch.empty((n, n), dtype=torch.float64, device=dev)
+    flags = _lib.KR_FREE_SURFACE if free_surface else 0
+    st = h.kr_misfit_hessian(layers.data_ptr(), L, p_t.data_ptr(), n_p, w_t.data_ptr(), n_w, flags,
+                             Ro.data_ptr(), H.data_ptr(), ws.data_ptr(), ws_bytes,
+                             stream_handle(dev))
+    _lib.check(st, "kr_misfit_hessian")
+    return H[:n - 1, :n - 1]
 
 
 def jacobian_dot(layers: torch.Tensor, p, omega, V, free_surface: bool = False):

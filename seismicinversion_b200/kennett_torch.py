@@ -385,10 +385,9 @@ def hessian(alpha, beta, rho, thickness, Q_alpha, Q_beta, p: float, omega, R_obs
             free_surface: bool = False) -> torch.Tensor:
     """Hessian of chi = ||R - R_obs||^2 over the packed parameters (``kennett_torch.py:644-684``).
 
-    Exact: column j is H e_j from the tangent-of-adjoint kernel (``kr_misfit_hvp``, all
-    columns in one launch; forward-mode dual numbers through the adjoint, no step size), the
-    second derivative the reference's torch.func.hessian takes by reverse over reverse.
-    Returned on ``omega``'s device as float64 (n_params, n_params), symmetrised.
+    Exact, with no step size: the second derivatives the reference's torch.func.hessian takes by
+    reverse over reverse, formed pair by pair of layers (``kr_misfit_hessian``).
+    Returned on ``omega``'s device as float64 (n_params, n_params).
     """
     from .taup_inversion import _Problem
 

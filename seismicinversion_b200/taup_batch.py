@@ -6,9 +6,8 @@
 stop on ||g|| < tol or relative misfit change < tol) in lockstep.  Per iteration:
 
 * the misfit gradients of all K current points are one batched adjoint launch
-  (``kr_batch_launch``); the exact Hessian (``hessian="exact"``) is one tangent-of-adjoint
-  launch per inversion (``kr_misfit_hvp``, every packed direction at once), the Gauss-Newton
-  Hessian 2 Re(J^H J) one ``kr_jacobian`` launch per inversion;
+  (``kr_batch_launch``); the exact Hessian (``hessian="exact"``) is one ``kr_misfit_hessian``
+  per inversion, the Gauss-Newton Hessian 2 Re(J^H J) one ``kr_jacobian`` launch per inversion;
 * the log transform, the damping initialisation, the K damped (H + lambda I) solves
   (batched ``torch.linalg.solve``), the trial points and their layer tables are device
   tensor operations;
@@ -127,9 +126,6 @@ def invert_taup_batch(true_models: list[LayerModel], p_values, nfreq: int = 64,
     owner_f = torch.arange(K, device=dev)
     nv = 4 * L + 1
 
-    basis = torch.zeros((P, 4 * L), dtype=_F, device=dev)
-    basis[torch.arange(P), torch.as_tensor(idx)] = 1.0
-
     def grad_and_hessian(x_phys):
         gbatch.layers.view(-1, 6, L).copy_(tables(x_phys, owner_g))
         gbatch.launch()
@@ -139,10 +135,8 @@ def invert_taup_batch(true_models: list[LayerModel], p_values, nfreq: int = 64,
         tabs = tables(x_phys, owner_f)
         H = torch.empty((K, P, P), dtype=_F, device=dev)
         for k in range(K):
-            if exact:  # H e_j for every packed j: one tangent-of-adjoint launch
-                HV = D.misfit_hvp(tabs[k].contiguous(), p_t, w_c, R_obs[k], basis)
-                Hk = HV[:, idx]
-                H[k] = 0.5 * (Hk + Hk.T)
+            if exact:
+                H[k] = D.misfit_hessian(tabs[k].contiguous(), p_t, w_c, R_obs[k])
             else:
                 _, J = D.jacobian(tabs[k].contiguous(), p_t, w_c, want_R=False)
                 Jp = J[:, idx, :]

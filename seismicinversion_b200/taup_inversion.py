@@ -8,8 +8,8 @@ all slownesses are one launch of the adjoint kernel (``kr_misfit_gradient``) ins
 per-slowness autograd pass, and the Hessian is either
 
 * ``hessian="exact"`` (default): the exact Hessian, as the reference's
-  ``torch.func.hessian`` gives it, from one launch of the tangent-of-adjoint kernel
-  (``kr_misfit_hvp``: H e_j for every packed parameter j, no step size); or
+  ``torch.func.hessian`` gives it, pair by pair of layers from one forward and one reverse
+  sweep per slowness and frequency (``kr_misfit_hessian``, no step size); or
 * ``hessian="gauss-newton"``: 2 Re(J^H J) from one ``kr_jacobian`` launch.
 
 The LaTeX / TikZ / plotting writers of the reference module are presentation, not compute,
@@ -113,11 +113,9 @@ class _Problem:
         return V
 
     def hessian_exact(self, phys: np.ndarray) -> np.ndarray:
-        """The exact Hessian over the packed parameters: H e_j for every j from one launch of
-        the tangent-of-adjoint kernel (kr_misfit_hvp), symmetrised."""
-        HV = D.misfit_hvp(self.table(phys), self.p, self.omega, self.R_obs, self.basis(), self.fs)
-        H = HV[:, self.idx].cpu().numpy()
-        return 0.5 * (H + H.T)
+        """The exact Hessian over the packed parameters (kr_misfit_hessian)."""
+        return D.misfit_hessian(self.table(phys), self.p, self.omega, self.R_obs,
+                                self.fs).cpu().numpy()
 
     def hessian_fd(self, phys: np.ndarray, step: float = 1e-5, stencil: int = 2) -> np.ndarray:
         """Central differences of the exact adjoint gradient, all perturbed models in one
