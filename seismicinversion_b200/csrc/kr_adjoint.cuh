@@ -139,7 +139,8 @@ struct Ray {
   cd a, b;
 };
 
-KR_HD void ray_step(const S3& X, const IfaceT<cd>& f, const Ray& g, Ray& x, Ray& z) {
+template <class F>  // any holder of the interface's td and ru
+KR_HD void ray_step(const S3& X, const F& f, const Ray& g, Ray& x, Ray& z) {
   const cd y1 = cdot2(f.td11, g.a, f.td12, g.b), y2 = cdot2(f.td21, g.a, f.td22, g.b);
   x.a = cdot2(X.a, y1, X.b, y2);
   x.b = cdot2(X.b, y1, X.d, y2);

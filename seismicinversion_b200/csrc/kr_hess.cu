@@ -14,7 +14,9 @@
 // Replaces torch.func.hessian of the reference's tau-p misfit (taup_inversion.py:177,
 // kennett_torch.py:644-684).
 //
-// 64 slownesses x 1024 frequencies x 21 layers (79 parameters): 21.3 ms by directions.
+// 64 slownesses x 1024 frequencies x 21 layers (79 parameters): 20.1 ms by directions, here
+// 0.10 ms for the rays, 0.79 ms for the pairs (38k FP64 instructions per warp and 32 frequencies;
+// eight warps an SM at 255 registers leave the FP64 pipe 35 % busy) and 0.08 ms for the rest.
 #include "kr_adjsum.cuh"
 #include "kr_hess.cuh"
 #include "kr_internal.cuh"
@@ -144,17 +146,26 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
 // layer; dx: a ring of nine layers, as only the next one up reads it), and after a barrier runs
 // its own column of pairs: itself, the layer below, and, with its g^(k) carried down in
 // registers, every deeper layer.  Each pair's 16 entries are summed over the half-warp's
-// frequencies through a padded tile.  16 frequencies per block: two blocks of a 21-layer model
-// fit an SM (108 KB each), so one's near stage covers the other's barrier.
+// frequencies through a padded tile and added to the block's row of partial sums by reductions
+// that nothing waits for (a load, an add and a store per pair stalled each pair on L2).  The
+// round's tangents and coefficients (nine interfaces) are staged in the tiles' memory, which the
+// pairs need only later: read through L1, of which two blocks leave 12 KB, they missed.
+// 16 frequencies per block: two blocks of a 21-layer model fit an SM (108 KB each), so one's
+// near stage covers the other's barrier.
 constexpr int kPairFreq = 16;
 constexpr int kPairGroups = kHessThreads / kPairFreq;  // layers per round
 constexpr int kPubVals = 16;                           // w 8, G 4, A 4
 constexpr int kDxSlots = kPairGroups + 1;
 constexpr int kTileRow = 10;                           // doubles per frequency, 8 used
 
+// Interfaces a round of layers touches, and where their data sits in the tiles' memory.
+constexpr int kRoundIfaces = kPairGroups + 1;
+constexpr size_t kTileBytes = sizeof(double) * kPairGroups * kPairFreq * kTileRow;
+static_assert(kRoundIfaces * (sizeof(ScatTan) + sizeof(HessIface)) <= kTileBytes,
+              "a round's tangents and coefficients fit the tiles");
+
 static size_t hess_pairs_smem(int L) {
-  return sizeof(cd) * kPairFreq * ((size_t)kPubVals * (L - 1) + 8 * kDxSlots) +
-         sizeof(double) * kPairGroups * kPairFreq * kTileRow;
+  return sizeof(cd) * kPairFreq * ((size_t)kPubVals * (L - 1) + 8 * kDxSlots) + kTileBytes;
 }
 // Layers whose published values fit a block's shared memory (50).
 constexpr size_t kHessSmemMax = 227 * 1024;
@@ -196,8 +207,9 @@ __global__ void __launch_bounds__(kHessThreads, 2)
 hess_pairs_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wc, int n_chunks,
                   const LayerD* __restrict__ dlay_all, const Iface* __restrict__ coef_all,
                   const ScatTan* __restrict__ tan_all, const double2* __restrict__ steps,
-                  const double2* __restrict__ seeds, int p0, int accumulate,
-                  double* __restrict__ partial) {
+                  const double2* __restrict__ seeds, int p0, double* __restrict__ partial) {
+  // the curvature kernel does not read this one's results: it may start when there is room
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(16) cd s_pub[];  // [I][kPubVals][16], [kDxSlots][8][16], tiles
   const int I = L - 1;
   cd* s_dx = s_pub + (size_t)I * kPubVals * kPairFreq;
@@ -208,7 +220,6 @@ hess_pairs_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wc, i
   double* part = partial + (size_t)blockIdx.x * (I * (I + 1) / 2) * 16;
   const cd zero = mk(0.0, 0.0);
   for (int chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x) {
-    const bool add = accumulate != 0 || chunk != (int)blockIdx.x;
     const int jp = chunk / n_wc, ip = p0 + jp;
     const int iw = (chunk % n_wc) * kPairFreq + q;
     const bool valid = iw < n_w;
@@ -233,15 +244,27 @@ hess_pairs_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wc, i
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const double s = half_sum8(v + 8 * half, tile, mask);
-        if (q < 8) {
-          double* d = dst + 8 * half + q;
-          *d = add ? *d + s : s;
-        }
+        // one block and one lane per address, in program order: a fixed order of additions
+        if (q < 8) atomicAdd(dst + 8 * half + q, s);
       }
     };
-    for (int base = I; base >= 1; base -= kPairGroups) {
-      const int l = base - h;
+    // the first (deepest) round takes the remainder, where columns are shortest: a round lasts as
+    // long as its longest column
+    const int first = (I - 1) % kPairGroups + 1;
+    for (int base = I, size = first; base >= 1; base -= size, size = kPairGroups) {
+      const int l = h < size ? base - h : 0;
       HessOwn own;
+      // interfaces i0 .. i0 + kRoundIfaces - 1 of the round's layers (those that exist)
+      const int i0 = base - size, ni = min(base, I - 1) - i0 + 1;
+      ScatTan* s_tan = reinterpret_cast<ScatTan*>(s_tile);
+      HessIface* s_if = reinterpret_cast<HessIface*>(s_tan + kRoundIfaces);
+      copy16(s_tan, tan_all + (size_t)ip * I + i0, sizeof(ScatTan) * ni);
+      for (int e = threadIdx.x; e < 7 * ni; e += kHessThreads) {
+        const int i = e / 7, c = e - 7 * i;  // ru11 .. td22 are entries 3 .. 9 of an Iface
+        reinterpret_cast<cd*>(s_if + i)[c] =
+            reinterpret_cast<const cd*>(coef_all + (size_t)ip * I + i0 + i)[3 + c];
+      }
+      __syncthreads();
       if (l >= 1) {
         HessStep lo, up;
         const bool full = l <= I - 1;
@@ -262,12 +285,17 @@ hess_pairs_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wc, i
         up.K = S3{zero, zero, zero};
         SmemPublisher pub{s_pub + (size_t)(l - 1) * kPubVals * kPairFreq + q,
                           s_dx + (l % kDxSlots) * 8 * kPairFreq + q};
-        const Iface* coef = coef_all + (size_t)ip * I;
-        const ScatTan* tan = tan_all + (size_t)ip * I;
-        hess_layer(l, I, w, seed, zeta, lo, up, coef[l - 1], coef[u], tan[l - 1], tan[u],
-                   dlay_all[(size_t)ip * L + l], pub, own);
+        hess_layer(l, I, w, seed, zeta, lo, up, s_if[l - 1 - i0], s_if[u - i0], s_tan[l - 1 - i0],
+                   s_tan[u - i0], dlay_all[(size_t)ip * L + l], pub, own);
       }
       __syncthreads();
+      if (valid && base - size - h >= 1) {
+        // the next round's steps, towards L2 while the pairs run
+        const double2* nx = st + (size_t)(base - size - h - 1) * kStepVals * n_w;
+#pragma unroll
+        for (int c = 0; c < kStepVals; ++c)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + (size_t)c * n_w));
+      }
       if (l >= 1) {
         double v[16];
 #pragma unroll
@@ -321,28 +349,34 @@ hess_curvature_kernel(const double* __restrict__ tab, int L, const double* __res
                       const cd* __restrict__ sums, double* __restrict__ out) {
   const int I = L - 1;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n_p * I * kHessItems) return;
-  const int item = (int)(t % kHessItems);
-  const size_t idx = t / kHessItems;
-  const int ip = (int)(idx / I), i = (int)(idx % I);
-  cd S[kSumVals];
-  const cd* src = sums + ((size_t)ip * n_wtiles * I + i) * kSumVals;
-  for (int k = 0; k < kSumVals; ++k) S[k] = src[k];
-  for (int u = 1; u < n_wtiles; ++u)
-    for (int k = 0; k < kSumVals; ++k) S[k] = S[k] + src[(size_t)u * I * kSumVals + k];
-  const LayerP* lp = lay + (size_t)ip * L;
-  const LayerD* ld = dlay + (size_t)ip * L;
-  LayerD2 d2[2];
-  for (int k = 0; k < 2; ++k) d2[k] = layer_derivs2(tab, L, i + k, lp[i + k], ld[i + k]);
-  out[t] = hess_curvature(tab, L, i, p[ip], lp, ld, d2, S, item);
+  if (t < (size_t)n_p * I * kHessItems) {
+    const int item = (int)(t % kHessItems);
+    const size_t idx = t / kHessItems;
+    const int ip = (int)(idx / I), i = (int)(idx % I);
+    cd S[kSumVals];
+    const cd* src = sums + ((size_t)ip * n_wtiles * I + i) * kSumVals;
+    for (int k = 0; k < kSumVals; ++k) S[k] = src[k];
+    for (int u = 1; u < n_wtiles; ++u)
+      for (int k = 0; k < kSumVals; ++k) S[k] = S[k] + src[(size_t)u * I * kSumVals + k];
+    const LayerP* lp = lay + (size_t)ip * L;
+    const LayerD* ld = dlay + (size_t)ip * L;
+    LayerD2 d2[2];
+    for (int k = 0; k < 2; ++k) d2[k] = layer_derivs2(tab, L, i + k, lp[i + k], ld[i + k]);
+    out[t] = hess_curvature(tab, L, i, p[ip], lp, ld, d2, S, item);
+  }
+  // launched as the pair kernel's programmatic dependent, to fill the SMs as its blocks finish:
+  // complete only after it, so that the assembly finds both
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Entry (l, j, m, k), m <= l, of the lower triangle: rows of `partial`, plus the curvature terms
-// of the interface(s) and phase the two parameters share.  32 entries x 8 row groups per block.
-__global__ void __launch_bounds__(256)
+// of the interface(s) and phase the two parameters share.  32 entries x 32 row groups per block:
+// each thread's loads are a serial chain through L2.
+constexpr int kAsmGroups = 32;
+__global__ void __launch_bounds__(32 * kAsmGroups)
 hess_assemble_kernel(int I, const double* __restrict__ partial, int n_rows, int n_p,
                      const double* __restrict__ curv, double* __restrict__ H) {
-  __shared__ double s[8][33];
+  __shared__ double s[kAsmGroups][33];
   const int n_ent = I * (I + 1) / 2 * 16;
   const int e = blockIdx.x * 32 + (threadIdx.x & 31), grp = threadIdx.x >> 5;
   double t = 0.0;
@@ -353,7 +387,7 @@ hess_assemble_kernel(int I, const double* __restrict__ partial, int n_rows, int 
     m = pair - l * (l - 1) / 2 + 1;
     j = (e >> 2) & 3;
     k = e & 3;
-    for (int r = grp; r < n_rows; r += 8) t += partial[(size_t)r * n_ent + e];
+    for (int r = grp; r < n_rows; r += kAsmGroups) t += partial[(size_t)r * n_ent + e];
     int item[3] = {-1, -1, -1}, at[3] = {0, 0, 0};
     auto sym = [](int a, int b) { return a >= b ? a * (a + 1) / 2 + b : b * (b + 1) / 2 + a; };
     if (l == m && k <= j) {
@@ -373,13 +407,13 @@ hess_assemble_kernel(int I, const double* __restrict__ partial, int n_rows, int 
     }
     for (int c = 0; c < 3; ++c)
       if (item[c] >= 0)
-        for (int r = grp; r < n_p; r += 8)
+        for (int r = grp; r < n_p; r += kAsmGroups)
           t += curv[((size_t)r * I + at[c]) * kHessItems + item[c]];
   }
   s[grp][threadIdx.x & 31] = t;
   __syncthreads();
   if (grp != 0 || e >= n_ent || (l == m && k > j)) return;
-  for (int r = 1; r < 8; ++r) t += s[r][threadIdx.x];
+  for (int r = 1; r < kAsmGroups; ++r) t += s[r][threadIdx.x];
   const int n = 4 * I, row = j * I + l - 1, col = k * I + m - 1;
   H[(size_t)row * n + col] = t;
   H[(size_t)col * n + row] = t;
@@ -387,7 +421,7 @@ hess_assemble_kernel(int I, const double* __restrict__ partial, int n_rows, int 
 
 static size_t a256s(size_t x) { return (x + 255) & ~(size_t)255; }
 
-constexpr int kHessRows = 148 * 4;  // blocks of the pair kernel, hence rows of partial sums
+constexpr int kHessRows = 148 * 2;  // resident blocks of the pair kernel, hence rows of partial sums
 
 struct HessWs {
   LayerP* lay;
@@ -487,6 +521,12 @@ extern "C" kr_status kr_misfit_hessian(const double* layers, int32_t n_layers, c
   }
   const int seg = checkpoint_spacing(I > 1 ? I - 1 : 1);
   const int rows = n_wc * (long long)w.turn < kHessRows ? n_wc * w.turn : kHessRows;
+  const int n_ent = I * (I + 1) / 2 * 16;
+  const cudaError_t me = cudaMemsetAsync(w.partial, 0, sizeof(double) * n_ent * (size_t)rows, st);
+  if (me != cudaSuccess) {
+    set_last_error("kr_misfit_hessian: memset", me);
+    return KR_ERR_CUDA;
+  }
   for (int p0 = 0; p0 < n_p; p0 += w.turn) {
     const int np = n_p - p0 < w.turn ? n_p - p0 : w.turn;
     hess_rays_kernel<<<(unsigned)(np * n_wtiles), kHessThreads, rs, st>>>(
@@ -496,17 +536,27 @@ extern "C" kr_status kr_misfit_hessian(const double* layers, int32_t n_layers, c
     if (s != KR_OK) return s;
     const int chunks = np * n_wc;
     hess_pairs_kernel<<<(unsigned)(chunks < rows ? chunks : rows), kHessThreads, ps, st>>>(
-        L, w2, n_w, n_wc, chunks, w.dlay, w.coef, w.tan, w.steps, w.seeds, p0, p0 > 0 ? 1 : 0,
-        w.partial);
+        L, w2, n_w, n_wc, chunks, w.dlay, w.coef, w.tan, w.steps, w.seeds, p0, w.partial);
     s = check_launch("kr_misfit_hessian: pairs");
     if (s != KR_OK) return s;
   }
-  hess_curvature_kernel<<<(unsigned)((n_curv + 127) / 128), 128, 0, st>>>(
-      layers, L, p, n_p, n_wtiles, w.lay, w.dlay, w.sums, w.curv);
-  s = check_launch("kr_misfit_hessian: curvature");
-  if (s != KR_OK) return s;
-  const int n_ent = I * (I + 1) / 2 * 16;
-  hess_assemble_kernel<<<(unsigned)((n_ent + 31) / 32), 256, 0, st>>>(I, w.partial, rows, n_p,
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3((unsigned)((n_curv + 127) / 128));
+  lc.blockDim = dim3(128);
+  lc.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = 1;
+  const cudaError_t ce = cudaLaunchKernelEx(&lc, hess_curvature_kernel, layers, L, p, n_p, n_wtiles,
+                                            (const LayerP*)w.lay, (const LayerD*)w.dlay,
+                                            (const cd*)w.sums, w.curv);
+  if (ce != cudaSuccess) {
+    set_last_error("kr_misfit_hessian: curvature", ce);
+    return KR_ERR_CUDA;
+  }
+  hess_assemble_kernel<<<(unsigned)((n_ent + 31) / 32), 32 * kAsmGroups, 0, st>>>(I, w.partial, rows, n_p,
                                                                       w.curv, H);
   return check_launch("kr_misfit_hessian: assemble");
 }

@@ -44,12 +44,19 @@ KR_HD Ray zero_ray() { return Ray{mk(0.0, 0.0), mk(0.0, 0.0)}; }
 KR_HD Ray sym_mac(const Ray& y, cd a, cd b, cd d, const Ray& v) {
   return Ray{cmac(cmac(y.a, a, v.a), b, v.b), cmac(cmac(y.b, b, v.a), d, v.b)};
 }
-KR_HD Ray td_mac(const Ray& y, const IfaceT<cd>& f, const Ray& v) {
+template <class F>
+KR_HD Ray td_mac(const Ray& y, const F& f, const Ray& v) {
   return Ray{cmac(cmac(y.a, f.td11, v.a), f.td12, v.b), cmac(cmac(y.b, f.td21, v.a), f.td22, v.b)};
 }
-KR_HD Ray tdt_mac(const Ray& y, const IfaceT<cd>& f, const Ray& v) {
+template <class F>
+KR_HD Ray tdt_mac(const Ray& y, const F& f, const Ray& v) {
   return Ray{cmac(cmac(y.a, f.td11, v.a), f.td21, v.b), cmac(cmac(y.b, f.td12, v.a), f.td22, v.b)};
 }
+
+// The coefficients of an interface that these formulas read.
+struct HessIface {
+  cd ru11, ru12, ru22, td11, td12, td21, td22;
+};
 
 // What the ray sweep leaves of step i (interface i): X, the phases of layer i + 1, g and K.
 struct HessStep {
@@ -60,7 +67,8 @@ struct HessStep {
 };
 
 // E (I + Ru X) v of a step.
-KR_HD Ray step_down(const S3& X, cd ea, cd eb, const IfaceT<cd>& f, const Ray& v) {
+template <class F>
+KR_HD Ray step_down(const S3& X, cd ea, cd eb, const F& f, const Ray& v) {
   const Ray u = sym_mac(v, f.ru11, f.ru12, f.ru22, sym_mac(zero_ray(), X.a, X.b, X.d, v));
   return Ray{ea * u.a, eb * u.b};
 }
@@ -122,9 +130,9 @@ struct HessOwn {
 #ifdef __CUDACC__
 #pragma nv_exec_check_disable
 #endif
-template <class Pub>
+template <class Pub, class F>
 KR_HD void hess_layer(int l, int I, cd w, cd seed, cd zeta, const HessStep& lo, const HessStep& up,
-                      const Iface& flo, const Iface& fup, const ScatTan& tlo, const ScatTan& tup,
+                      const F& flo, const F& fup, const ScatTan& tlo, const ScatTan& tup,
                       const LayerD& d, Pub& pub, HessOwn& own) {
   const bool low_full = l <= I - 1;  // step l - 1 is a Kennett step, not the bottom interface
   const bool has_up = l <= I - 1, up_full = l <= I - 2;
@@ -145,16 +153,21 @@ KR_HD void hess_layer(int l, int I, cd w, cd seed, cd zeta, const HessStep& lo, 
       tangent_rays(tlo, 3 + j, lo.g, x, low_full, a, b);
       if (has_up) tangent_rays(tup, j, up.g, xu, up_full, au, bu);
     }
-    cd da = zero, db = zero;  // dl = omega d(i eta h) / d theta, likewise neta
-    if (j == 0) da = w * d.ca_alpha;
-    if (j == 1) db = w * d.cb_beta;
-    if (j == 3) {
-      da = w * d.ca_h;
-      db = w * d.cb_h;
+    // dl = omega d(i eta h) / d theta, likewise neta: alpha and h act on the first, beta and h on
+    // the second (all zero in the half-space)
+    const bool in_a = j == 0 || j == 3, in_b = j == 1 || j == 3;
+    cd da = zero, db = zero;
+    Ray c = zero_ray();
+    if (in_a) {
+      da = w * (j == 0 ? d.ca_alpha : d.ca_h);
+      c.a = da * x.a;
+      b.a = cmac(b.a, da, z.a);
     }
-    if (!low_full) da = db = zero;
-    b.a = cmac(b.a, da, z.a);
-    b.b = cmac(b.b, db, z.b);
+    if (in_b) {
+      db = w * (j == 1 ? d.cb_beta : d.cb_h);
+      c.b = db * x.b;
+      b.b = cmac(b.b, db, z.b);
+    }
     Ray q = zero_ray(), dx = zero_ray(), e = zero_ray(), xb = zero_ray();
     if (low_full) {
       Ray ug = au;
@@ -162,7 +175,8 @@ KR_HD void hess_layer(int l, int I, cd w, cd seed, cd zeta, const HessStep& lo, 
         xb = sym_mac(zero_ray(), up.X.a, up.X.b, up.X.d, bu);
         ug = tdt_mac(ug, fup, xb);
       }
-      q = Ray{cmac(da * x.a, lo.ea, ug.a), cmac(db * x.b, lo.eb, ug.b)};
+      q = c;
+      if (j < 3) q = Ray{cmac(c.a, lo.ea, ug.a), cmac(c.b, lo.eb, ug.b)};
       dx = sym_mac(q, lo.X.a, lo.X.b, lo.X.d, sym_mac(b, flo.ru11, flo.ru12, flo.ru22, q));
       e = sym_mac(b, flo.ru11, flo.ru12, flo.ru22, dx);
     }
@@ -199,7 +213,8 @@ KR_HD void hess_layer(int l, int I, cd w, cd seed, cd zeta, const HessStep& lo, 
 #endif
     for (int k = 0; k <= j; ++k) {
       cd s = dot2(b, dxs[k]) + dot2(q, es[k]) + dot2(tg, kts[k]);
-      if (j != 2 && k != 2) s = s - ((da * das[k]) * xza + (db * dbs[k]) * xzb);
+      if (in_a && (k == 0 || k == 3)) s = cmac(s, -(da * das[k]), xza);
+      if (in_b && (k == 1 || k == 3)) s = cmac(s, -(db * dbs[k]), xzb);
       if (j < 3) s = s + dot2(bu, xbu[k]);
       const cd v = seed2 * s;
       const cd u = A * own.J[k];
