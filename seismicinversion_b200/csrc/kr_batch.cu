@@ -239,7 +239,7 @@ __device__ __forceinline__ void forward_item(const ItemRec& item, const kr_model
   const int passes = n_tiles >= 2 * (THREADS / 32) ? kPasses : 1, parts = kPasses / passes;
   for (int t = threadIdx.x >> 5; t < n_tiles * parts; t += THREADS / 32) {
     const int q = t / parts, pass = (t - q * parts) * passes;
-    sweep_tile<NPH, F>(om, NPH > 0 ? tiles.w0[q] : make_double2(0.0, 0.0), u0 + q, pass,
+    sweep_tile<KennettForm, NPH, F>(om, NPH > 0 ? tiles.w0[q] : make_double2(0.0, 0.0), u0 + q, pass,
                        pass + passes, item.w0, item.w0 + item.nw, L, lay, coef, tab,
                        NPH > 0 && ok && tiles.off[q] == 0, hm, (d.flags & KR_FREE_SURFACE) != 0,
                        Rp);

@@ -1,5 +1,6 @@
-// Global Matrix Method reflectivity with the block-Riccati sweep: an independent FP64
-// evaluation of R(omega, p) behind the same boundary as kr_reflectivity.
+// Global Matrix Method reflectivity with the block-Riccati sweep: an FP64 evaluation of
+// R(omega, p) from the layers' eigenvectors and the continuity of displacement and traction,
+// without reflection / transmission coefficients, behind the same boundary as kr_reflectivity.
 //
 // Follows tmnestor/SeismicInversion, GlobalMatrix/:
 //   layer eigenvectors     layer_matrix.py:201-258 (E_d, E_u 4x2; ocean e_d, e_u)
@@ -8,256 +9,145 @@
 //   ocean extraction       riccati_solver.py:297-330
 //   entry point            gmm_torch.py:229-305 (R / (1 + R) with the free surface)
 //
-// One thread per (omega, p), one slowness per block (the layout of reflectivity_kernel):
-// the block prologue puts the layer terms, the eigenvector terms of every layer and the
-// phase table in shared memory.  The 4x4 complex systems are solved by Gaussian elimination
-// with partial pivoting on |Re| + |Im| (the pivot rule of the LAPACK solve the reference
-// calls), fully unrolled so that row exchanges are register selects, not indexed memory.
-#include <stdlib.h>
-
-#include "kr_phase.cuh"
+// The 4x4 systems do not depend on omega but through Z = diag(ph) Y of the layer below, so they
+// are solved once per (slowness, interface): with E = [E_d E_u] of each layer,
+//     [diag(ph_k); Y_k] = Q [I; Z_k+1] D,   Q = E_k^-1 E_k+1 (4x4),
+// hence Y_k diag(ph_k)^-1 = (Q21 + Q22 Z)(Q11 + Q12 Z)^-1 and Z_k = diag(ph_k) (that) diag(ph_k).
+// E^-1 is in closed form: in sums s = d + u and differences t = d - u of the amplitudes the rows
+// decouple into (s_P, t_S) and (t_P, s_S), 2x2 blocks of determinants rho nu and rho eta.
+// Per (omega, p, interface) that leaves two 2x2 products, one 2x2 inverse and one more product:
+// ~156 FP64 operations where the pivoted elimination of the 4x4 system took ~600 (943
+// instructions); 1024 x 1023 of a 21-layer model 949 -> 278 us.
+#include "kr_forward.cuh"
 
 namespace kr {
 
-constexpr int kGmmThreads = 128;
-static_assert(kGmmThreads == kPhTile, "one tile is one phase-table tile");
-
-// Eigenvector terms of one solid layer (p real):
-//   E_d = [[p, neta], [eta, -p], [-gamma, a], [b, gamma]],
-//   E_u = [[p, -neta], [-eta, -p], [-gamma, -a], [-b, gamma]],
-// gamma = rho (1 - 2 beta_c^2 p^2), a = 2 mu p neta, b = 2 mu p eta, mu = rho beta_c^2.
-struct LayerG {
-  cd eta, neta, gamma, a, b;
+// Interface k >= 1: Q up to a factor per interface (it cancels in the quotient), row by row.
+// Interface 0 (ocean bottom): the eigenvector terms of layer 1, the ocean's eta and density, p.
+struct GmmCoef {
+  cd q11[4], q12[4], q21[4], q22[4];
 };
 
-KR_HD LayerG gmm_layer(const LayerP& lp, double p) {
-  const cd cp = mk(p, 0.0);
-  const cd crho = mk(lp.rho, 0.0);
-  const cd mu = (crho * lp.betac) * lp.betac;
-  LayerG g;
-  g.eta = lp.eta;
-  g.neta = lp.neta;
-  g.gamma = crho * (1.0 - ((2.0 * lp.betac) * lp.betac) * cp * cp);
-  g.a = ((2.0 * mu) * cp) * lp.neta;
-  g.b = ((2.0 * mu) * cp) * lp.eta;
-  return g;
-}
-
-__device__ __forceinline__ void e_down(const LayerG& g, double p, cd E[4][2]) {
-  E[0][0] = mk(p, 0.0);
-  E[0][1] = g.neta;
-  E[1][0] = g.eta;
-  E[1][1] = mk(-p, 0.0);
-  E[2][0] = -g.gamma;
-  E[2][1] = g.a;
-  E[3][0] = g.b;
-  E[3][1] = g.gamma;
-}
-
-__device__ __forceinline__ void e_up(const LayerG& g, double p, cd E[4][2]) {
-  E[0][0] = mk(p, 0.0);
-  E[0][1] = -g.neta;
-  E[1][0] = -g.eta;
-  E[1][1] = mk(-p, 0.0);
-  E[2][0] = -g.gamma;
-  E[2][1] = -g.a;
-  E[3][0] = -g.b;
-  E[3][1] = g.gamma;
-}
-
-KR_HD double cabs1(cd z) { return fabs(z.x) + fabs(z.y); }
-
-__device__ __forceinline__ void swap_rows(cd (&A)[4][4], cd (&B)[4][2], int c, int piv) {
-  // rows c and piv (piv >= c); compile-time indices only
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    if (r <= c) continue;
-    const bool s = (piv == r);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const cd t = A[c][j];
-      A[c][j] = s ? A[r][j] : t;
-      A[r][j] = s ? t : A[r][j];
-    }
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const cd t = B[c][j];
-      B[c][j] = s ? B[r][j] : t;
-      B[r][j] = s ? t : B[r][j];
-    }
+static __device__ __noinline__ void gmm_store(double p, int k, const LayerP* lay, GmmCoef* out) {
+  const LayerP& u = lay[k];
+  const LayerP& l = lay[k + 1];
+  const cd mul = l.rho * (l.betac * l.betac);
+  GmmCoef o;
+  if (k == 0) {
+    // E_d = [[p, neta], [eta, -p], [-gamma, a], [b, gamma]], E_u with eta and neta negated
+    const cd gamma = l.rho - (2.0 * p * p) * mul;
+    o.q11[0] = u.eta;
+    o.q11[1] = mk(u.rho, p);
+    o.q11[2] = l.eta;
+    o.q11[3] = gamma;
+    o.q12[0] = (2.0 * p) * (mul * l.neta);
+    o.q12[1] = (2.0 * p) * (mul * l.eta);
+    o.q12[2] = o.q12[3] = mk(0.0, 0.0);
+    for (int e = 0; e < 4; ++e) o.q21[e] = o.q22[e] = mk(0.0, 0.0);
+    *out = o;
+    return;
   }
+  const cd d = 2.0 * (mul - u.rho * (u.betac * u.betac));
+  const cd pd = (p * p) * d;
+  const cd a = (l.rho - u.rho) - pd, b = l.rho - pd, c = u.rho + pd;
+  const cd ie = recip(u.eta), in = recip(u.neta);
+  const cd cp = (c * l.eta) * ie, cs = (c * l.neta) * in;   // c eta2 / eta1, c neta2 / neta1
+  const cd ap = p * (a * ie), as = p * (a * in);            // p a / eta1, p a / neta1
+  const cd dn = p * (d * l.neta), de = p * (d * l.eta);     // p d neta2, p d eta2
+  o.q11[0] = b + cp;  o.q11[1] = ap - dn;  o.q11[2] = de - as;     o.q11[3] = b + cs;
+  o.q12[0] = b - cp;  o.q12[1] = ap + dn;  o.q12[2] = -(de + as);  o.q12[3] = b - cs;
+  o.q21[0] = b - cp;  o.q21[1] = -(ap + dn);  o.q21[2] = de + as;  o.q21[3] = b - cs;
+  o.q22[0] = b + cp;  o.q22[1] = dn - ap;  o.q22[2] = as - de;     o.q22[3] = b + cs;
+  *out = o;
 }
 
-// Solves A X = B (4x4, two right-hand sides) in place: on return B holds X.
-__device__ __forceinline__ void solve4x2(cd (&A)[4][4], cd (&B)[4][2]) {
-  cd inv[4];
+// s + M Z for 2x2 matrices given row by row.
+__device__ __forceinline__ void mac22(const cd s[4], const cd m[4], const cd z[4], cd o[4]) {
+  o[0] = cmac(cmac(s[0], m[0], z[0]), m[1], z[2]);
+  o[1] = cmac(cmac(s[1], m[0], z[1]), m[1], z[3]);
+  o[2] = cmac(cmac(s[2], m[2], z[0]), m[3], z[2]);
+  o[3] = cmac(cmac(s[3], m[2], z[1]), m[3], z[3]);
+}
+// A B^-1
+__device__ __forceinline__ void div22(const cd a[4], const cd b[4], cd y[4]) {
+  const cd id = recip_near(cdot2(b[0], b[3], -b[1], b[2]));
+  y[0] = cdot2(a[0], b[3], -a[1], b[2]) * id;
+  y[1] = cdot2(a[1], b[0], -a[0], b[1]) * id;
+  y[2] = cdot2(a[2], b[3], -a[3], b[2]) * id;
+  y[3] = cdot2(a[3], b[0], -a[2], b[1]) * id;
+}
+
+struct GmmForm {
+  typedef GmmCoef Coef;
+  static __device__ __forceinline__ void store(double p, int i, const LayerP* lay,
+                                               const LayerRoots*, Coef* out) {
+    gmm_store(p, i, lay, out);
+  }
+  template <int F, class Ph>
+  static __device__ __forceinline__ void sweep(int n_layers, const Coef* coef, const Ph& ph,
+                                               bool fs, cd R[F]) {
+    const int M = n_layers - 2;  // interfaces M .. 1 between solids
+    cd P[F], Q[F], S[F], E[F];
+    cd y[F][4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    int piv = c;
-    double best = cabs1(A[c][c]);
+    for (int f = 0; f < F; ++f)
 #pragma unroll
-    for (int r = c + 1; r < 4; ++r) {
-      const double m = cabs1(A[r][c]);
-      if (m > best) {
-        best = m;
-        piv = r;
+      for (int e = 0; e < 4; ++e) y[f][e] = mk(0.0, 0.0);
+    if (M >= 1) {  // nothing comes back from the half-space
+      cd y0[4];
+      div22(coef[M].q21, coef[M].q11, y0);
+#pragma unroll
+      for (int f = 0; f < F; ++f)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[f][e] = y0[e];
+    }
+#pragma unroll 1
+    for (int k = M - 1; k >= 1; --k) {
+      ph.pqs(k + 1, P, Q, S);
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const cd z[4] = {P[f] * y[f][0], S[f] * y[f][1], S[f] * y[f][2], Q[f] * y[f][3]};
+        cd a[4], b[4];
+        mac22(coef[k].q21, coef[k].q22, z, a);
+        mac22(coef[k].q11, coef[k].q12, z, b);
+        div22(a, b, y[f]);
       }
     }
-    swap_rows(A, B, c, piv);
-    inv[c] = recip(A[c][c]);
+    if (M >= 1) ph.pqs(1, P, Q, S);
+    ph.ocean(E);
+    // ocean bottom: layer 1's displacement and traction rows [u_z], [sigma], [tau] of
+    // E_d + E_u Z; tau = 0 and continuity of u_z and sigma with e_d = (eta0, -rho0),
+    // e_u = (-eta0, -rho0)
+    const GmmCoef& o = coef[0];
+    const cd eta0 = o.q11[0], eta = o.q11[2], gamma = o.q11[3], ea = o.q12[0], eb = o.q12[1];
+    const double rho0 = o.q11[1].x, p = o.q11[1].y;
 #pragma unroll
-    for (int r = c + 1; r < 4; ++r) {
-      const cd l = A[r][c] * inv[c];
+    for (int f = 0; f < F; ++f) {
+      cd z[4];
 #pragma unroll
-      for (int j = c + 1; j < 4; ++j) A[r][j] = cmac(A[r][j], -l, A[c][j]);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) B[r][j] = cmac(B[r][j], -l, B[c][j]);
-    }
-  }
-#pragma unroll
-  for (int c = 3; c >= 0; --c) {
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      cd s = B[c][j];
-#pragma unroll
-      for (int k = c + 1; k < 4; ++k) s = cmac(s, -A[c][k], B[k][j]);
-      B[c][j] = s * inv[c];
-    }
-  }
-}
-
-// Riccati sweep for one (omega, p); returns R without the free-surface operator.
-template <class Ph>
-__device__ __forceinline__ cd gmm_sweep(int L, double p, const LayerG* g, const Ph& ph,
-                                        double rho0) {
-  const int M = L - 2;
-  cd Y[2][2] = {{mk(0.0, 0.0), mk(0.0, 0.0)}, {mk(0.0, 0.0), mk(0.0, 0.0)}};
-  for (int k = M; k >= 1; --k) {
-    // E_eff of the layer below interface k
-    cd Ee[4][2];
-    e_down(g[k + 1], p, Ee);
-    if (k < M) {
-      cd Eu[4][2];
-      e_up(g[k + 1], p, Eu);
-      const cd pa = ph.a(k + 1), pb = ph.b(k + 1);
-      const cd Z00 = pa * Y[0][0], Z01 = pa * Y[0][1], Z10 = pb * Y[1][0], Z11 = pb * Y[1][1];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        Ee[r][0] = cmac2(Ee[r][0], Eu[r][0], Z00, Eu[r][1], Z10);
-        Ee[r][1] = cmac2(Ee[r][1], Eu[r][0], Z01, Eu[r][1], Z11);
+      for (int e = 0; e < 4; ++e) z[e] = mk(0.0, 0.0);
+      if (M >= 1) {
+        z[0] = P[f] * y[f][0];
+        z[1] = S[f] * y[f][1];
+        z[2] = S[f] * y[f][2];
+        z[3] = Q[f] * y[f][3];
       }
-    }
-    // F = [E_u(k) | -E_eff], right-hand side -E_d(k) diag(ph(k))
-    cd F[4][4], B[4][2];
-    {
-      cd Eu[4][2], Ed[4][2];
-      e_up(g[k], p, Eu);
-      e_down(g[k], p, Ed);
-      const cd pa = ph.a(k), pb = ph.b(k);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        F[r][0] = Eu[r][0];
-        F[r][1] = Eu[r][1];
-        F[r][2] = -Ee[r][0];
-        F[r][3] = -Ee[r][1];
-        B[r][0] = -(Ed[r][0] * pa);
-        B[r][1] = -(Ed[r][1] * pb);
-      }
-    }
-    solve4x2(F, B);
-    Y[0][0] = B[0][0];
-    Y[0][1] = B[0][1];
-    Y[1][0] = B[1][0];
-    Y[1][1] = B[1][1];
-  }
-  // ocean extraction at the ocean bottom
-  cd E1[4][2];
-  e_down(g[1], p, E1);
-  if (M >= 1) {
-    cd Eu[4][2];
-    e_up(g[1], p, Eu);
-    const cd pa = ph.a(1), pb = ph.b(1);
-    const cd Z00 = pa * Y[0][0], Z01 = pa * Y[0][1], Z10 = pb * Y[1][0], Z11 = pb * Y[1][1];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      E1[r][0] = cmac2(E1[r][0], Eu[r][0], Z00, Eu[r][1], Z10);
-      E1[r][1] = cmac2(E1[r][1], Eu[r][0], Z01, Eu[r][1], Z11);
+      // rows 1 (u_z), 2 (sigma), 3 (tau) of E_d + E_u Z
+      const cd u0 = cmac(eta, -eta, z[0]) - p * z[2], u1 = cmac(mk(-p, 0.0), -eta, z[1]) - p * z[3];
+      const cd s0 = cmac(cmac(-gamma, -gamma, z[0]), -ea, z[2]);
+      const cd s1 = cmac(cmac(ea, -gamma, z[1]), -ea, z[3]);
+      const cd t0 = cmac(cmac(eb, -eb, z[0]), gamma, z[2]);
+      const cd t1 = cmac(cmac(gamma, -eb, z[1]), gamma, z[3]);
+      // D = (t1, -t0) up to a factor makes the traction vanish; eliminating the factor from
+      // u_z = eta0 (1 - r), sigma = -rho0 (1 + r) (amplitudes at the ocean bottom) gives r
+      const cd uz = cdot2(u0, t1, -u1, t0), sg = cdot2(s0, t1, -s1, t0);
+      const cd en = eta0 * sg, ru = rho0 * uz;
+      const cd r = (en + ru) * recip_near(en - ru);
+      const cd v = E[f] * r;
+      R[f] = fs ? v * recip(1.0 + v) : v;
     }
   }
-  const cd eta0 = g[0].eta;
-  const cd e0 = ph.a(0);
-  const cd crho = mk(rho0, 0.0);
-  // e_d = (eta0, -rho0), e_u = (-eta0, -rho0)
-  const cd eu0 = -eta0, eu1 = -crho, ed0 = eta0, ed1 = -crho;
-  cd m00 = cdot2(eu0, E1[2][0], -eu1, E1[1][0]);
-  cd m01 = cdot2(eu0, E1[2][1], -eu1, E1[1][1]);
-  cd m10 = E1[3][0], m11 = E1[3][1];
-  cd r0 = cdot2(eu0, ed1, -eu1, ed0) * e0, r1 = mk(0.0, 0.0);
-  // 2x2 solve with partial pivoting
-  if (cabs1(m10) > cabs1(m00)) {
-    cd t = m00; m00 = m10; m10 = t;
-    t = m01; m01 = m11; m11 = t;
-    t = r0; r0 = r1; r1 = t;
-  }
-  const cd i00 = recip(m00);
-  const cd l = m10 * i00;
-  const cd u11 = cmac(m11, -l, m01);
-  const cd y1 = cmac(r1, -l, r0);
-  const cd d1 = y1 * recip(u11);
-  const cd d0 = cmac(r0, -m01, d1) * i00;
-  const cd uz = cdot2(E1[1][0], d0, E1[1][1], d1);
-  const cd U0 = cmac(uz, -ed0, e0) * recip(eu0);
-  return e0 * U0;
-}
-
-constexpr int kGmmTabTiles = 16;
-
-// Shared memory: LayerP[L], LayerG[L], phase table (when the model tabulates).
-static size_t gmm_smem(int L, bool table) {
-  return sizeof(LayerP) * (size_t)L + sizeof(LayerG) * (size_t)L +
-         (table ? phase_table_bytes(L, kGmmTabTiles) : 0);
-}
-
-// Four blocks of 128 threads per SM (128 registers): 13.34 ms on the 21-layer gather grid
-// against 13.47 at the compiler's 134 registers (three blocks) and 13.59 at five (96).
-__global__ void __launch_bounds__(kGmmThreads, 4)
-gmm_kernel(const double* __restrict__ tab, int L, const double* __restrict__ p, int n_p,
-           const double2* __restrict__ omega, int n_w, int n_wtiles, int tiles_per_block,
-           int free_surface, int use_table, double2* __restrict__ R) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ unsigned s_bad;
-  LayerP* s_layer = reinterpret_cast<LayerP*>(smem);
-  LayerG* s_g = reinterpret_cast<LayerG*>(smem + sizeof(LayerP) * L);
-  cd* s_ph = reinterpret_cast<cd*>(smem + sizeof(LayerP) * L + sizeof(LayerG) * L);
-  const int groups = (n_wtiles + tiles_per_block - 1) / tiles_per_block;
-  const int ip = blockIdx.x / groups;
-  const int t0 = (blockIdx.x % groups) * tiles_per_block;
-  const int t1 = min(n_wtiles, t0 + tiles_per_block);
-  const double pj = p[ip];
-  for (int l = threadIdx.x; l < L; l += blockDim.x) {
-    const LayerP lp = layer_terms(tab, L, l, pj);
-    s_layer[l] = lp;
-    s_g[l] = gmm_layer(lp, pj);
-  }
-  __syncthreads();
-  unsigned mask = 0u;
-  const int entries = phase_entries(kGmmTabTiles);
-  if (use_table)
-    mask = build_phase_table(omega, n_w, grid_line(omega, n_w), t0, t1 - t0, entries, L,
-                             s_layer, s_ph, &s_bad);
-  const double rho0 = s_layer[0].rho;
-  double2* Rp = R + (size_t)ip * n_w;
-  for (int t = t0; t < t1; ++t) {
-    const int iw = t * kGmmThreads + threadIdx.x;
-    if (iw >= n_w) break;
-    const double2 wv = omega[iw];
-    const PhaseAuto ph{((mask >> (t - t0)) & 1u) != 0, phase_at(s_ph, entries, iw, t0),
-                       PhaseDirect{mk(wv.x, wv.y), s_layer}};
-    cd r = gmm_sweep(L, pj, s_g, ph, rho0);
-    if (free_surface) r = r * recip(1.0 + r);
-    Rp[iw] = make_double2(r.x, r.y);
-  }
-}
+};
 
 }  // namespace kr
 
@@ -272,25 +162,17 @@ extern "C" kr_status kr_gmm_reflectivity(const double* layers, int32_t n_layers,
   if (n_p == 0 || n_w == 0) return KR_OK;
   if (!layers || !p || !omega || !R) return KR_ERR_INVALID_ARGUMENT;
   if (!aligned16(omega) || !aligned16(R)) return KR_ERR_INVALID_ARGUMENT;
-  const int n_wtiles = (n_w + kGmmThreads - 1) / kGmmThreads;
-  // tiles per block: enough slownesses x tile groups for ~8 waves, at most kGmmTabTiles
-  long long tpb = ((long long)n_p * n_wtiles) / (148LL * 4 * 8);
-  if (tpb < 1) tpb = 1;
-  if (tpb > kGmmTabTiles) tpb = kGmmTabTiles;
-  if (tpb > n_wtiles) tpb = n_wtiles;
-  const long long blocks = (long long)n_p * ((n_wtiles + tpb - 1) / tpb);
-  if (blocks > 0x7fffffffLL) return KR_ERR_TOO_LARGE;
-  const bool table = phase_table_model(n_layers);
-  const size_t smem = gmm_smem(n_layers, table);
   cudaStream_t st = (cudaStream_t)stream;
-  static SmemLimit lim;
-  if (smem > 48 * 1024) {
-    const kr_status a = raise_smem_limit((const void*)gmm_kernel, smem, lim,
-                                         "kr_gmm_reflectivity: smem attribute");
-    if (a != KR_OK) return a;
+  constexpr const char* kWhat = "kr_gmm_reflectivity";
+  switch (sweep_phases(n_layers)) {
+    case 0:
+      return launch_forward<GmmForm, 0, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
+                                                 R, st);
+    case 2:
+      return launch_forward<GmmForm, 2, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
+                                                 R, st);
+    default:
+      return launch_forward<GmmForm, 3, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
+                                                 R, st);
   }
-  gmm_kernel<<<(unsigned)blocks, kGmmThreads, smem, st>>>(
-      layers, n_layers, p, n_p, reinterpret_cast<const double2*>(omega), n_w, n_wtiles, (int)tpb,
-      (flags & KR_FREE_SURFACE) ? 1 : 0, table ? 1 : 0, reinterpret_cast<double2*>(R));
-  return check_launch("kr_gmm_reflectivity");
 }

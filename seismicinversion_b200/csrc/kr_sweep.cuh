@@ -1,5 +1,6 @@
 // The forward sweep of one slowness over a uniform frequency grid, warp by warp, shared by the
-// per-model and the batched forward kernels (so that both give the same bits).
+// per-model and the batched forward kernels (so that both give the same bits) and, with its own
+// form of the recursion, by the global-matrix kernel.
 //
 // What bounds it is the FP64 pipe: ~115 FP64 instructions per (omega, p, interface) in
 // kennett_step_x when the squared and mixed phase factors P = ea^2, Q = eb^2, S = ea eb come
@@ -131,36 +132,44 @@ struct SweepDirect {
   }
 };
 
-// The upward sweep of F frequencies: R at the surface.
-template <int F, class Ph>
-__device__ __forceinline__ void sweep_frequencies(int n_layers, const Iface* coef, const Ph& ph,
-                                                  bool fs, cd R[F]) {
-  const int I = n_layers - 1;
-  M2 r[F];
-#pragma unroll
-  for (int f = 0; f < F; ++f) {
-    r[f].a = coef[I - 1].rd11;
-    r[f].b = coef[I - 1].rd12;
-    r[f].d = coef[I - 1].rd22;
+// The Kennett recursion as a form of the sweep: its interface coefficients, formed once per
+// (slowness, interface), and the upward sweep of F frequencies, giving R at the surface.
+struct KennettForm {
+  typedef Iface Coef;
+  static __device__ __forceinline__ void store(double p, int i, const LayerP* lay,
+                                               const LayerRoots* roots, Coef* out) {
+    interface_store(p, i, lay, roots, out);
   }
-  cd P[F], Q[F], S[F], rpp[F], E[F];
-#pragma unroll 1
-  for (int i = I - 2; i >= 1; --i) {
-    ph.pqs(i + 1, P, Q, S);
+  template <int F, class Ph>
+  static __device__ __forceinline__ void sweep(int n_layers, const Coef* coef, const Ph& ph,
+                                               bool fs, cd R[F]) {
+    const int I = n_layers - 1;
+    M2 r[F];
 #pragma unroll
     for (int f = 0; f < F; ++f) {
-      cd x11, x12, x22;
-      r[f] = kennett_step_x(r[f], P[f], Q[f], S[f], coef[i], x11, x12, x22);
+      r[f].a = coef[I - 1].rd11;
+      r[f].b = coef[I - 1].rd12;
+      r[f].d = coef[I - 1].rd22;
+    }
+    cd P[F], Q[F], S[F], rpp[F], E[F];
+#pragma unroll 1
+    for (int i = I - 2; i >= 1; --i) {
+      ph.pqs(i + 1, P, Q, S);
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        cd x11, x12, x22;
+        r[f] = kennett_step_x(r[f], P[f], Q[f], S[f], coef[i], x11, x12, x22);
+      }
+    }
+    if (I > 1) ph.pqs(1, P, Q, S);
+    ph.ocean(E);
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      rpp[f] = I > 1 ? kennett_last_step_pp(r[f], P[f], Q[f], S[f], coef[0]) : r[f].a;
+      R[f] = pp_surface2(rpp[f], E[f], fs);
     }
   }
-  if (I > 1) ph.pqs(1, P, Q, S);
-  ph.ocean(E);
-#pragma unroll
-  for (int f = 0; f < F; ++f) {
-    rpp[f] = I > 1 ? kennett_last_step_pp(r[f], P[f], Q[f], S[f], coef[0]) : r[f].a;
-    R[f] = pp_surface2(rpp[f], E[f], fs);
-  }
-}
+};
 
 // The two kinds of sweep out of line, so that the hot loop's registers are its own: inlined
 // next to the exponentials and the task bookkeeping it spilled inside the loop.
@@ -168,17 +177,18 @@ template <int F>
 struct SweepOut {
   cd R[F];
 };
-template <int NPH, int F>
-__device__ __noinline__ SweepOut<F> sweep_table(int n_layers, const Iface* coef, const cd* lo,
-                                                const cd* hm, bool fs) {
+template <class Form, int NPH, int F>
+__device__ __noinline__ SweepOut<F> sweep_table(int n_layers, const typename Form::Coef* coef,
+                                                const cd* lo, const cd* hm, bool fs) {
   SweepOut<F> o;
-  sweep_frequencies<F>(n_layers, coef, SweepTable<NPH, F>{lo, hm}, fs, o.R);
+  Form::template sweep<F>(n_layers, coef, SweepTable<NPH, F>{lo, hm}, fs, o.R);
   return o;
 }
-static __device__ __noinline__ cd sweep_direct(int n_layers, const Iface* coef, const LayerP* lay,
-                                               cd w, bool fs) {
+template <class Form>
+__device__ __noinline__ cd sweep_direct(int n_layers, const typename Form::Coef* coef,
+                                        const LayerP* lay, cd w, bool fs) {
   cd R[1];
-  sweep_frequencies<1>(n_layers, coef, SweepDirect{w, lay}, fs, R);
+  Form::template sweep<1>(n_layers, coef, SweepDirect{w, lay}, fs, R);
   return R[0];
 }
 
@@ -211,11 +221,11 @@ __device__ __forceinline__ void sweep_tiles_check(const double2* __restrict__ om
 // 128 u + 32 F q), frequencies outside [k_lo, k_hi) skipped.  `w0`: the tile's first frequency;
 // `use`: whether the tile and the slowness's lo / mid entries `tab` may be used (NPH > 0); hm:
 // the warp's scratch.  The tile's hi entries are evaluated once and stay in registers.
-template <int NPH, int F>
+template <class Form, int NPH, int F>
 __device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, double2 w0, int u,
                                            int pass0, int pass1, int k_lo, int k_hi, int n_layers,
-                                           const LayerP* lay, const Iface* coef, const cd* tab,
-                                           bool use, cd* hm, bool fs, double2* __restrict__ Rp) {
+                                           const LayerP* lay, const typename Form::Coef* coef,
+                                           const cd* tab, bool use, cd* hm, bool fs, double2* __restrict__ Rp) {
   const int lane = threadIdx.x & 31;
   constexpr int N = NPH > 0 ? NPH : 1;
   constexpr int kHi = NPH == 3 ? (3 * (kPqsLayers - 1) + 31) / 32 : (2 * (kPairLayers - 1) + 31) / 32;
@@ -247,8 +257,8 @@ __device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, do
         }
       }
       __syncwarp();
-      const SweepOut<F> o = sweep_table<N, F>(n_layers, coef, tab + (lane & (kPhLo - 1)),
-                                              hm + (lane >> 4), fs);
+      const SweepOut<F> o = sweep_table<Form, N, F>(n_layers, coef, tab + (lane & (kPhLo - 1)),
+                                                    hm + (lane >> 4), fs);
 #pragma unroll
       for (int f = 0; f < F; ++f) {
         const int k = kb + 32 * f + lane;
@@ -261,7 +271,7 @@ __device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, do
       const int k = kb + 32 * f + lane;
       if (k < k_lo || k >= k_hi) continue;
       const double2 wv = omega[k];
-      const cd R = sweep_direct(n_layers, coef, lay, mk(wv.x, wv.y), fs);
+      const cd R = sweep_direct<Form>(n_layers, coef, lay, mk(wv.x, wv.y), fs);
       Rp[k] = make_double2(R.x, R.y);
     }
   }
