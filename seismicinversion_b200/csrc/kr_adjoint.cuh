@@ -190,24 +190,24 @@ KR_HD Acc acc_zero() {
   return z;
 }
 // s += x y (complex), or s += Re(x y) (real: 2 FP64 operations instead of 4)
-KR_HD void acc_add(cd& s, cd x, cd y) { s = s + x * y; }
+KR_HD void acc_add(cd& s, cd x, cd y) { s = cmac(s, x, y); }
 KR_HD void acc_add(double& s, cd x, cd y) { s = fma(x.x, y.x, fma(-x.y, y.y, s)); }
 
-// Adds the coefficient-tangent contractions of one interface to its upper / lower layer.
-template <class AccT>
-KR_HD void contract(const ScatTan& t, const cd cbar[10], AccT& up, AccT& lo) {
-  decltype(up.a) s[6];
-  for (int j = 0; j < 6; ++j) set_zero(s[j]);
-  for (int k = 0; k < 10; ++k) {
-    if (cbar[k].x == 0.0 && cbar[k].y == 0.0) continue;
-    for (int j = 0; j < 6; ++j) acc_add(s[j], cbar[k], t.t[k][j]);
+// Adds the coefficient-tangent contractions of one interface to its upper / lower layer, over
+// its first N coefficients (10; 3, Rd alone, at the bottom interface).
+template <int N, class AccT>
+KR_HD void contract(const ScatTan& t, const cd cbar[N], AccT& up, AccT& lo) {
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int k = 0; k < N; ++k) {
+    acc_add(up.a, cbar[k], t.t[k][0]);
+    acc_add(up.b, cbar[k], t.t[k][1]);
+    acc_add(up.r, cbar[k], t.t[k][2]);
+    acc_add(lo.a, cbar[k], t.t[k][3]);
+    acc_add(lo.b, cbar[k], t.t[k][4]);
+    acc_add(lo.r, cbar[k], t.t[k][5]);
   }
-  up.a = up.a + s[0];
-  up.b = up.b + s[1];
-  up.r = up.r + s[2];
-  lo.a = lo.a + s[3];
-  lo.b = lo.b + s[4];
-  lo.r = lo.r + s[5];
 }
 
 // Tape of one (omega, p) pair, in local memory: up to kSegMax steps of X (the three entries of
@@ -251,7 +251,6 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
   const int I = L - 1;
   const int nsteps = I - 1;  // step s applies interface i = I - 2 - s
   const int ncp = nsteps > 0 ? (nsteps + seg - 1) / seg : 0;
-  const int top0 = (ncp - 1) * seg;  // first step of the top segment (reversed first)
   S3 cp[kCpMax];
   S3 sg[kSegMax];
   cd sea[kSegMax], seb[kSegMax];
@@ -259,17 +258,21 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
   // kept on the tape, as in adjoint_pair_sums
   const bool keep_ph = !ph.cheap();
   M2 r = m2(coef[I - 1].rd11, coef[I - 1].rd12, coef[I - 1].rd12, coef[I - 1].rd22);
-  for (int s = 0; s < nsteps; ++s) {
-    if (s % seg == 0) cp[s / seg] = s3(r);
-    const int i = I - 2 - s;
-    const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
-    S3 x;
-    r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
-    if (s >= top0) {  // the top segment is recorded now and never recomputed
-      sg[s - top0] = x;
-      if (keep_ph) {
-        sea[s - top0] = ea;
-        seb[s - top0] = eb;
+  for (int q = 0; q < ncp; ++q) {
+    cp[q] = s3(r);
+    const int s0 = q * seg, s1 = s0 + seg < nsteps ? s0 + seg : nsteps;
+    const bool top = q == ncp - 1;  // the top segment is recorded now and never recomputed
+    for (int s = s0; s < s1; ++s) {
+      const int i = I - 2 - s;
+      const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
+      S3 x;
+      r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
+      if (top) {
+        sg[s - s0] = x;
+        if (keep_ph) {
+          sea[s - s0] = ea;
+          seb[s - s0] = eb;
+        }
       }
     }
   }
@@ -320,7 +323,7 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
       ray_step(sg[s - s0], coef[i], g, x, z);
       cd cbar[10];
       ray_adjoints(g, x, cbar);
-      contract(tan[i], cbar, cur, nxt);
+      contract<10>(tan[i], cbar, cur, nxt);
       const LayerD& d = dlay[i + 1];
       const cd w2 = 2.0 * w;
       const cd fa = (z.a * x.a) * w2, fb = (z.b * x.b) * w2;
@@ -336,12 +339,8 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
     }
   }
   // bottom interface I-1 initialises RRd = Rd
-  cd cbar[10];
-  cbar[0] = g.a * g.a;
-  cbar[1] = (2.0 * g.a) * g.b;
-  cbar[2] = g.b * g.b;
-  for (int k = 3; k < 10; ++k) cbar[k] = mk(0.0, 0.0);
-  contract(tan[I - 1], cbar, cur, nxt);
+  const cd rbar[3] = {g.a * g.a, (2.0 * g.a) * g.b, g.b * g.b};
+  contract<3>(tan[I - 1], rbar, cur, nxt);
   sink.layer(I - 1, cur);
   sink.layer(L - 1, nxt);
 }
@@ -382,7 +381,6 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
   const int I = L - 1;
   const int nsteps = I - 1;  // step s applies interface i = I - 2 - s
   const int ncp = nsteps > 0 ? (nsteps + seg - 1) / seg : 0;
-  const int top0 = (ncp - 1) * seg;
   S3 cp[kCpMax];
   S3 sg[kSegMax];
   cd sea[kSegMax], seb[kSegMax];
@@ -390,17 +388,21 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
   // kept on the tape: 48 instead of 80 bytes of local memory per step
   const bool keep_ph = !ph.cheap();
   M2 r = m2(coef[I - 1].rd11, coef[I - 1].rd12, coef[I - 1].rd12, coef[I - 1].rd22);
-  for (int s = 0; s < nsteps; ++s) {
-    if (s % seg == 0) cp[s / seg] = s3(r);
-    const int i = I - 2 - s;
-    const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
-    S3 x;
-    r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
-    if (s >= top0) {
-      sg[s - top0] = x;
-      if (keep_ph) {
-        sea[s - top0] = ea;
-        seb[s - top0] = eb;
+  for (int q = 0; q < ncp; ++q) {
+    cp[q] = s3(r);
+    const int s0 = q * seg, s1 = s0 + seg < nsteps ? s0 + seg : nsteps;
+    const bool top = q == ncp - 1;  // the top segment is recorded now and never recomputed
+    for (int s = s0; s < s1; ++s) {
+      const int i = I - 2 - s;
+      const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
+      S3 x;
+      r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
+      if (top) {
+        sg[s - s0] = x;
+        if (keep_ph) {
+          sea[s - s0] = ea;
+          seb[s - s0] = eb;
+        }
       }
     }
   }

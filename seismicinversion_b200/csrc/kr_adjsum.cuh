@@ -5,8 +5,85 @@
 #pragma once
 
 #include "kr_adjoint.cuh"
+#include "kr_phase.cuh"
+#include "kr_sweep.cuh"
 
 namespace kr {
+
+// ------------------------------------------------------------------------------------------
+// Phase factors ea, eb of one lane for the derivative sweeps, on tiles of the grid's line
+// (kr_phase.cuh): lo[j] = exp(j delta c), j < 16, shared by the block, and, per warp and pass of
+// 32 frequencies from kb, hm[m] = exp(omega_{kb + 16 m} c), m < 2, each one direct exp, so a
+// lookup is one product of two reads at fixed offsets.  The derivatives need ea and eb
+// themselves in the reverse sweep, so these two are tabulated, not P, Q, S.
+//
+// Models of up to kRayTabLayers layers tabulate: a 48-layer block of the batched gradient is
+// 107 KB, two per SM; above, the table would cost a resident block.  Every derivative kernel
+// applies the same rules, so they agree bit for bit.
+// ------------------------------------------------------------------------------------------
+constexpr int kRayTabLayers = 48;
+__host__ __device__ inline bool ray_table_model(int n_layers) { return n_layers <= kRayTabLayers; }
+
+struct RayTable {
+  const cd* lo;  // the lane's lo entry of phase 0 ([2 (L - 1)][16])
+  const cd* hm;  // the lane's hm entry of phase 0 ([2 (L - 1)][2])
+  __device__ __forceinline__ cd a(int l) const { return hm[4 * l] * lo[2 * kPhLo * l]; }
+  __device__ __forceinline__ cd b(int l) const {
+    return hm[4 * l + 2] * lo[2 * kPhLo * l + kPhLo];
+  }
+  __device__ __forceinline__ bool cheap() const { return true; }
+};
+
+__host__ __device__ inline size_t ray_lo_values(int n_layers) {
+  return (size_t)kPhLo * 2 * (n_layers - 1);
+}
+__host__ __device__ inline size_t ray_hm_values(int n_layers) { return 4 * (size_t)(n_layers - 1); }
+__host__ __device__ inline size_t ray_table_bytes(int n_layers, int warps) {
+  return sizeof(cd) * (ray_lo_values(n_layers) + warps * ray_hm_values(n_layers));
+}
+
+// Block-cooperative: the lo entries; returns whether this thread's are usable.  The caller
+// synchronises.
+__device__ __forceinline__ bool ray_lo_fill(const GridLine& g, int n_layers, const LayerP* lay,
+                                            cd* lo) {
+  bool ok = true;
+  for (int e = threadIdx.x; e < 2 * (n_layers - 1) * kPhLo; e += blockDim.x) {
+    const cd v = cexp_(((double)(e % kPhLo) * g.d) * sweep_exponent<2>(lay, e / kPhLo));
+    ok &= phase_usable(v);
+    lo[e] = v;
+  }
+  return ok;
+}
+
+// Warp-cooperative: the hm entries of the pass from frequency kb; returns (warp-uniform) whether
+// all are usable.
+__device__ __forceinline__ bool ray_hm_fill(const double2* __restrict__ omega, int n_w, int kb,
+                                            int n_layers, const LayerP* lay, cd* hm) {
+  bool bad = false;
+  const int lane = threadIdx.x & 31;
+  // lanes take m = lane & 1 of phase id; past the grid's end the entry is not used
+  const double2 w = omega[min(kb + kPhLo * (lane & 1), n_w - 1)];
+  for (int e = lane; e < 4 * (n_layers - 1); e += 32) {
+    const cd v = cexp_(mk(w.x, w.y) * sweep_exponent<2>(lay, e >> 1));
+    bad |= !phase_usable(v);
+    hm[e] = v;
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  __syncwarp();
+  return !bad;
+}
+
+// The lane's table for a warp whose hm entries are at `hm`.
+__device__ __forceinline__ RayTable ray_table(const cd* lo, const cd* hm) {
+  const int lane = threadIdx.x & 31;
+  return RayTable{lo + (lane & (kPhLo - 1)), hm + (lane >> 4)};
+}
+
+// Whether frequency k = w of the grid is on its line.
+__device__ __forceinline__ bool on_line(const GridLine& g, int k, double2 w) {
+  return fabs(w.x - fma((double)k, g.d.x, g.w0.x)) <= g.tol &&
+         fabs(w.y - fma((double)k, g.d.y, g.w0.y)) <= g.tol;
+}
 
 // Staging of the warp sums of 12 explicit values per lane (the dual adjoint of the
 // Hessian-vector products): a padded 32 x 13 tile.  Tile row stride in complex values:
@@ -55,6 +132,14 @@ __device__ __forceinline__ void warp_add12(const cd v[kSumVals], cd* stage, cd* 
 constexpr int kRayStride = 36;
 constexpr int kRayStage = 6 * kRayStride;  // complex values per warp
 constexpr int kRayRow = 24;                // doubles per step and warp
+
+// Bytes of `warps` warps' staging rows, or of the layer terms and roots a block's prologue keeps
+// in their place where those are larger (deep models).
+__host__ __device__ inline size_t ray_stage_bytes(int L, int warps) {
+  const size_t a = sizeof(cd) * kRayStage * (size_t)warps;
+  const size_t b = (sizeof(LayerP) + sizeof(LayerRoots)) * (size_t)L;
+  return a > b ? a : b;
+}
 
 // Shared memory of the ray sums for `warps` warps: per warp L rows and its staging rows.
 __host__ __device__ inline size_t raysum_smem_bytes(int L, int warps) {

@@ -53,7 +53,7 @@ struct PlanHeader {
   int32_t threads, tile_w, grid_fwd, grid_grad;
   int64_t off_models, off_pairs, off_fwd, off_grad, total_bytes;
   int32_t n_fwd_deep, n_grad_deep;  // the lists' leading items, of models deeper than kPqsLayers
-  int32_t counters[4];  // item counters: forward deep / shallow, gradient [2]
+  int32_t counters[4];  // item counters: forward deep / shallow, gradient deep / shallow
 };
 
 __host__ __device__ inline size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -319,20 +319,46 @@ struct BatchGradSink {
   }
 };
 
+// Passes of 32 frequencies of an item: the warp's first pass and its stride are in units of whole
+// warps, so that every pass lies in one tile and its phases come from two hm entries.
+#define KR_FOR_PASSES(kb) \
+  for (int kb = (item.w0 & ~31) + (int)(threadIdx.x & ~31u); kb < item.w0 + item.nw; kb += THREADS)
+
+// The lo entries and tile verdicts of a gradient item; returns whether the lo entries may be
+// used.  Contains block barriers; all threads call it.
+__device__ __forceinline__ bool ray_item_tables(const ItemRec& item, const kr_model_desc& d,
+                                                const double2* om, const LayerP* lay, cd* lo,
+                                                SweepTiles& tiles) {
+  const bool table = ray_table_model(d.n_layers);
+  const int u0 = item.w0 / kPhTile, n = (item.w0 + item.nw - 1) / kPhTile - u0 + 1;
+  if (table) sweep_tiles_clear(tiles, n);
+  __syncthreads();
+  bool ok = table;
+  if (table) {
+    const GridLine g = grid_line(om, d.n_w);
+    sweep_tiles_check(om, d.n_w, g, u0, n, tiles);
+    ok = ray_lo_fill(g, d.n_layers, lay, lo);
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
+// Gradient items of models whose frequency sums exceed shared memory (more than ~118 layers in
+// the batch): the contraction per (omega, p), as deriv_sweep_kernel.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
 batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all,
                       const double2* __restrict__ obs_all, double2* __restrict__ R_all,
-                      double* __restrict__ chi_grad, int stage, int tab_entries) {
-  // [THREADS / 32][4L + 1] accumulators (padded to 16 bytes), then the item's slowness data,
-  // then (tab_entries > 0, models that tabulate) the phase table of the item's tiles
+                      double* __restrict__ chi_grad, int stage) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // [THREADS / 32][4L + 1] accumulators (padded to 16 bytes), then (models that tabulate) the
+  // phase table, then, if `stage`, the item's slowness data
   extern __shared__ __align__(16) double s_wacc[];
-  __shared__ unsigned s_bad;
+  __shared__ SweepTiles s_tiles;
   PlanHeader* h = reinterpret_cast<PlanHeader*>(plan);
   const kr_model_desc* models = reinterpret_cast<const kr_model_desc*>(plan + h->off_models);
   const PairRec* pairs = reinterpret_cast<const PairRec*>(plan + h->off_pairs);
   const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_grad);
-  const int n_items = h->n_grad;
+  const int n_items = h->n_grad_deep;
   __shared__ int s_item;
   ItemFeed feed(&h->counters[2], &s_item);
   for (;;) {
@@ -345,8 +371,10 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
     const int L = d.n_layers;
     const int nv = 4 * L + 1;
     for (int k = threadIdx.x; k < (THREADS / 32) * nv; k += THREADS) s_wacc[k] = 0.0;
+    cd* lo = reinterpret_cast<cd*>(s_wacc + ((THREADS / 32) * nv + 1) / 2 * 2);
+    unsigned char* b = reinterpret_cast<unsigned char*>(lo);
+    if (ray_table_model(L)) b += ray_table_bytes(L, THREADS / 32);
     if (stage) {
-      unsigned char* b = reinterpret_cast<unsigned char*>(s_wacc + ((THREADS / 32) * nv + 1) / 2 * 2);
       ScatTan* st = reinterpret_cast<ScatTan*>(b);
       Iface* sc = reinterpret_cast<Iface*>(b + sizeof(ScatTan) * (L - 1));
       LayerP* sl = reinterpret_cast<LayerP*>(b + (sizeof(ScatTan) + sizeof(Iface)) * (L - 1));
@@ -363,26 +391,16 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
     }
     __syncthreads();
     const double2* om = omega_all + d.omega_off;
-    const int u0 = item.w0 / kPhTile;
-    cd* s_ph = reinterpret_cast<cd*>(
-        reinterpret_cast<unsigned char*>(s_wacc + ((THREADS / 32) * nv + 1) / 2 * 2) +
-        pair_smem_bytes(L));
-    unsigned mask = 0u;
-    if (stage && tab_entries > 0 && phase_table_model(L))
-      mask = build_phase_table(om, d.n_w, grid_line(om, d.n_w), u0,
-                               (item.w0 + item.nw - 1) / kPhTile - u0 + 1, tab_entries, L,
-                               v.lay, s_ph, &s_bad);
+    const bool lo_ok = ray_item_tables(item, d, om, v.lay, lo, s_tiles);
+    cd* hm = lo + ray_lo_values(L) + (threadIdx.x >> 5) * ray_hm_values(L);
     double* row = s_wacc + (threadIdx.x >> 5) * nv;
     const int seg = checkpoint_spacing(L - 2 > 0 ? L - 2 : 1);
     const bool fs = (d.flags & KR_FREE_SURFACE) != 0;
-    for (int k0 = 0; k0 < item.nw; k0 += THREADS) {
-      const int iw = item.w0 + k0 + threadIdx.x;
-      const bool valid = k0 + threadIdx.x < item.nw;
-      cd w = mk(0.0, 0.0);
-      if (valid) {
-        const double2 wv = omega_all[d.omega_off + iw];
-        w = mk(wv.x, wv.y);
-      }
+    KR_FOR_PASSES(kb) {
+      const int iw = kb + (threadIdx.x & 31);
+      const bool valid = iw >= item.w0 && iw < item.w0 + item.nw;
+      const double2 wv = om[min(iw, d.n_w - 1)];
+      const cd w = mk(wv.x, wv.y);
       BatchGradSink<THREADS> sink;
       sink.valid = valid;
       sink.L = L;
@@ -390,10 +408,13 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
       const size_t e = (size_t)pr.j * d.n_w + (valid ? iw : 0);
       sink.obs = obs_all + d.obs_off + e;
       sink.R_out = (d.flags & KR_BATCH_STORE_R) ? R_all + d.R_off + e : nullptr;
-      const int iwt = valid ? iw : item.w0;
-      const PhaseAuto ph{((mask >> (iwt / kPhTile - u0)) & 1u) != 0,
-                         phase_at(s_ph, tab_entries, iwt, u0), PhaseDirect{w, v.lay}};
-      jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan, ph, sink);
+      const bool tab = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0 &&
+                       ray_hm_fill(om, d.n_w, kb, L, v.lay, hm);
+      if (tab)
+        jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan, ray_table(lo, hm), sink);
+      else
+        jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan, PhaseDirect{w, v.lay}, sink);
+      __syncwarp();
       double c2 = valid ? (sink.res.x * sink.res.x + sink.res.y * sink.res.y) : 0.0;
       for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);
       if ((threadIdx.x & 31) == 0) row[4 * L] += c2;
@@ -408,33 +429,32 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
 }
 
 // Gradient items with the contraction moved out of the frequency loop (kr_adjsum.cuh): the
-// block's warps sum the per-step adjoints of every frequency of the item, then contract once
-// per (pair, interface).  Dynamic smem: per-warp sum rows (sized for max_layers) and staging
-// tiles (which then hold the item's [4L] result), then the item's interface coefficients and
-// layer terms and (models that tabulate) the phase table of its tiles.  Register budget: 256 threads per SM
-// (its shared memory admits two 128-thread blocks per SM; a 168-register cap only spills).
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 256 / THREADS)
+// block's warps take the item's passes of 32 frequencies in turn and sum the per-step adjoints
+// into their rows; the block contracts once per (pair, interface).  Dynamic smem, laid out for
+// the item's own model: per-warp sum rows and staging rows (which then hold the item's [4L]
+// result), interface coefficients and layer terms, and (models that tabulate) the phase table.
+// Two depth classes as in the forward kernel: three blocks of 128 threads per SM for models of
+// up to 30 layers (72 KB), two for deeper ones (107 KB).
+template <int THREADS, bool DEEP>
+__global__ void __launch_bounds__(THREADS, (DEEP ? 256 : 384) / THREADS)
 batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_all,
                        const double2* __restrict__ obs_all, double2* __restrict__ R_all,
-                       double* __restrict__ chi_grad, int max_layers, int tab_entries) {
+                       double* __restrict__ chi_grad) {
+  // the other class may fill in as this one's blocks finish
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int W = THREADS / 32;
   extern __shared__ __align__(16) double s_raw[];
-  __shared__ unsigned s_bad;
+  __shared__ SweepTiles s_tiles;
   __shared__ double s_chi[W];
   PlanHeader* h = reinterpret_cast<PlanHeader*>(plan);
   const kr_model_desc* models = reinterpret_cast<const kr_model_desc*>(plan + h->off_models);
   const PairRec* pairs = reinterpret_cast<const PairRec*>(plan + h->off_pairs);
-  const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_grad);
-  const int n_items = h->n_grad;
+  const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_grad) +
+                         (DEEP ? 0 : h->n_grad_deep);
+  const int n_items = DEEP ? h->n_grad_deep : h->n_grad - h->n_grad_deep;
   const int warp = threadIdx.x >> 5;
-  double* acc = s_raw;
-  cd* stage = reinterpret_cast<cd*>(acc + (size_t)W * sum_rows(max_layers) * kRayRow);
-  // the item's [4L] result reuses the staging rows once the sweeps are done
-  double* s_out = reinterpret_cast<double*>(stage);
-  unsigned char* area = reinterpret_cast<unsigned char*>(stage + W * kRayStage);
   __shared__ int s_item;
-  ItemFeed feed(&h->counters[2], &s_item);
+  ItemFeed feed(&h->counters[DEEP ? 2 : 3], &s_item);
   for (;;) {
     const int it = feed.next();
     if (it >= n_items) break;
@@ -443,31 +463,26 @@ batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_al
     const kr_model_desc d = models[pr.model];
     const PairView v = pair_view(plan, pr, d);
     const int L = d.n_layers, I = L - 1;
-    Iface* sc = reinterpret_cast<Iface*>(area);
-    LayerP* sl = reinterpret_cast<LayerP*>(area + sizeof(Iface) * I);
-    cd* s_ph = reinterpret_cast<cd*>(area + prologue_smem_bytes(L));
+    double* acc = s_raw;
+    cd* stage = reinterpret_cast<cd*>(acc + (size_t)W * sum_rows(L) * kRayRow);
+    Iface* sc = reinterpret_cast<Iface*>(stage + W * kRayStage);
+    LayerP* sl = reinterpret_cast<LayerP*>(sc + I);
+    cd* lo = reinterpret_cast<cd*>(sl + L);
+    cd* hm = lo + ray_lo_values(L) + warp * ray_hm_values(L);
     sums_zero(acc, L, W);
     copy16(sc, v.coef, sizeof(Iface) * I);
     copy16(sl, v.lay, sizeof(LayerP) * L);
     __syncthreads();
     const double2* om = omega_all + d.omega_off;
-    const int u0 = item.w0 / kPhTile;
-    unsigned mask = 0u;
-    if (tab_entries > 0 && phase_table_model(L))
-      mask = build_phase_table(om, d.n_w, grid_line(om, d.n_w), u0,
-                               (item.w0 + item.nw - 1) / kPhTile - u0 + 1, tab_entries, L, sl,
-                               s_ph, &s_bad);
+    const bool lo_ok = ray_item_tables(item, d, om, sl, lo, s_tiles);
     const int seg = checkpoint_spacing(L - 2 > 0 ? L - 2 : 1);
     const bool fs = (d.flags & KR_FREE_SURFACE) != 0;
     double c2 = 0.0;
-    for (int k0 = 0; k0 < item.nw; k0 += THREADS) {
-      const int iw = item.w0 + k0 + threadIdx.x;
-      const bool valid = k0 + threadIdx.x < item.nw;
-      cd w = mk(0.0, 0.0);
-      if (valid) {
-        const double2 wv = om[iw];
-        w = mk(wv.x, wv.y);
-      }
+    KR_FOR_PASSES(kb) {
+      const int iw = kb + (threadIdx.x & 31);
+      const bool valid = iw >= item.w0 && iw < item.w0 + item.nw;
+      const double2 wv = om[min(iw, d.n_w - 1)];
+      const cd w = mk(wv.x, wv.y);
       const size_t e = (size_t)pr.j * d.n_w + (valid ? iw : 0);
       RaySumSink sink;
       sink.valid = valid;
@@ -477,14 +492,19 @@ batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_al
       sink.acc = acc + (size_t)warp * sum_rows(L) * kRayRow;
       sink.stage = stage + warp * kRayStage;
       sink.I = I;
-      const int iwt = valid ? iw : item.w0;
-      const PhaseAuto ph{((mask >> (iwt / kPhTile - u0)) & 1u) != 0,
-                         phase_at(s_ph, tab_entries, iwt, u0), PhaseDirect{w, sl}};
-      adjoint_rays(L, w, fs, seg, sc, ph, sink);
+      const bool tab = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0 &&
+                       ray_hm_fill(om, d.n_w, kb, L, sl, hm);
+      if (tab)
+        adjoint_rays(L, w, fs, seg, sc, ray_table(lo, hm), sink);
+      else
+        adjoint_rays(L, w, fs, seg, sc, PhaseDirect{w, sl}, sink);
+      __syncwarp();  // the hm entries are read before the next pass overwrites them
       if (valid) c2 += sink.res.x * sink.res.x + sink.res.y * sink.res.y;
     }
     for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);
     if ((threadIdx.x & 31) == 0) s_chi[warp] = c2;
+    // the item's [4L] result goes where the staging rows were
+    double* s_out = reinterpret_cast<double*>(stage);
     sums_finish(acc, L, W, v.tan, v.dlay, s_out);
     __syncthreads();
     for (int k = threadIdx.x; k < 4 * L; k += THREADS) atomicAdd(chi_grad + d.grad_off + k, s_out[k]);
@@ -494,6 +514,8 @@ batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_al
       atomicAdd(chi_grad + d.grad_off + 4 * L, t);
     }
   }
+  // complete only after the class launched before this one
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 static int occupancy_grid(const void* fn, int threads, size_t smem) {
@@ -578,51 +600,28 @@ static size_t fwd_smem(int threads, int max_layers, bool deep) {
                   prologue_smem_bytes(max_layers));
 }
 
-// Phase-table entries per phase for items of tile_w frequencies (0: direct exponentials for
-// every model).  Only models that tabulate in kr_reflectivity (phase_table_model) use the
-// table, so the smem reserved is that of the largest such model.
-static int fwd_table_entries(int tile_w) {
-  const int tiles = (tile_w + kPhTile - 1) / kPhTile + 1;
-  return tiles > kPhMaxTiles ? 0 : phase_entries(tiles);
-}
-
-// gradient kernel dynamic smem, whether the slowness data is staged, and the phase-table
-// entries (0: none).  The table of a model that tabulates (at most phase_table_max_layers()
-// layers) sits after that model's own staged data, inside the staging area sized for the
-// largest model where it fits.
-static size_t grad_smem(int threads, int max_layers, int tab_entries, int* stage, int* tab) {
+// batch_gradient_kernel's dynamic smem and whether the slowness data is staged.
+static size_t grad_smem(int threads, int max_layers, int* stage) {
   const size_t acc = sizeof(double) * (((size_t)(threads / 32) * (4 * max_layers + 1) + 1) / 2 * 2);
+  const size_t table = ray_table_bytes(std::min(max_layers, kRayTabLayers), threads / 32);
   const size_t pair = pair_smem_bytes(max_layers);
-  *stage = (acc + pair <= kBatchStageMax) ? 1 : 0;
-  *tab = 0;
-  if (!*stage) return acc;
-  size_t area = pair;
-  if (tab_entries > 0) {
-    const int lt = std::min(max_layers, phase_table_max_layers());
-    const size_t need = pair_smem_bytes(lt) + sizeof(cd) * (size_t)tab_entries * 2 * (lt - 1);
-    if (acc + std::max(area, need) <= kBatchStageMax) {
-      area = std::max(area, need);
-      *tab = tab_entries;
-    }
-  }
-  return acc + area;
+  *stage = (acc + table + pair <= kBatchStageMax) ? 1 : 0;
+  return acc + table + (*stage ? pair : 0);
 }
 
-// Dynamic smem of batch_grad_sums_kernel (0 if it does not fit) and the phase-table entries it
-// uses (0: none), for blocks of THREADS threads.
-static size_t sums_smem(int threads, int max_layers, int tab_entries, int* tab) {
-  size_t area = prologue_smem_bytes(max_layers);
-  *tab = 0;
-  if (tab_entries > 0) {
-    const int lt = std::min(max_layers, phase_table_max_layers());
-    area = std::max(area, prologue_smem_bytes(lt) +
-                              sizeof(cd) * (size_t)tab_entries * 2 * (size_t)(lt - 1));
-    *tab = tab_entries;
+// Dynamic smem of batch_grad_sums_kernel for models of up to max_layers (0 if it does not fit):
+// the largest of its models, which need not be the deepest, as only some tabulate.
+static size_t sums_smem(int threads, int max_layers) {
+  const int w = threads / 32;
+  size_t most = 0;
+  for (int L = 2; L <= max_layers; ++L) {
+    const size_t b = raysum_smem_bytes(L, w) + prologue_smem_bytes(L) +
+                     (ray_table_model(L) ? ray_table_bytes(L, w) : 0);
+    most = std::max(most, b);
   }
   // the staging rows hold the item's [4L] result after its sweeps
   if (sizeof(cd) * kRayStage * (threads / 32) < sizeof(double) * 4 * (size_t)max_layers) return 0;
-  const size_t smem = raysum_smem_bytes(max_layers, threads / 32) + area;
-  return smem <= kBatchStageMax ? smem : 0;
+  return most <= kBatchStageMax ? most : 0;
 }
 
 // KR_DERIV_SUMS=0 keeps the per-step contraction for gradient items (comparison runs).
@@ -633,31 +632,6 @@ static bool batch_sums_enabled() {
     v = (e && atoi(e) == 0) ? 0 : 1;
   }
   return v == 1;
-}
-
-template <int THREADS>
-static kr_status grids(PlanHeader& h, int max_layers, int tab_entries, size_t* gsm, int* stage,
-                       int* gtab, bool* sums) {
-  int stab = 0;
-  const size_t ssm = batch_sums_enabled() ? sums_smem(THREADS, max_layers, tab_entries, &stab) : 0;
-  *sums = ssm > 0;
-  if (*sums) {
-    *gsm = ssm;
-    *gtab = stab;
-    *stage = 1;
-  } else {
-    *gsm = grad_smem(THREADS, max_layers, tab_entries, stage, gtab);
-  }
-  // limits only ever rise (raise_smem_limit), so batches of different shapes launched from
-  // several host threads at once never find a kernel's limit lowered under them
-  static SmemLimit slim, glim;
-  const void* gk = *sums ? (const void*)batch_grad_sums_kernel<THREADS>
-                        : (const void*)batch_gradient_kernel<THREADS>;
-  if (*gsm > 48 * 1024 && raise_smem_limit(gk, *gsm, *sums ? slim : glim,
-                                           "kr_batch_launch: gradient smem") != KR_OK)
-    return KR_ERR_CUDA;
-  h.grid_grad = occupancy_grid(gk, THREADS, *gsm);
-  return KR_OK;
 }
 
 }  // namespace kr
@@ -801,27 +775,60 @@ static kr_status launch_batch_forward(unsigned char* pl, int max_layers, const d
   return KR_OK;
 }
 
+// One class of the gradient items on a resident grid.  `after`: as the programmatic dependent of
+// the class launched before it.
+template <int THREADS, bool DEEP>
+static kr_status launch_batch_gradient(unsigned char* pl, int max_layers, const double2* w,
+                                       const double2* obs, double2* R, double* chi_grad, bool after,
+                                       cudaStream_t st) {
+  const int L = DEEP ? max_layers : std::min(max_layers, kPqsLayers);
+  const size_t sums = (DEEP && !batch_sums_enabled()) ? 0 : sums_smem(THREADS, L);
+  static SmemLimit slim, glim;
+  if (!sums) {
+    int stage = 0;
+    const size_t smem = grad_smem(THREADS, L, &stage);
+    const void* fn = (const void*)batch_gradient_kernel<THREADS>;
+    if (smem > 46 * 1024 &&
+        raise_smem_limit(fn, smem, glim, "kr_batch_launch: gradient smem") != KR_OK)
+      return KR_ERR_CUDA;
+    batch_gradient_kernel<THREADS><<<occupancy_grid(fn, THREADS, smem), THREADS, smem, st>>>(
+        pl, w, obs, R, chi_grad, stage);
+    return check_launch("kr_batch_launch: gradient");
+  }
+  const void* fn = (const void*)batch_grad_sums_kernel<THREADS, DEEP>;
+  if (sums > 46 * 1024 &&
+      raise_smem_limit(fn, sums, slim, "kr_batch_launch: gradient smem") != KR_OK)
+    return KR_ERR_CUDA;
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(occupancy_grid(fn, THREADS, sums));
+  lc.blockDim = dim3(THREADS);
+  lc.dynamicSmemBytes = sums;
+  lc.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = attr;
+  lc.numAttrs = after ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&lc, batch_grad_sums_kernel<THREADS, DEEP>, pl, w, obs, R,
+                                           chi_grad);
+  if (e != cudaSuccess) {
+    set_last_error("kr_batch_launch: gradient", e);
+    return KR_ERR_CUDA;
+  }
+  return KR_OK;
+}
+
 // One batch launch for a block size of THREADS (32: one warp per work item, i.e. per
-// (model, slowness) pair and frequency range; 64 / 128: two / four warps per item).
+// (model, slowness) pair and frequency range; 64 / 128: two / four warps per item).  Grid sizes
+// come from occupancy queries (host-side, capture-safe).
 template <int THREADS>
 static kr_status launch_batch(unsigned char* pl, const kr_batch_config* cfg, int max_layers,
                               const double* layers, const double* p, const double* omega,
                               const double* R_obs, double* R, double* chi_grad,
                               cudaStream_t st) {
-  // Grid sizes from an occupancy query (host-side, capture-safe).
-  PlanHeader h{};
-  size_t gsm = 0;
-  int stage = 0;
-  const int tab = fwd_table_entries(cfg->tile_w);
-  int gtab = 0;
-  bool sums = false;
-  kr_status s = grids<THREADS>(h, max_layers, tab, &gsm, &stage, &gtab, &sums);
-  if (s != KR_OK) {
-    set_last_error_msg("kr_batch_launch: shared-memory attribute");
-    return s;
-  }
+  (void)cfg;
   batch_reset_kernel<<<148, 128, 0, st>>>(pl, chi_grad);
-  s = check_launch("kr_batch_launch: reset");
+  kr_status s = check_launch("kr_batch_launch: reset");
   if (s != KR_OK) return s;
   int gs = 4;
   while (gs < max_layers && gs < kPrepBlock) gs *= 2;
@@ -829,7 +836,7 @@ static kr_status launch_batch(unsigned char* pl, const kr_batch_config* cfg, int
   s = check_launch("kr_batch_launch: prep");
   if (s != KR_OK) return s;
   // a batch without observed data has no gradient models: no tangents, no gradient kernel
-  const bool grads = R_obs != nullptr;
+  const bool grads = R_obs != nullptr, deep = max_layers > kPqsLayers;
   if (grads) {
     // tangents on a resident-sized grid: every block starts at once and releases the forward
     // kernel, its programmatic dependent
@@ -838,23 +845,19 @@ static kr_status launch_batch(unsigned char* pl, const kr_batch_config* cfg, int
     if (s != KR_OK) return s;
   }
   const double2* w = reinterpret_cast<const double2*>(omega);
+  const double2* obs = reinterpret_cast<const double2*>(R_obs);
   double2* R2 = reinterpret_cast<double2*>(R);
-  if (max_layers > kPqsLayers) {
+  if (deep) {
     s = launch_batch_forward<THREADS, true>(pl, max_layers, w, R2, grads, st);
     if (s != KR_OK) return s;
   }
-  s = launch_batch_forward<THREADS, false>(pl, max_layers, w, R2, grads || max_layers > kPqsLayers,
-                                           st);
+  s = launch_batch_forward<THREADS, false>(pl, max_layers, w, R2, grads || deep, st);
   if (s != KR_OK || !grads) return s;
-  if (sums)
-    batch_grad_sums_kernel<THREADS><<<h.grid_grad, THREADS, gsm, st>>>(
-        pl, w, reinterpret_cast<const double2*>(R_obs), reinterpret_cast<double2*>(R), chi_grad,
-        max_layers, gtab);
-  else
-    batch_gradient_kernel<THREADS><<<h.grid_grad, THREADS, gsm, st>>>(
-        pl, w, reinterpret_cast<const double2*>(R_obs), reinterpret_cast<double2*>(R), chi_grad,
-        stage, gtab);
-  return check_launch("kr_batch_launch: gradient");
+  if (deep) {
+    s = launch_batch_gradient<THREADS, true>(pl, max_layers, w, obs, R2, chi_grad, false, st);
+    if (s != KR_OK) return s;
+  }
+  return launch_batch_gradient<THREADS, false>(pl, max_layers, w, obs, R2, chi_grad, deep, st);
 }
 
 }  // namespace kr

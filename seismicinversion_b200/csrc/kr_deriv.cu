@@ -4,10 +4,9 @@
 // Kernels (stream-ordered, no host synchronisation):
 //   deriv_prep_kernel  : per (p, interface, tangent column or coefficients): layer terms and
 //                        derivative factors, interface coefficients and their 10 x 6 tangents
-//                        -> workspace (JAC, and GRAD / VJP on the per-step path)
-//   deriv_coef_kernel, deriv_tan_kernel : the same in two kernels for the frequency-sum sweep,
-//                        which is launched as the tangent kernel's programmatic dependent and
-//                        waits for the tangents only before its contraction
+//                        -> workspace (kr_prep.cuh).  The frequency-sum sweep forms its own
+//                        coefficients, is launched as this kernel's programmatic dependent and
+//                        waits for it only before its contraction
 //   deriv_sum_kernel   : GRAD / VJP, per (omega, p): forward sweep with a tape of up to 64
 //                        steps (deeper models checkpoint and recompute segments), seed
 //                        2 conj(R - R_obs) (GRAD) or conj(gR) (VJP), reverse sweep; the per-step
@@ -64,51 +63,6 @@ static DerivWs deriv_ws(void* base, int L, int n_p, size_t n_blocks) {
   off = a256(off + sizeof(double) * n_blocks * (size_t)(4 * L + 1));
   w.bytes = off;
   return w;
-}
-
-// The same preparation in two kernels, for the frequency-sum sweep, which needs the
-// coefficients from its first step but the tangents only in its final contraction:
-// deriv_coef_kernel (block per slowness and chunk of kPrepThreads interfaces: layer terms
-// staged in shared memory, then one thread per interface for the coefficients, exactly as in
-// deriv_prep_kernel) and deriv_tan_kernel (one thread per (slowness, interface, tangent
-// column), from the layer terms deriv_coef_kernel wrote), which lets the sweep launch at once
-// (griddepcontrol.launch_dependents) so that the tangents overlap the sweep.
-__global__ void __launch_bounds__(kPrepThreads)
-deriv_coef_kernel(const double* __restrict__ tab, int L, const double* __restrict__ p,
-                  int n_chunks, LayerP* lay, LayerD* dlay, Iface* coef) {
-  __shared__ LayerP s_lp[kPrepThreads + 1];
-  const int I = L - 1;
-  const int j = blockIdx.x / n_chunks;
-  const int i0 = (blockIdx.x % n_chunks) * kPrepThreads;
-  const int i1 = min(i0 + kPrepThreads, I);  // the chunk's interfaces [i0, i1), layers i0 .. i1
-  const double pj = p[j];
-  for (int l = i0 + threadIdx.x; l <= i1; l += blockDim.x) {
-    const LayerP lp = layer_terms(tab, L, l, pj);
-    s_lp[l - i0] = lp;
-    if (l < i1 || i1 == I) {  // each layer written by one block
-      lay[(size_t)j * L + l] = lp;
-      dlay[(size_t)j * L + l] = layer_derivs(tab, L, l, pj, lp);
-    }
-  }
-  __syncthreads();
-  const int i = i0 + threadIdx.x;
-  if (i < i1) coef[(size_t)j * I + i] = interface_coeffs(pj, i, s_lp[i - i0], s_lp[i + 1 - i0]);
-}
-
-__global__ void __launch_bounds__(kPrepThreads)
-deriv_tan_kernel(const double* __restrict__ p, int n_p, int L, const LayerP* __restrict__ lay,
-                 const LayerD* __restrict__ dlay, ScatTan* tan) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int I = L - 1;
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)n_p * I * 6) return;
-  const int col = (int)(t % 6);
-  const size_t idx = t / 6;
-  const int j = (int)(idx / I), i = (int)(idx % I);
-  const size_t e = (size_t)j * L + i;
-  cd c[10];
-  interface_tangent_col(p[j], i, lay[e], dlay[e], lay[e + 1], dlay[e + 1], col, c);
-  for (int k = 0; k < 10; ++k) tan[idx].t[k][col] = c[k];
 }
 
 // Jacobian mode: writes dR/dtheta of layer l.
@@ -192,10 +146,9 @@ deriv_sweep_kernel(int L, const double* __restrict__ p, int n_p,
                    double* __restrict__ partial) {
   // dynamic smem: [warps][4L + 1] per-warp accumulators (GRAD), then, if `stage`, this
   // block's slowness data (tangents, coefficients, layer terms, layer derivatives), then, if
-  // `table`, the phase-factor table of this block's frequency tile (kr_phase.cuh)
+  // `table`, the phase-factor table of this block's frequency tile (kr_adjsum.cuh)
   constexpr bool GRAD = MODE != kModeJac;
   extern __shared__ __align__(16) double s_wacc[];
-  __shared__ unsigned s_bad;
   const int ip = blockIdx.x / n_wtiles;
   const int iw = (blockIdx.x % n_wtiles) * kDerThreads + threadIdx.x;
   const bool valid = iw < n_w;
@@ -234,15 +187,18 @@ deriv_sweep_kernel(int L, const double* __restrict__ p, int n_p,
   }
   const int tile = blockIdx.x % n_wtiles;
   const size_t acc_bytes = GRAD ? sizeof(double) * (((kDerThreads / 32) * nv + 1) / 2 * 2) : 0;
-  cd* s_ph = reinterpret_cast<cd*>(reinterpret_cast<unsigned char*>(s_wacc) + acc_bytes +
+  cd* s_lo = reinterpret_cast<cd*>(reinterpret_cast<unsigned char*>(s_wacc) + acc_bytes +
                                    pair_smem_bytes(L));
-  bool use_tab = false;
-  if (table)
-    use_tab = (build_phase_table(omega, n_w, grid_line(omega, n_w), tile, 1, kPhHead + 1, L, lay,
-                                 s_ph, &s_bad) &
-               1u) != 0;
-  const PhaseAuto ph{use_tab, phase_at(s_ph, kPhHead + 1, valid ? iw : tile * kDerThreads, tile),
-                     PhaseDirect{w, lay}};
+  cd* hm = s_lo + ray_lo_values(L) + (threadIdx.x >> 5) * ray_hm_values(L);
+  bool use_tab = table != 0;
+  if (use_tab) {
+    const GridLine g = grid_line(omega, n_w);
+    use_tab = ray_lo_fill(g, L, lay, s_lo);
+    if (valid) use_tab &= on_line(g, iw, make_double2(w.x, w.y));
+    use_tab = __syncthreads_and(use_tab) != 0;
+    if (use_tab)
+      use_tab = ray_hm_fill(omega, n_w, tile * kDerThreads + (threadIdx.x & ~31), L, lay, hm);
+  }
   PairSink<MODE> sink;
   sink.L = L;
   sink.ip = ip;
@@ -253,7 +209,10 @@ deriv_sweep_kernel(int L, const double* __restrict__ p, int n_p,
   sink.R_out = R_out;
   sink.J = J;
   sink.s_wacc = s_wacc;
-  jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan, ph, sink);
+  if (use_tab)
+    jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan, ray_table(s_lo, hm), sink);
+  else
+    jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan, PhaseDirect{w, lay}, sink);
   if (GRAD) {
     const cd res = sink.res;
     double c2 = valid ? (res.x * res.x + res.y * res.y) : 0.0;
@@ -291,49 +250,63 @@ reduce_partials_kernel(const double* __restrict__ partial, int n_blocks, int str
 }
 
 // GRAD / VJP with the contraction moved out of the frequency loop (kr_adjsum.cuh): block =
-// one slowness x 128 frequencies; dynamic smem: per-warp sum rows and staging tiles, then the
-// slowness's interface coefficients and layer terms, then (table models) the phase table.
-// Writes the block's [4L] contributions and chi to partial[block][4L + 1].
+// one slowness x 128 frequencies.  The block forms its own layer terms, coefficients and phase
+// table (the stages of the forward kernel's prologue), so nothing but the contraction waits for
+// deriv_prep_kernel, whose programmatic dependent it is.  Dynamic smem: per-warp sum rows and
+// staging rows (first the layer terms and roots, which only the prologue reads), the interface
+// coefficients, then (table models) the phase table: 52 KB for 21 layers, four blocks per SM, so
+// that the 512 blocks of a 64 x 1024 gradient are one wave.  Writes the block's [4L] contributions and chi to
+// partial[block][4L + 1].
 template <int MINB>
 __global__ void __launch_bounds__(kDerThreads, MINB)
-deriv_sum_kernel(int L, int n_p, const double2* __restrict__ omega, int n_w, int n_wtiles,
-                 int free_surface, int vjp, int seg, int table, const LayerP* __restrict__ lay_all,
-                 const LayerD* __restrict__ dlay_all, const Iface* __restrict__ coef_all,
-                 const ScatTan* __restrict__ tan_all, const double2* __restrict__ obs,
-                 double2* __restrict__ R_out, double* __restrict__ partial) {
+deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restrict__ p,
+                 const double2* __restrict__ omega, int n_w, int n_wtiles, int free_surface,
+                 int vjp, int seg, int table, const LayerP* __restrict__ lay_all,
+                 const LayerD* __restrict__ dlay_all, const ScatTan* __restrict__ tan_all,
+                 const double2* __restrict__ obs, double2* __restrict__ R_out,
+                 double* __restrict__ partial) {
   // the reduction after this kernel may launch as soon as every block of it has started
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int W = kDerThreads / 32;
   extern __shared__ __align__(16) double s_raw[];
-  __shared__ unsigned s_bad;
   __shared__ double s_chi[W];
   const int I = L - 1;
   const int ip = blockIdx.x / n_wtiles;
   const int tile = blockIdx.x % n_wtiles;
   const int iw = tile * kDerThreads + threadIdx.x;
   const bool valid = iw < n_w;
-  const int warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double* acc = s_raw;
   cd* stage = reinterpret_cast<cd*>(acc + (size_t)W * sum_rows(L) * kRayRow);
-  unsigned char* b = reinterpret_cast<unsigned char*>(stage + W * kRayStage);
-  Iface* sc = reinterpret_cast<Iface*>(b);
-  LayerP* sl = reinterpret_cast<LayerP*>(b + sizeof(Iface) * I);
-  cd* s_ph = reinterpret_cast<cd*>(b + sizeof(Iface) * I + sizeof(LayerP) * L);
+  unsigned char* b = reinterpret_cast<unsigned char*>(stage) + ray_stage_bytes(L, W);
+  LayerP* s_lay = reinterpret_cast<LayerP*>(stage);
+  LayerRoots* s_root = reinterpret_cast<LayerRoots*>(s_lay + L);
+  Iface* s_if = reinterpret_cast<Iface*>(b);
+  cd* s_lo = reinterpret_cast<cd*>(s_if + I);
+  const double pj = p[ip];
   sums_zero(acc, L, W);
-  copy16(sc, coef_all + (size_t)ip * I, sizeof(Iface) * I);
-  copy16(sl, lay_all + (size_t)ip * L, sizeof(LayerP) * L);
-  __syncthreads();
+  for (int t = threadIdx.x; t < 2 * L; t += kDerThreads) {
+    const int half = t >= L ? 1 : 0, l = t - half * L;
+    layer_store(tab6, L, l, half, pj, s_lay + l, s_root + l);
+  }
   cd w = mk(0.0, 0.0);
   if (valid) {
     const double2 wv = omega[iw];
     w = mk(wv.x, wv.y);
   }
-  bool use_tab = false;
-  if (table)
-    use_tab = (build_phase_table(omega, n_w, grid_line(omega, n_w), tile, 1, kPhHead + 1, L, sl,
-                                 s_ph, &s_bad) & 1u) != 0;
-  const PhaseAuto ph{use_tab, phase_at(s_ph, kPhHead + 1, valid ? iw : tile * kDerThreads, tile),
-                     PhaseDirect{w, sl}};
+  __syncthreads();
+  for (int i = threadIdx.x; i < I; i += kDerThreads)
+    interface_store(pj, i, s_lay, s_root, s_if + i);
+  bool ok = table != 0;
+  cd* hm = s_lo + ray_lo_values(L) + warp * ray_hm_values(L);
+  if (ok) {
+    const GridLine g = grid_line(omega, n_w);
+    ok = ray_lo_fill(g, L, s_lay, s_lo);
+    if (valid) ok &= on_line(g, iw, make_double2(w.x, w.y));
+  }
+  ok = __syncthreads_and(ok) != 0;
+  if (ok) ok = ray_hm_fill(omega, n_w, tile * kDerThreads + 32 * warp, L, s_lay, hm);
+  __syncthreads();  // the layer terms are read before the staging rows overwrite them
   const size_t e = (size_t)ip * n_w + (valid ? iw : 0);
   RaySumSink sink;
   sink.valid = valid;
@@ -343,14 +316,21 @@ deriv_sum_kernel(int L, int n_p, const double2* __restrict__ omega, int n_w, int
   sink.acc = acc + (size_t)warp * sum_rows(L) * kRayRow;
   sink.stage = stage + warp * kRayStage;
   sink.I = I;
-  adjoint_rays(L, w, free_surface != 0, seg, sc, ph, sink);
+  if (ok) {
+    adjoint_rays(L, w, free_surface != 0, seg, s_if, ray_table(s_lo, hm), sink);
+  } else {
+    // direct exponentials read the layer terms of the preparation
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    adjoint_rays(L, w, free_surface != 0, seg, s_if, PhaseDirect{w, lay_all + (size_t)ip * L},
+                 sink);
+  }
   double c2 = valid ? (sink.res.x * sink.res.x + sink.res.y * sink.res.y) : 0.0;
   for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);
-  if ((threadIdx.x & 31) == 0) s_chi[warp] = c2;
+  if (lane == 0) s_chi[warp] = c2;
   double* dst = partial + (size_t)blockIdx.x * (4 * L + 1);
-  // the tangents may still be in the making (deriv_tan_kernel, launched ahead of this kernel
-  // as its programmatic prerequisite): wait for that grid's completion and its writes; a
-  // no-op when the kernel was launched without the dependency
+  // the tangents may still be in the making (deriv_prep_kernel, launched ahead of this kernel as
+  // its programmatic prerequisite): wait for that grid's completion and its writes; a no-op when
+  // the kernel was launched without the dependency
   asm volatile("griddepcontrol.wait;" ::: "memory");
   sums_finish(acc, L, W, tan_all + (size_t)ip * I, dlay_all + (size_t)ip * L, dst);
   if (threadIdx.x == 0) {
@@ -364,8 +344,9 @@ deriv_sum_kernel(int L, int n_p, const double2* __restrict__ omega, int n_w, int
 constexpr size_t kStageSmemMax = 160 * 1024;
 
 // Register budget of the sweep kernels: blocks of 128 threads per SM (2 -> up to 255
-// registers, 3 -> 168).  KR_DERIV_MINB or kr_set_deriv_variant; default 2 (the frequency-sum
-// kernel needs 164 registers either way: 80.6 us per 64 x 1024 gradient at both settings).
+// registers, 3 -> 168).  KR_DERIV_MINB or kr_set_deriv_variant; by default 3 for the per-step
+// sweeps (64 x 1024 x 21-layer Jacobian 106 us against 111 at 2) and 4 (128 registers) for the
+// frequency-sum sweep (gradient 75 us against 88 at 3, where 512 blocks are more than one wave).
 static int g_deriv_minb = -1;
 
 static int deriv_minb_setting() {
@@ -376,8 +357,8 @@ static int deriv_minb_setting() {
   }
   return g_deriv_minb;
 }
-static int deriv_minb() { return deriv_minb_setting() == 3 ? 3 : 2; }
-static int sum_minb() { return deriv_minb(); }
+static int deriv_minb() { return deriv_minb_setting() == 2 ? 2 : 3; }
+static int sum_minb() { return deriv_minb_setting() == 3 ? 3 : 4; }
 
 template <int MODE, int MINB>
 static kr_status launch_sweep_v(unsigned blocks, size_t smem, cudaStream_t st, int L,
@@ -414,8 +395,9 @@ static kr_status launch_sweep(int minb, unsigned blocks, size_t smem, cudaStream
 
 // Dynamic smem of deriv_sum_kernel for a model of L layers (0 if it does not fit).
 static size_t sum_kernel_smem(int L, int table) {
-  const size_t smem = raysum_smem_bytes(L, kDerThreads / 32) + prologue_smem_bytes(L) +
-                      (table ? phase_table_bytes(L, 1) : 0);
+  const int W = kDerThreads / 32;
+  const size_t smem = sizeof(double) * W * kRayRow * sum_rows(L) + ray_stage_bytes(L, W) +
+                      sizeof(Iface) * (size_t)(L - 1) + (table ? ray_table_bytes(L, W) : 0);
   return smem <= kStageSmemMax ? smem : 0;
 }
 
@@ -430,19 +412,19 @@ static bool deriv_sums_enabled() {
 }
 
 template <int MINB>
-static kr_status launch_sum_v(unsigned blocks, size_t smem, cudaStream_t st, int L, int n_p,
-                              const double2* omega, int n_w, int n_wtiles, int fs, int vjp,
-                              int seg, int table, const LayerP* lay, const LayerD* dlay,
-                              const Iface* coef, const ScatTan* tan, const double2* obs,
+static kr_status launch_sum_v(unsigned blocks, size_t smem, cudaStream_t st, const double* layers,
+                              int L, const double* p, const double2* omega, int n_w, int n_wtiles,
+                              int fs, int vjp, int seg, int table, const LayerP* lay,
+                              const LayerD* dlay, const ScatTan* tan, const double2* obs,
                               double2* R, double* partial) {
   static SmemLimit lim;
-  if (smem > 48 * 1024) {
+  if (smem > 47 * 1024) {  // with the static arrays above the 48 KB default
     const kr_status a = raise_smem_limit((const void*)deriv_sum_kernel<MINB>, smem, lim,
                                          "kr_deriv: smem attribute");
     if (a != KR_OK) return a;
   }
-  // programmatic dependent launch: the sweep may start while the tangent kernel ahead of it
-  // on the stream still runs; it waits for it (griddepcontrol.wait) only before contracting
+  // programmatic dependent launch: the sweep may start while the preparation ahead of it on the
+  // stream still runs; it waits for it (griddepcontrol.wait) only before contracting
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(kDerThreads);
@@ -453,9 +435,9 @@ static kr_status launch_sum_v(unsigned blocks, size_t smem, cudaStream_t st, int
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, deriv_sum_kernel<MINB>, L, n_p, omega, n_w,
-                                           n_wtiles, fs, vjp, seg, table, lay, dlay, coef, tan,
-                                           obs, R, partial);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, deriv_sum_kernel<MINB>, layers, L, p, omega, n_w,
+                                           n_wtiles, fs, vjp, seg, table, lay, dlay, tan, obs, R,
+                                           partial);
   if (e != cudaSuccess) {
     set_last_error("kr_deriv: sweep launch", e);
     return KR_ERR_CUDA;
@@ -476,31 +458,11 @@ static kr_status launch_deriv(const double* layers, int L, const double* p, int 
   if (!ws || ws_bytes < w.bytes) return KR_ERR_WORKSPACE;
   const int I = L - 1;
   const int seg = checkpoint_spacing(I - 1 > 0 ? I - 1 : 1);
-  const int sum_table = phase_table_model(L) ? 1 : 0;
+  const int sum_table = ray_table_model(L) ? 1 : 0;
   const size_t sum_smem = (GRAD && deriv_sums_enabled()) ? sum_kernel_smem(L, sum_table) : 0;
-  kr_status s = KR_OK;
-  if (sum_smem) {
-    // coefficients first; the tangents then overlap the frequency-sum sweep
-    const int n_cc = (I + kPrepThreads - 1) / kPrepThreads;
-    const size_t n_tan = (size_t)n_p * I * 6;
-    if ((size_t)n_p * n_cc > 0x7fffffffULL || (n_tan + kPrepThreads - 1) / kPrepThreads > 0x7fffffffULL)
-      return KR_ERR_TOO_LARGE;
-    deriv_coef_kernel<<<(unsigned)(n_p * n_cc), kPrepThreads, 0, st>>>(layers, L, p, n_cc, w.lay,
-                                                                       w.dlay, w.coef);
-    s = check_launch("kr_deriv: layers and coefficients");
-    if (s != KR_OK) return s;
-    deriv_tan_kernel<<<(unsigned)((n_tan + kPrepThreads - 1) / kPrepThreads), kPrepThreads, 0,
-                       st>>>(p, n_p, L, w.lay, w.dlay, w.tan);
-    s = check_launch("kr_deriv: tangents");
-    if (s != KR_OK) return s;
-  } else {
-    const int n_chunks = (kPrepItems * I + kPrepThreads - 1) / kPrepThreads;
-    if ((size_t)n_p * n_chunks > 0x7fffffffULL) return KR_ERR_TOO_LARGE;
-    deriv_prep_kernel<<<(unsigned)(n_p * n_chunks), kPrepThreads, 0, st>>>(
-        layers, L, p, n_chunks, w.lay, w.dlay, w.coef, w.tan);
-    s = check_launch("kr_deriv: layers and interfaces");
-    if (s != KR_OK) return s;
-  }
+  kr_status s = launch_prep(layers, L, p, n_p, w.lay, w.dlay, w.coef, w.tan, st,
+                            "kr_deriv: layers and interfaces");
+  if (s != KR_OK) return s;
   if (sum_smem) {
     const int fs = (flags & KR_FREE_SURFACE) ? 1 : 0;
     const int vjp = MODE == kModeVjp ? 1 : 0;
@@ -508,10 +470,10 @@ static kr_status launch_deriv(const double* layers, int L, const double* p, int 
     const double2* w2 = reinterpret_cast<const double2*>(omega);
     double2* R2 = reinterpret_cast<double2*>(R);
     s = sum_minb() == 3
-            ? launch_sum_v<3>((unsigned)n_blocks, sum_smem, st, L, n_p, w2, n_w, n_wtiles, fs,
-                              vjp, seg, sum_table, w.lay, w.dlay, w.coef, w.tan, o, R2, w.partial)
-            : launch_sum_v<2>((unsigned)n_blocks, sum_smem, st, L, n_p, w2, n_w, n_wtiles, fs,
-                              vjp, seg, sum_table, w.lay, w.dlay, w.coef, w.tan, o, R2, w.partial);
+            ? launch_sum_v<3>((unsigned)n_blocks, sum_smem, st, layers, L, p, w2, n_w, n_wtiles,
+                              fs, vjp, seg, sum_table, w.lay, w.dlay, w.tan, o, R2, w.partial)
+            : launch_sum_v<4>((unsigned)n_blocks, sum_smem, st, layers, L, p, w2, n_w, n_wtiles,
+                              fs, vjp, seg, sum_table, w.lay, w.dlay, w.tan, o, R2, w.partial);
     if (s != KR_OK) return s;
     s = check_launch("kr_deriv: sweep");
     if (s != KR_OK) return s;
@@ -539,8 +501,8 @@ static kr_status launch_deriv(const double* layers, int L, const double* p, int 
   const int stage = (acc + pair <= kStageSmemMax) ? 1 : 0;
   // phase table of the block's tile after the staged slowness data (models that tabulate in
   // kr_reflectivity, so R here is bit-identical to the forward kernel's)
-  const int table = (stage && phase_table_model(L)) ? 1 : 0;
-  const size_t smem = acc + (stage ? pair : 0) + (table ? phase_table_bytes(L, 1) : 0);
+  const int table = (stage && ray_table_model(L)) ? 1 : 0;
+  const size_t smem = acc + (stage ? pair : 0) + (table ? ray_table_bytes(L, kDerThreads / 32) : 0);
   s = launch_sweep<MODE>(deriv_minb(), (unsigned)n_blocks, smem, st, L, p, n_p,
                          reinterpret_cast<const double2*>(omega), n_w, n_wtiles,
                          (flags & KR_FREE_SURFACE) ? 1 : 0, seg, stage, table, w.lay, w.dlay, w.coef,

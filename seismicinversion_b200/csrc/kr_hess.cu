@@ -80,7 +80,6 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
                  cd* __restrict__ sums) {
   constexpr int W = kHessThreads / 32;
   extern __shared__ __align__(16) double s_raw[];
-  __shared__ unsigned s_bad;
   const int I = L - 1;
   const int jp = blockIdx.x / n_wtiles, ip = p0 + jp;  // slowness within the turn, and overall
   const int tile = blockIdx.x % n_wtiles;
@@ -92,7 +91,7 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
   cd* stage = reinterpret_cast<cd*>(acc + (size_t)W * nrow);
   Iface* sc = reinterpret_cast<Iface*>(stage + W * kRayStage);
   LayerP* sl = reinterpret_cast<LayerP*>(sc + I);
-  cd* s_ph = reinterpret_cast<cd*>(sl + L);
+  cd* s_lo = reinterpret_cast<cd*>(sl + L);
   sums_zero(acc, L, W);
   copy16(sc, coef_all + (size_t)ip * I, sizeof(Iface) * I);
   copy16(sl, lay_all + (size_t)ip * L, sizeof(LayerP) * L);
@@ -102,12 +101,15 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
     const double2 wv = omega[iw];
     w = mk(wv.x, wv.y);
   }
-  bool use_tab = false;
-  if (table)
-    use_tab = (build_phase_table(omega, n_w, grid_line(omega, n_w), tile, 1, kPhHead + 1, L, sl,
-                                 s_ph, &s_bad) & 1u) != 0;
-  const PhaseAuto ph{use_tab, phase_at(s_ph, kPhHead + 1, valid ? iw : tile * kHessThreads, tile),
-                     PhaseDirect{w, sl}};
+  bool use_tab = table != 0;
+  cd* hm = s_lo + ray_lo_values(L) + warp * ray_hm_values(L);
+  if (use_tab) {
+    const GridLine g = grid_line(omega, n_w);
+    use_tab = ray_lo_fill(g, L, sl, s_lo);
+    if (valid) use_tab &= on_line(g, iw, make_double2(w.x, w.y));
+    use_tab = __syncthreads_and(use_tab) != 0;
+    if (use_tab) use_tab = ray_hm_fill(omega, n_w, tile * kHessThreads + 32 * warp, L, sl, hm);
+  }
   const size_t k = valid ? iw : 0;
   HessRaySink sink;
   sink.valid = valid;
@@ -121,7 +123,10 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
   sink.acc = acc + (size_t)warp * nrow;
   sink.stage = stage + warp * kRayStage;
   sink.K = S3{mk(0.0, 0.0), mk(0.0, 0.0), mk(0.0, 0.0)};
-  adjoint_rays(L, w, free_surface != 0, seg, sc, ph, sink);
+  if (use_tab)
+    adjoint_rays(L, w, free_surface != 0, seg, sc, ray_table(s_lo, hm), sink);
+  else
+    adjoint_rays(L, w, free_surface != 0, seg, sc, PhaseDirect{w, sl}, sink);
   __syncthreads();
   for (int e = threadIdx.x; e < nrow; e += kHessThreads) {
     double s = acc[e];
@@ -496,19 +501,17 @@ extern "C" kr_status kr_misfit_hessian(const double* layers, int32_t n_layers, c
   if (!workspace || workspace_bytes < w.bytes) return KR_ERR_WORKSPACE;
   const int n_wtiles = (n_w + kHessThreads - 1) / kHessThreads;
   const int n_wc = (n_w + kPairFreq - 1) / kPairFreq;
-  const int n_prep = (kPrepItems * I + kPrepThreads - 1) / kPrepThreads;
   const size_t n_curv = (size_t)n_p * I * kHessItems;
-  if ((size_t)n_p * n_prep > 0x7fffffffULL || (size_t)n_p * n_wc > 0x7fffffffULL ||
+  if ((size_t)n_p * n_wc > 0x7fffffffULL ||
       (n_curv + 127) / 128 > 0x7fffffffULL)
     return KR_ERR_TOO_LARGE;
   const double2* w2 = reinterpret_cast<const double2*>(omega);
-  deriv_prep_kernel<<<(unsigned)(n_p * n_prep), kPrepThreads, 0, st>>>(layers, L, p, n_prep, w.lay,
-                                                                       w.dlay, w.coef, w.tan);
-  kr_status s = check_launch("kr_misfit_hessian: layers and interfaces");
+  kr_status s = launch_prep(layers, L, p, n_p, w.lay, w.dlay, w.coef, w.tan, st,
+                            "kr_misfit_hessian: layers and interfaces");
   if (s != KR_OK) return s;
-  const int table = phase_table_model(L) ? 1 : 0;
+  const int table = ray_table_model(L) ? 1 : 0;
   const size_t rs = raysum_smem_bytes(L, kHessThreads / 32) + prologue_smem_bytes(L) +
-                    (table ? phase_table_bytes(L, 1) : 0);
+                    (table ? ray_table_bytes(L, kHessThreads / 32) : 0);
   const size_t ps = hess_pairs_smem(L);
   static SmemLimit rlim, plim;
   if (rs > 48 * 1024) {

@@ -13,14 +13,20 @@ namespace kr {
 // coefficients and the workspace copy of its upper layer (and of the half-space, for the last
 // interface), so no lane of a warp waits on another's extra work.  The coefficients read the
 // layer terms back from shared memory after a barrier, as the forward kernel's prologue
-// does, so they round exactly as there (R bit-identical across entry points).
+// does, so they round exactly as there (R bit-identical across entry points).  Blocks of 128 threads:
+// with 64, twice as many SMs are busy with 250 registers a thread while the frequency-sum sweep
+// runs beside this kernel (64 x 32 gradient 65 us against 56), and kernels that wait for it gain
+// nothing (64 x 1024 Jacobian 106.4 against 106.2).
 constexpr int kPrepThreads = 128;
-constexpr int kPrepItems = 7;                                  // per interface
-constexpr int kPrepLayers = kPrepThreads / kPrepItems + 3;     // layers one chunk touches
+constexpr int kPrepItems = 7;                               // per interface
+constexpr int kPrepLayers = kPrepThreads / kPrepItems + 3;  // layers one chunk touches
 
 static __global__ void __launch_bounds__(kPrepThreads)
 deriv_prep_kernel(const double* __restrict__ tab, int L, const double* __restrict__ p,
                   int n_chunks, LayerP* lay, LayerD* dlay, Iface* coef, ScatTan* tan) {
+  // a sweep that forms its own coefficients may start at once (it waits for this grid before it
+  // reads the tangents)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ LayerP s_lp[kPrepLayers];
   __shared__ LayerD s_ld[kPrepLayers];
   const int I = L - 1;
@@ -54,6 +60,16 @@ deriv_prep_kernel(const double* __restrict__ tab, int L, const double* __restric
   cd c[10];
   interface_tangent_col(pj, i, up, s_ld[i - l0], lo, s_ld[i + 1 - l0], item, c);
   for (int k = 0; k < 10; ++k) tan[idx].t[k][item] = c[k];
+}
+
+static kr_status launch_prep(const double* layers, int L, const double* p, int n_p, LayerP* lay,
+                             LayerD* dlay, Iface* coef, ScatTan* tan, cudaStream_t st,
+                             const char* what) {
+  const int n_chunks = (kPrepItems * (L - 1) + kPrepThreads - 1) / kPrepThreads;
+  if ((size_t)n_p * n_chunks > 0x7fffffffULL) return KR_ERR_TOO_LARGE;
+  deriv_prep_kernel<<<(unsigned)(n_p * n_chunks), kPrepThreads, 0, st>>>(layers, L, p, n_chunks, lay,
+                                                                         dlay, coef, tan);
+  return check_launch(what);
 }
 
 }  // namespace kr
