@@ -50,20 +50,18 @@ __host__ __device__ constexpr double hankel_a(int k) {
 __host__ __device__ constexpr double hankel_p(int m) { return (m % 2 ? -1.0 : 1.0) * hankel_a(2 * m); }
 __host__ __device__ constexpr double hankel_q(int m) { return (m % 2 ? -1.0 : 1.0) * hankel_a(2 * m + 1); }
 
-// sqrt(pi x) J0(x) = P u + Q v with u = cos x + sin x, v = cos x - sin x, y = 1 / x and
-// the first NT terms of P and Q.  The first omitted terms bound the truncation error
-// (A&S 9.2.10); the absolute J0 error is below 7e-16 for NT = 7 at x >= 25 and below 1e-16
+// The first NT terms of P and x Q at q = 1 / x^2.  The first omitted terms bound the truncation
+// error (A&S 9.2.10); the absolute J0 error is below 7e-16 for NT = 7 at x >= 25 and below 1e-16
 // for NT = 5 at x >= 60, NT = 4 at x >= 100, NT = 3 at x >= 300 and NT = 2 at x >= 3000.
 template <int NT>
-__device__ __forceinline__ double j0_asym_scaled(double y, double u, double v) {
-  const double q = y * y;
-  double P = hankel_p(NT - 1), Qs = hankel_q(NT - 1);
+__device__ __forceinline__ void hankel_series(double q, double& P, double& Q) {
+  P = hankel_p(NT - 1);
+  Q = hankel_q(NT - 1);
 #pragma unroll
   for (int m = NT - 2; m >= 0; --m) {
     P = fma(P, q, hankel_p(m));
-    Qs = fma(Qs, q, hankel_q(m));
+    Q = fma(Q, q, hankel_q(m));
   }
-  return fma(P, u, Qs * (y * v));
 }
 
 // J0(x) for x >= kJ0X0 given c = cos x, s = sin x.
@@ -83,13 +81,16 @@ __device__ __forceinline__ double j0_asymptotic(double x, double c, double s) {
 
 // J0(x) for 0 <= x < 25 from the piecewise Taylor table (kr_j0_table.h, staged in shared
 // memory with rows padded to kJ0Row doubles so that lanes on different intervals fall on
-// different banks): interval k = floor(x), t = x - (k + 1/2), degree-15 Horner in t.
+// different banks): interval k and t = x - (k + 1/2) from one rounding (no conversions, which
+// are slow for 64 bits; an integer x may take either neighbour), degree-15 Horner in t.
 // Absolute error below 5e-16 against SciPy's j0 on [0, 25).
 constexpr int kJ0Row = kJ0TabDegree + 2;
 __device__ __forceinline__ double j0_table(const double* s_j0, double x) {
-  const int k = min((int)x, kJ0TabIntervals - 1);
-  const double t = x - ((double)k + 0.5);
-  const double* a = s_j0 + k * kJ0Row;
+  constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
+  const double w = x - 0.5;
+  const double z = w + kRound;
+  const double t = w - (z - kRound);
+  const double* a = s_j0 + min(__double2loint(z), kJ0TabIntervals - 1) * kJ0Row;
   double v = a[kJ0TabDegree];
 #pragma unroll
   for (int n = kJ0TabDegree - 1; n >= 0; --n) v = fma(v, t, a[n]);
@@ -98,15 +99,13 @@ __device__ __forceinline__ double j0_table(const double* s_j0, double x) {
 
 // Slowness steps between exact sincos anchors when p is an arithmetic progression.
 constexpr int kRotSteps = 32;
-// Slownesses staged per shared-memory chunk: (p_j, pw_j dp) and (1 / p_j, pw_j dp / sqrt p_j).
-constexpr int kChunk = 128;
-
 // R rows are staged through shared memory in tiles of kSub slownesses x 32 frequencies
 // (16 KB) in a ring of three with cp.async: the 8 offset warps of a block read each R
 // element from shared memory instead of each loading it from L1 / L2, two tiles are in
 // flight while one is summed, and one block barrier per tile suffices (the barrier that
 // publishes tile t also shows every warp done with tile t - 1, whose buffer then takes
-// tile t + 2).  kSub equals the rotation anchor spacing.
+// tile t + 2).  kSub equals the rotation anchor spacing.  One warp in turn forms the next tile's
+// factors of the slowness alone.
 constexpr int kSub = kRotSteps;
 constexpr int kRing = 3;
 constexpr size_t kRingBytes = sizeof(double2) * kRing * kSub * kBsW;  // dynamic shared memory
@@ -136,196 +135,294 @@ __device__ __forceinline__ void stage_R(double2 (*tile)[kBsW], const double2* __
   }
 }
 
-// Terms of one staged tile for one thread on the fast path: exact cos / sin anchor at the
-// tile's first slowness, rotation of (u, v) = (cos + sin, cos - sin) in between.  The
-// amplitude 1 / sqrt(pi omega r) is common to the thread and applied to (ax, ay) by the
-// caller; 1 / sqrt(p_j) is staged.
-template <int NT, int M>
-__device__ __forceinline__ void fast_terms(const double2* __restrict__ ig_p,
-                                           const double2* __restrict__ r_p, int m, double inv_omr,
-                                           double cdl, double sd, double& u, double& v,
-                                           double& ax, double& ay) {
+// Terms of one staged tile for one thread on the fast path.  With z = 1 / (omega r),
+//   sqrt(pi omega r) f_j J0(x_j) = (f_j / sqrt p_j) P u + (f_j / p_j^1.5) Q v,
+//   u = cos x + sin x, v = (cos x - sin x) z, P and Q at 1 / x^2 = z^2 / p_j^2:
+// what depends on the slowness alone is staged, what depends on the thread alone waits until
+// the end, 2 NT + 5 operations a term with the two of the sum (2 NT + 6 with 1 / x formed per
+// term and the weight applied to J0).  The tile starts from an exact cos and sin; from one
+// slowness to the next (u, v) turn by the step's angle d: in three shears (3 operations; tn =
+// tan(d / 2) / z, sn = z sin d), or, where a lane's d lies near half a turn and tan(d / 2) is
+// large, by products (4 operations; cs = cos d, s1 = sin d / z, sn).
+struct TileTurn {
+  double tn, sn, cs, s1;
+};
+
+template <int NT, bool SHEAR, int M>
+__device__ __forceinline__ void fast_terms(const double2* __restrict__ w_p,
+                                           const double* __restrict__ q_p,
+                                           const double2* __restrict__ r_p, int m, double z2,
+                                           const TileTurn& d, double u, double v, double& ax,
+                                           double& ay) {
 #pragma unroll 8
   for (int k = 0; k < (M > 0 ? M : m); ++k) {
-    const double2 ig = ig_p[k];
+    const double2 w = w_p[k];
     const double2 rv = r_p[k * kBsW];
-    const double t = j0_asym_scaled<NT>(ig.x * inv_omr, u, v) * ig.y;
-    const double u2 = fma(u, cdl, v * sd);
-    v = fma(v, cdl, -u * sd);
-    u = u2;
+    double P, Q;
+    hankel_series<NT>(q_p[k] * z2, P, Q);
+    const double t = fma(w.x, P * u, w.y * (Q * v));
+    if (SHEAR) {
+      u = fma(d.tn, v, u);
+      v = fma(-d.sn, u, v);
+      u = fma(d.tn, v, u);
+    } else {
+      const double u2 = fma(u, d.cs, v * d.s1);
+      v = fma(v, d.cs, -u * d.sn);
+      u = u2;
+    }
     ax = fma(t, rv.x, ax);
     ay = fma(t, rv.y, ay);
   }
 }
 
 template <int NT>
-__device__ __forceinline__ void fast_tile(const double2* s_pf, const double2* s_ig,
-                                          const double2 (*tile)[kBsW], int k0, int m, int lane,
-                                          double om, double r, double inv_omr, double cdl,
-                                          double sd, double& ax, double& ay) {
-  double s, c;
-  sincos((om * s_pf[k0].x) * r, &s, &c);
-  double u = c + s, v = c - s;
+__device__ __forceinline__ void fast_tile(const double2* w_p, const double* q_p,
+                                          const double2* r_p, int m, bool shear, double z2,
+                                          const TileTurn& d, double u, double v, double& ax,
+                                          double& ay) {
   // full tiles run a loop of compile-time length (no remainder handling)
-  if (m == kSub)
-    fast_terms<NT, kSub>(s_ig + k0, &tile[0][lane], kSub, inv_omr, cdl, sd, u, v, ax, ay);
+  if (m == kSub && shear)
+    fast_terms<NT, true, kSub>(w_p, q_p, r_p, kSub, z2, d, u, v, ax, ay);
+  else if (m == kSub)
+    fast_terms<NT, false, kSub>(w_p, q_p, r_p, kSub, z2, d, u, v, ax, ay);
   else
-    fast_terms<NT, 0>(s_ig + k0, &tile[0][lane], m, inv_omr, cdl, sd, u, v, ax, ay);
+    fast_terms<NT, false, 0>(w_p, q_p, r_p, m, z2, d, u, v, ax, ay);
 }
 
 // One thread per (omega, offset) and slowness slice.  Grid: x = slowness slice, y = offset
 // group, z = frequency tile, so the hardware starts the low-frequency tiles (small J0
 // arguments, the slowest blocks) first and the cheap high-frequency tiles fill the tail.
-// Per chunk of the slice the block stages (p_j, pw_j dp) and (1 / p_j, pw_j dp / sqrt p_j)
-// in shared memory and checks once whether the chunk continues the slice's arithmetic
-// progression (to 4.5 ulp); inside such a chunk cos / sin of x_j = (omega p_j) r advance by
-// one rotation per slowness, with an exact sincos anchor every kRotSteps.  R arrives in
-// tiles through a ring of three buffers (stage_R).  omega is factored out of the weight:
-// U = omega * sum_j J0(x_j) (pw_j dp) R_j.  Four blocks of 256 threads per SM (64 registers,
-// 40 bytes of spills; 128-slowness chunks keep four blocks' shared memory within the SM's
-// 228 KB): the kernel is bound by each warp's dependency chains, so more resident warps
-// help despite the spills (21-layer gather grid: 2.98 ms at two blocks and 124 registers,
-// 2.65 at three and 80, 2.635 at four, U bit-identical).
+// Per tile the block stages the slownesses' factors in shared memory with a check whether the
+// tile continues the slice's arithmetic progression (to 4.5 ulp); inside such a tile cos / sin of
+// x_j = (omega p_j) r advance by one rotation per slowness from an exact anchor.  A tile whose
+// arguments stay below 25 sums from the table alone, one that crosses 25 decides term by term.
+// omega is factored out of the weight: U = omega * sum_j J0(x_j) (pw_j dp) R_j.  Four blocks of 256
+// threads per SM (64 registers): with three distinct operands in most of its instructions the
+// kernel is bound by the register ports and by each warp's dependency chains, so more resident
+// warps help despite some spills.  Two offsets per thread share the loads of R and of factors
+// already multiplied by the weight (11 operations a term instead of 14), but leave 24 or 16 warps
+// per SM: 2.58 to 2.9 ms on 8192 slownesses x 2047 frequencies x 100 offsets against 2.47 ms,
+// which took 2.59 with 16 operations a term, chunks of 128 slownesses between drained rings, and
+// per-term branches below 25 (2048 x 511 x 37: 127 -> 100 us, 1000 x 300 x 100: 118 -> 89).
 __global__ void __launch_bounds__(kBsW * kBsR, 4)
 bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ p,
                       const double* __restrict__ pw, int n_p, double dp,
                       const double* __restrict__ omega, int n_w,
                       const double* __restrict__ offsets, int n_r, int p_per_slice,
                       double2* __restrict__ partial) {
-  __shared__ double2 s_pf[kChunk];  // (p_j, pw_j dp)
-  __shared__ double2 s_ig[kChunk];  // (1 / p_j, pw_j dp / sqrt(p_j))
+  __shared__ double2 s_pf[2][kSub];  // (p_j, f_j) with f_j = pw_j dp
+  __shared__ double2 s_w[2][kSub];   // (f_j / sqrt p_j, f_j / p_j^1.5)
+  __shared__ double s_q[2][kSub];    // 1 / p_j^2
+  __shared__ int s_line[2];          // the tile lies on the progression
   __shared__ double s_j0[kJ0TabIntervals * kJ0Row];
   extern __shared__ __align__(16) unsigned char s_dyn[];
   double2(*s_R)[kSub][kBsW] = reinterpret_cast<double2(*)[kSub][kBsW]>(s_dyn);  // [kRing]
   const int tid = threadIdx.y * kBsW + threadIdx.x;
   for (int e = tid; e < kJ0TabIntervals * kJ0Row; e += kBsW * kBsR) {
     const int k = e / kJ0Row, n = e - k * kJ0Row;
-    s_j0[e] = n <= kJ0TabDegree ? kJ0Taylor[k][n] : 0.0;  // made visible by the chunk barrier
+    s_j0[e] = n <= kJ0TabDegree ? kJ0Taylor[k][n] : 0.0;  // made visible by the first barrier
   }
   const int lane = threadIdx.x;
   const int iw0 = blockIdx.z * kBsW;
-  const int iw = iw0 + lane;
   const int ir = blockIdx.y * kBsR + threadIdx.y;
   const int j_begin = blockIdx.x * p_per_slice;
   const int j_end = min(n_p, j_begin + p_per_slice);
-  const bool active = iw < n_w && ir < n_r;
-  const double om = active ? omega[iw] : 0.0;
-  const double r = active ? offsets[ir] : 0.0;
+  const bool working = ir < n_r;  // a warp without an offset only stages
+  // lanes beyond the grid repeat its last frequency, so that they take their warp's path
+  const double om = omega[min(iw0 + lane, n_w - 1)];
+  const double r = working ? offsets[ir] : 0.0;
   const double omr = om * r;
-  // per-thread factors of 1 / x and sqrt(1 / (pi x)) with x = omr p (used where x >= 25)
-  const double inv_omr = omr > 0.0 ? 1.0 / omr : 0.0;
-  const double isq_pomr = omr > 0.0 ? rsqrt(3.14159265358979323846 * omr) : 0.0;
+  // z^2 and what it meets stay finite, or x is 0 throughout; for the whole warp, whose lanes
+  // vote below
+  const bool regular =
+      __all_sync(0xffffffffu, (omr >= 1e-100 && omr <= 1e100) || omr == 0.0);
+  const double z = omr > 0.0 ? 1.0 / omr : 0.0;
   // Linear model of the slice's slownesses: p_j ~ p0 + (j - j_begin) * step.
   const double p0 = __ldg(p + j_begin);
   const double step =
       (j_end - j_begin >= 2) ? (__ldg(p + j_end - 1) - p0) / (double)(j_end - 1 - j_begin) : 0.0;
   double sd, cdl;
   sincos(omr * step, &sd, &cdl);
-  double c = 0.0, s = 0.0;
-  int since = kRotSteps;  // steps since the last exact anchor (kRotSteps: none valid)
+  // shears up to 2 pi / 3, where tan(d / 2) is 1.7 (the whole warp, or products)
+  const bool shear = __all_sync(0xffffffffu, cdl >= -0.5);
+  const double half_tan = sd / (1.0 + cdl);
   double ax = 0.0, ay = 0.0;  // fast-path terms, without the factor 1 / sqrt(pi omega r)
   double bx = 0.0, by = 0.0;  // other terms, complete
-  for (int jc = j_begin; jc < j_end; jc += kChunk) {
-    const int n = min(kChunk, j_end - jc);
-    __syncthreads();  // the previous chunk's readers of s_pf, s_ig, s_R are done
+  const int n = j_end - j_begin, ntile = (n + kSub - 1) / kSub;
+  auto prepare = [&](int t) {  // one warp
+    const int b = t & 1, j = t * kSub + lane;
     bool ok = true;
-    if (tid < n) {
-      const int j = jc + tid;
-      const double pj = __ldg(p + j);
-      const double f = __ldg(pw + j) * dp;
-      s_pf[tid] = make_double2(pj, f);
-      s_ig[tid] = make_double2(1.0 / pj, f * rsqrt(pj));
-      const double lin = fma((double)(j - j_begin), step, p0);
-      ok = fabs(pj - lin) <= 1e-15 * fabs(pj);
+    if (j < n) {
+      const double pj = __ldg(p + j_begin + j);
+      const double f = __ldg(pw + j_begin + j) * dp;
+      const double y = 1.0 / pj;
+      const double w = f * rsqrt(pj);
+      s_pf[b][lane] = make_double2(pj, f);
+      s_w[b][lane] = make_double2(w, w * y);
+      s_q[b][lane] = y * y;
+      ok = fabs(pj - fma((double)j, step, p0)) <= 1e-15 * fabs(pj);
     }
-    const int nsub = (n + kSub - 1) / kSub;
-    // tiles 0 and 1 now, tile sb + 2 in iteration sb; every thread commits one group per
-    // step (empty ones included), so wait_group 1 at iteration sb means tile sb has landed
-    stage_R(s_R[0], R, jc, min(kSub, n), iw0, n_w);
+    ok = __all_sync(0xffffffffu, ok);
+    if (lane == 0) s_line[b] = ok;
+  };
+  // tiles 0 and 1 now, tile t + 2 in iteration t; every thread commits one group per step (empty
+  // ones included), so wait_group 1 at iteration t means tile t has landed
+  stage_R(s_R[0], R, j_begin, min(kSub, n), iw0, n_w);
+  cp_async_commit();
+  if (ntile > 1) stage_R(s_R[1], R, j_begin + kSub, min(kSub, n - kSub), iw0, n_w);
+  cp_async_commit();
+  if (threadIdx.y == 0) prepare(0);
+  for (int t = 0, ring = 0; t < ntile; ++t, ring = ring == kRing - 1 ? 0 : ring + 1) {
+    cp_async_wait_1();  // this thread's copies of tile t have landed
+    __syncthreads();    // ... and every thread's; every thread is done with tile t - 1
+    if (t + 2 < ntile)
+      stage_R(s_R[ring == 0 ? kRing - 1 : ring - 1], R, j_begin + (t + 2) * kSub,
+              min(kSub, n - (t + 2) * kSub), iw0, n_w);
     cp_async_commit();
-    if (nsub > 1) stage_R(s_R[1], R, jc + kSub, min(kSub, n - kSub), iw0, n_w);
-    cp_async_commit();
-    const bool uniform = __syncthreads_and(ok) != 0;
-    if (!uniform) since = kRotSteps;
-    const bool rising = active && uniform && step > 0.0 && omr > 0.0;
-    for (int sb = 0; sb < nsub; ++sb) {
-      cp_async_wait_1();  // this thread's copies of tile sb have landed
-      __syncthreads();    // ... and every thread's; every thread is done with tile sb - 1
-      if (sb + 2 < nsub)
-        stage_R(s_R[(sb + 2) % kRing], R, jc + (sb + 2) * kSub,
-                min(kSub, n - (sb + 2) * kSub), iw0, n_w);
-      cp_async_commit();
-      const double2(*tile)[kBsW] = s_R[sb % kRing];
-      const int k0 = sb * kSub, m = min(kSub, n - k0);
-      // Fast tile: slownesses in arithmetic progression with x increasing from >= 25, so
-      // every term takes the asymptotic branch with the anchor / rotation scheme (no
-      // data-dependent branches in the inner loop).  The number of expansion terms follows
-      // from the tile's smallest argument.
-      const double x_first = (om * s_pf[k0].x) * r;
-      const bool fast = rising && x_first >= kJ0X0;
-      const int nt = x_first >= 3000.0 ? 2 : x_first >= 300.0 ? 3 : x_first >= 100.0 ? 4
-                   : x_first >= 60.0 ? 5 : 7;
-      if (fast) {
-        since = kRotSteps;
-        switch (nt) {
-          case 2: fast_tile<2>(s_pf, s_ig, tile, k0, m, lane, om, r, inv_omr, cdl, sd, ax, ay); break;
-          case 3: fast_tile<3>(s_pf, s_ig, tile, k0, m, lane, om, r, inv_omr, cdl, sd, ax, ay); break;
-          case 4: fast_tile<4>(s_pf, s_ig, tile, k0, m, lane, om, r, inv_omr, cdl, sd, ax, ay); break;
-          case 5: fast_tile<5>(s_pf, s_ig, tile, k0, m, lane, om, r, inv_omr, cdl, sd, ax, ay); break;
-          default: fast_tile<7>(s_pf, s_ig, tile, k0, m, lane, om, r, inv_omr, cdl, sd, ax, ay); break;
-        }
-      } else if (active) {
-        // not unrolled: fewer spills at 64 registers, 2.593 vs 2.615 ms (unroll 4) and
-        // 2.723 (unroll 8) on the 21-layer gather grid, U bit-identical
+    if (t + 1 < ntile && threadIdx.y == (t + 1) % kBsR) prepare(t + 1);
+    if (!working) continue;
+    const double2* r_p = &s_R[ring][0][lane];
+    const double2 *pf_p = s_pf[t & 1], *w_p = s_w[t & 1];
+    const double* q_p = s_q[t & 1];
+    const int m = min(kSub, n - t * kSub);
+    const bool rising = s_line[t & 1] && step > 0.0 && regular;
+    // Fast tile: slownesses in arithmetic progression with x increasing from >= 25 in every
+    // lane, so every term takes the asymptotic branch with the anchor / rotation scheme (no
+    // data-dependent branches in the inner loop).  The number of expansion terms follows
+    // from the warp's smallest argument.
+    const double x_first = (om * pf_p[0].x) * r;
+    const int nt = x_first >= 3000.0 ? 2 : x_first >= 300.0 ? 3 : x_first >= 100.0 ? 4
+                 : x_first >= 60.0 ? 5 : x_first >= kJ0X0 ? 7 : 8;
+    const int terms = __reduce_max_sync(0xffffffffu, rising ? nt : 8);
+    if (terms < 8) {
+      double s, c;
+      sincos(x_first, &s, &c);
+      const TileTurn d = {half_tan * omr, sd * z, cdl, sd * omr};
+      const double u = c + s, v = (c - s) * z, z2 = z * z;
+      switch (terms) {
+        case 2: fast_tile<2>(w_p, q_p, r_p, m, shear, z2, d, u, v, ax, ay); break;
+        case 3: fast_tile<3>(w_p, q_p, r_p, m, shear, z2, d, u, v, ax, ay); break;
+        case 4: fast_tile<4>(w_p, q_p, r_p, m, shear, z2, d, u, v, ax, ay); break;
+        case 5: fast_tile<5>(w_p, q_p, r_p, m, shear, z2, d, u, v, ax, ay); break;
+        default: fast_tile<7>(w_p, q_p, r_p, m, shear, z2, d, u, v, ax, ay); break;
+      }
+      continue;
+    }
+    if (rising && __all_sync(0xffffffffu, (om * pf_p[m - 1].x) * r < kJ0X0)) {
+      // every term from the table
+#pragma unroll 2
+      for (int k = 0; k < m; ++k) {
+        const double2 pf = pf_p[k];
+        const double2 rv = r_p[k * kBsW];
+        const double t = j0_table(s_j0, (om * pf.x) * r) * pf.y;
+        bx = fma(t, rv.x, bx);
+        by = fma(t, rv.y, by);
+      }
+    } else if (rising) {
+      // the tile crosses x = 25
+      double s, c;
+      sincos(x_first, &s, &c);
+      const double sn = sd * z, s1 = sd * omr, z2 = z * z;
+      double u = c + s, v = (c - s) * z;
 #pragma unroll 1
-        for (int k = 0; k < m; ++k) {
-          const double2 pf = s_pf[k0 + k];
-          const double2 rv = tile[k][lane];
-          const double x = (om * pf.x) * r;
-          double jv;
-          if (x < kJ0X0) {
-            jv = x > -kJ0X0 ? j0_table(s_j0, fabs(x)) : j0(x);
-            since = kRotSteps;
-          } else {
-            if (since < kRotSteps) {
-              const double c2 = fma(c, cdl, -s * sd);
-              s = fma(s, cdl, c * sd);
-              c = c2;
-              ++since;
-            } else {
-              sincos(x, &s, &c);
-              since = uniform ? 1 : kRotSteps;
-            }
-            jv = j0_asymptotic(x, c, s);
-          }
-          const double t = jv * pf.y;
+      for (int k = 0; k < m; ++k) {
+        const double2 pf = pf_p[k];
+        const double2 rv = r_p[k * kBsW];
+        const double x = (om * pf.x) * r;
+        if (x < kJ0X0) {
+          const double t = j0_table(s_j0, x) * pf.y;
           bx = fma(t, rv.x, bx);
           by = fma(t, rv.y, by);
+        } else {
+          const double2 w = w_p[k];
+          double P, Q;
+          hankel_series<kJ0Terms>(q_p[k] * z2, P, Q);
+          const double t = fma(w.x, P * u, w.y * (Q * v));
+          ax = fma(t, rv.x, ax);
+          ay = fma(t, rv.y, ay);
         }
+        const double u2 = fma(u, cdl, v * s1);
+        v = fma(v, cdl, -u * sn);
+        u = u2;
+      }
+    } else {
+      // slownesses off the progression, offset 0, omega 0: each term by itself
+#pragma unroll 1
+      for (int k = 0; k < m; ++k) {
+        const double2 pf = pf_p[k];
+        const double2 rv = r_p[k * kBsW];
+        const double x = (om * pf.x) * r;
+        double jv;
+        if (x < kJ0X0) {
+          jv = x > -kJ0X0 ? j0_table(s_j0, fabs(x)) : j0(x);
+        } else {
+          double s, c;
+          sincos(x, &s, &c);
+          jv = j0_asymptotic(x, c, s);
+        }
+        const double t = jv * pf.y;
+        bx = fma(t, rv.x, bx);
+        by = fma(t, rv.y, by);
       }
     }
   }
-  if (active)
-    partial[((size_t)blockIdx.x * n_r + ir) * n_w + iw] =
-        make_double2(fma(ax, isq_pomr, bx) * om, fma(ay, isq_pomr, by) * om);
-}
-
-__global__ void reduce_slices_kernel(const double2* __restrict__ partial, int n_slices,
-                                     size_t n_elem, double2* __restrict__ U) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n_elem;
-       i += (size_t)gridDim.x * blockDim.x) {
-    double x = 0.0, y = 0.0;
-    for (int s = 0; s < n_slices; ++s) {
-      double2 v = partial[(size_t)s * n_elem + i];
-      x += v.x;
-      y += v.y;
-    }
-    U[i] = make_double2(x, y);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (working && iw0 + lane < n_w) {
+    const double amp = omr > 0.0 ? rsqrt(3.14159265358979323846 * omr) : 0.0;
+    partial[((size_t)blockIdx.x * n_r + ir) * n_w + iw0 + lane] =
+        make_double2(fma(ax, amp, bx) * om, fma(ay, amp, by) * om);
   }
 }
 
+// U = sum of the slices' partials: 32 elements per block, eight threads per element (slices s,
+// s + 8, ...), whose sums are added in order.
+__global__ void __launch_bounds__(256)
+reduce_slices_kernel(const double2* __restrict__ partial, int n_slices, size_t n_elem,
+                     double2* __restrict__ U) {
+  __shared__ double2 s_sum[8][32];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+  const size_t i = blockIdx.x * (size_t)32 + lane;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  double x = 0.0, y = 0.0;
+  if (i < n_elem) {
+#pragma unroll 4
+    for (int s = part; s < n_slices; s += 8) {
+      const double2 v = partial[(size_t)s * n_elem + i];
+      x += v.x;
+      y += v.y;
+    }
+  }
+  s_sum[part][lane] = make_double2(x, y);
+  __syncthreads();
+  if (part != 0 || i >= n_elem) return;
+#pragma unroll
+  for (int k = 1; k < 8; ++k) {
+    x += s_sum[k][lane].x;
+    y += s_sum[k][lane].y;
+  }
+  U[i] = make_double2(x, y);
+}
+
+// The sum of the slices starts its launch while the last of them finish.
+static kr_status launch_reduce(const double2* partial, int n_slices, size_t n_elem, double* U,
+                               cudaStream_t st, const char* where) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((n_elem + 31) / 32));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, reduce_slices_kernel, partial, n_slices, n_elem,
+                                           reinterpret_cast<double2*>(U));
+  if (e != cudaSuccess) set_last_error(where, e);
+  return cuda_status(e);
+}
+
 // The R ring lives in dynamic shared memory above the 48 KB default (with the static arrays
-// ~56 KB per block, four blocks per SM); the limit is raised once per device.
+// ~54 KB per block, four blocks per SM); the limit is raised once per device.
 static SmemLimit g_ring_limit;
 static kr_status bessel_ring_attribute(const char* where) {
   return raise_smem_limit((const void*)bessel_partial_kernel, kRingBytes, g_ring_limit, where);
@@ -337,20 +434,23 @@ struct BesselPlan {
   size_t partial_bytes;
 };
 
+static int whole_tiles(int n) { return (n + kSub - 1) / kSub * kSub; }
+
 static BesselPlan bessel_plan(int n_p, int n_w, int n_r) {
   BesselPlan b;
   const long long tiles = (long long)((n_w + kBsW - 1) / kBsW) * ((n_r + kBsR - 1) / kBsR);
-  // About 96 blocks of 256 threads per SM in total (~24 waves at 4 resident blocks per SM:
-  // shorter blocks even out the slow low-frequency tiles; on the 21-layer gather grid
-  // 2.612 ms against 2.633 at 64 and 2.623 at 128; with three resident blocks 2.65 at 64,
-  // 2.73 at 32, 2.85 at 16), but no slice shorter than 64 slownesses.
+  // About 96 blocks of 256 threads per SM in total (~24 waves at 4 resident blocks per SM: shorter
+  // blocks even out the slow low-frequency tiles; 8192 slownesses x 2047 frequencies x 100 offsets
+  // take 2.467 ms, 2.474 at 64 and 2.468 at 160), but no slice shorter than two tiles
+  // (2048 x 511 x 37: 100 us, 105 with three tiles, 109 with four; one tile takes 100 there but 175
+  // against 163 at 6000 x 1000 x 10, where the slices' prologues weigh more).
   const long long target = 148LL * 96;
   long long s = (target + tiles - 1) / (tiles > 0 ? tiles : 1);
   long long smax = (n_p + 63) / 64;
   if (s > smax) s = smax;
   if (s < 1) s = 1;
   if (s > 65535) s = 65535;
-  b.p_per_slice = (int)((n_p + s - 1) / s);
+  b.p_per_slice = whole_tiles((int)((n_p + s - 1) / s));
   b.n_slices = (int)((n_p + b.p_per_slice - 1) / b.p_per_slice);
   if (b.n_slices < 1) b.n_slices = 1;
   b.partial_bytes = (size_t)b.n_slices * n_r * n_w * sizeof(double2);
@@ -474,12 +574,7 @@ extern "C" kr_status kr_bessel_sum(const double* R, const double* p, const doubl
       b.p_per_slice, partial);
   kr_status s = check_launch("kr_bessel_sum: partial");
   if (s != KR_OK) return s;
-  const size_t n_elem = (size_t)n_r * n_w;
-  int blocks = (int)((n_elem + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  reduce_slices_kernel<<<blocks, 256, 0, st>>>(partial, b.n_slices, n_elem,
-                                               reinterpret_cast<double2*>(U));
-  return check_launch("kr_bessel_sum: reduce");
+  return launch_reduce(partial, b.n_slices, (size_t)n_r * n_w, U, st, "kr_bessel_sum: reduce");
 }
 
 extern "C" size_t kr_traces_workspace_bytes(int32_t n_r, int32_t nw) {
@@ -644,7 +739,7 @@ extern "C" kr_status kr_bessel_sum_noalloc(const double* R, const double* p, con
   BesselPlan b = bessel_plan(n_p, n_w, n_r);
   const int cap = (int)(kNoAllocScratchBytes / slice_bytes);
   int n_slices = b.n_slices < cap ? b.n_slices : cap;
-  const int p_per_slice = (n_p + n_slices - 1) / n_slices;
+  const int p_per_slice = whole_tiles((n_p + n_slices - 1) / n_slices);
   n_slices = (n_p + p_per_slice - 1) / p_per_slice;
   double2* partial = reinterpret_cast<double2*>(scratch);
   dim3 grid(n_slices, (n_r + kBsR - 1) / kBsR, (n_w + kBsW - 1) / kBsW);
@@ -655,10 +750,6 @@ extern "C" kr_status kr_bessel_sum_noalloc(const double* R, const double* p, con
       p_per_slice, partial);
   s = check_launch("kr_bessel_sum_noalloc: partial");
   if (s != KR_OK) return s;
-  const size_t n_elem = (size_t)n_r * n_w;
-  int blocks = (int)((n_elem + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  reduce_slices_kernel<<<blocks, 256, 0, st>>>(partial, n_slices, n_elem,
-                                               reinterpret_cast<double2*>(U));
-  return check_launch("kr_bessel_sum_noalloc: reduce");
+  return launch_reduce(partial, n_slices, (size_t)n_r * n_w, U, st,
+                       "kr_bessel_sum_noalloc: reduce");
 }
