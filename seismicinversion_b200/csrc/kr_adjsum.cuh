@@ -13,9 +13,15 @@ namespace kr {
 // ------------------------------------------------------------------------------------------
 // Phase factors ea, eb of one lane for the derivative sweeps, on tiles of the grid's line
 // (kr_phase.cuh): lo[j] = exp(j delta c), j < 16, shared by the block, and, per warp and pass of
-// 32 frequencies from kb, hm[m] = exp(omega_{kb + 16 m} c), m < 2, each one direct exp, so a
+// 32 frequencies from kb, hm[m], m < 2: the forward sweep's hi mid at frequency kb + 16 m, so a
 // lookup is one product of two reads at fixed offsets.  The derivatives need ea and eb
 // themselves in the reverse sweep, so these two are tabulated, not P, Q, S.
+//
+// hm is exp(omega_{kb + 16 m} c) as the forward sweep rounds it, not the closer direct exp: the
+// rounding of omega_{128 u} c is common to a tile's frequencies, and a misfit's adjoint made from
+// the forward sweep's R meets this sweep's R in sums over frequency where all but their difference
+// cancels.  With direct exps the water layer's alpha and h gradients of 5- to 31-layer models on 4
+// to 63 slownesses had errors of up to 1.3e-12 of the largest entry, instead of 3e-14.
 //
 // Models of up to kRayTabLayers layers tabulate: a 48-layer block of the batched gradient is
 // 107 KB, two per SM; above, the table would cost a resident block.  Every derivative kernel
@@ -55,6 +61,16 @@ __device__ __forceinline__ bool ray_lo_fill(const GridLine& g, int n_layers, con
   return ok;
 }
 
+// exp(a + b) without the rounding of a + b: the sum's remainder (Knuth's two-sum) enters to first
+// order, exactly enough as it is below an ulp of the sum.
+__device__ __forceinline__ cd cexp_sum(cd a, cd b) {
+  const cd s = a + b;
+  const double tx = s.x - a.x, ty = s.y - a.y;
+  const cd r = mk((a.x - (s.x - tx)) + (b.x - tx), (a.y - (s.y - ty)) + (b.y - ty));
+  const cd v = cexp_(s);
+  return v + v * r;
+}
+
 // Warp-cooperative: the hm entries of the pass from frequency kb; returns (warp-uniform) whether
 // all are usable.
 __device__ __forceinline__ bool ray_hm_fill(const double2* __restrict__ omega, int n_w, int kb,
@@ -62,9 +78,12 @@ __device__ __forceinline__ bool ray_hm_fill(const double2* __restrict__ omega, i
   bool bad = false;
   const int lane = threadIdx.x & 31;
   // lanes take m = lane & 1 of phase id; past the grid's end the entry is not used
-  const double2 w = omega[min(kb + kPhLo * (lane & 1), n_w - 1)];
+  const GridLine g = grid_line(omega, n_w);
+  const double2 w = omega[min(kb & ~(kPhTile - 1), n_w - 1)];
+  const cd mid = (double)((kb & (kPhTile - 1)) + kPhLo * (lane & 1)) * g.d;
   for (int e = lane; e < 4 * (n_layers - 1); e += 32) {
-    const cd v = cexp_(mk(w.x, w.y) * sweep_exponent<2>(lay, e >> 1));
+    const cd c = sweep_exponent<2>(lay, e >> 1);
+    const cd v = cexp_sum(mk(w.x, w.y) * c, mid * c);
     bad |= !phase_usable(v);
     hm[e] = v;
   }

@@ -7,10 +7,9 @@
 //     exp(omega_k c) = (hi[u] * mid[t / 16]) * lo[t % 16],
 //     lo[j] = exp(j delta c) (j < 16),  mid[m] = exp(16 m delta c) (m < 8),
 //     hi[u] = exp(omega_{128 u} c)       (the tile's own first frequency)
-// in the forward kernels (kr_sweep.cuh), with hi mid = exp(omega_{128 u + 16 m} c) evaluated
-// directly in the derivative kernels (kr_adjsum.cuh); each entry is one direct exp of an exactly
-// formed argument, and a product of table reads replaces an exp and a sincos per layer, phase
-// and frequency.  A tile whose frequencies leave the line, or whose entries exceed 1e100 in
+// in the forward kernels (kr_sweep.cuh); the derivative kernels (kr_adjsum.cuh) keep hi mid as
+// one entry of the same rounding.  Each entry is one direct exp of an exactly formed argument,
+// and a product of table reads replaces an exp and a sincos per layer, phase and frequency.  A tile whose frequencies leave the line, or whose entries exceed 1e100 in
 // magnitude (so that no product can overflow), evaluates its phases directly.
 #pragma once
 
