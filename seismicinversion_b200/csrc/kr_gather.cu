@@ -434,7 +434,9 @@ struct BesselPlan {
   size_t partial_bytes;
 };
 
-static int whole_tiles(int n) { return (n + kSub - 1) / kSub * kSub; }
+static int whole_tiles(int n) {
+  return n > 0x7fffffff - kSub ? n : (n + kSub - 1) / kSub * kSub;
+}
 
 static BesselPlan bessel_plan(int n_p, int n_w, int n_r) {
   BesselPlan b;
