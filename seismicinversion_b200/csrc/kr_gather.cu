@@ -19,6 +19,7 @@
 #include <mutex>
 #include <vector>
 
+#include "kr_bessel.cuh"
 #include "kr_internal.cuh"
 #include "kr_j0_table.h"
 
@@ -81,16 +82,12 @@ __device__ __forceinline__ double j0_asymptotic(double x, double c, double s) {
 
 // J0(x) for 0 <= x < 25 from the piecewise Taylor table (kr_j0_table.h, staged in shared
 // memory with rows padded to kJ0Row doubles so that lanes on different intervals fall on
-// different banks): interval k and t = x - (k + 1/2) from one rounding (no conversions, which
-// are slow for 64 bits; an integer x may take either neighbour), degree-15 Horner in t.
+// different banks): interval and offset t by j0_interval, degree-15 Horner in t.
 // Absolute error below 5e-16 against SciPy's j0 on [0, 25).
 constexpr int kJ0Row = kJ0TabDegree + 2;
 __device__ __forceinline__ double j0_table(const double* s_j0, double x) {
-  constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52
-  const double w = x - 0.5;
-  const double z = w + kRound;
-  const double t = w - (z - kRound);
-  const double* a = s_j0 + min(__double2loint(z), kJ0TabIntervals - 1) * kJ0Row;
+  double t;
+  const double* a = s_j0 + j0_interval(x, kJ0TabIntervals, t) * kJ0Row;
   double v = a[kJ0TabDegree];
 #pragma unroll
   for (int n = kJ0TabDegree - 1; n >= 0; --n) v = fma(v, t, a[n]);
@@ -285,7 +282,7 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
     const double2 *pf_p = s_pf[t & 1], *w_p = s_w[t & 1];
     const double* q_p = s_q[t & 1];
     const int m = min(kSub, n - t * kSub);
-    const bool rising = s_line[t & 1] && step > 0.0 && regular;
+    const bool rising = rising_tile(s_line[t & 1] != 0, step, pf_p[0].x, regular);
     // Fast tile: slownesses in arithmetic progression with x increasing from >= 25 in every
     // lane, so every term takes the asymptotic branch with the anchor / rotation scheme (no
     // data-dependent branches in the inner loop).  The number of expansion terms follows
@@ -346,7 +343,8 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
         u = u2;
       }
     } else {
-      // slownesses off the progression, offset 0, omega 0: each term by itself
+      // slownesses off the progression, falling or below zero, a negative or extreme omega r: each
+      // term by itself
 #pragma unroll 1
       for (int k = 0; k < m; ++k) {
         const double2 pf = pf_p[k];
