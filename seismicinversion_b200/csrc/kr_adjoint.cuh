@@ -291,7 +291,7 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
     ob0 = ob0 * seed;
     f0 = f0 * seed;
   }
-  Ray g = {csqrt(ob0), mk(0.0, 0.0)};
+  Ray g = {csqrt_any(ob0), mk(0.0, 0.0)};
   AccT cur, nxt;
   acc_zero(cur);
   acc_zero(nxt);
@@ -416,7 +416,7 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
   const cd ob0 = ((e0 * e0) * dy) * seed;
   const cd f0 = (2.0 * (e0 * r.a) * dy * e0 * w) * seed;
   sink.top(f0);
-  Ray g = {csqrt(ob0), mk(0.0, 0.0)};
+  Ray g = {csqrt_any(ob0), mk(0.0, 0.0)};
   for (int q = ncp - 1; q >= 0; --q) {
     const int s0 = q * seg;
     const int s1 = s0 + seg < nsteps ? s0 + seg : nsteps;

@@ -52,7 +52,7 @@ struct HessRaySink {
       const cd zeta = fs ? (-2.0 * seed) * recip(1.0 - R) : mk(0.0, 0.0);
       seeds[0] = make_double2(seed.x, seed.y);
       seeds[1] = make_double2(zeta.x, zeta.y);
-      sigma = csqrt(seed);
+      sigma = csqrt_any(seed);
     }
     return mk(1.0, 0.0);
   }

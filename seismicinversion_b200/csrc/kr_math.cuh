@@ -91,12 +91,32 @@ KR_HD cd operator/(cd a, cd b) { return a * recip(b); }
 KR_HD cd operator/(cd a, double s) { return mk(a.x / s, a.y / s); }
 
 // Principal square root, branch cut on the negative real axis, sqrt(conj z) = conj sqrt z
-// (C99 csqrt semantics, the convention NumPy and torch use).
+// (C99 csqrt semantics, the convention NumPy and torch use).  For slownesses and their products;
+// near the ends of the range see csqrt_any.
 KR_HD cd csqrt(cd z) {
   if (z.x == 0.0 && z.y == 0.0) return mk(0.0, z.y);
   double t = sqrt(0.5 * (fabs(z.x) + hypot(z.x, z.y)));
   if (z.x >= 0.0) return mk(t, z.y / (2.0 * t));
   return mk(fabs(z.y) / (2.0 * t), copysign(t, z.y));
+}
+
+// csqrt of any magnitude, scaled by a power of four near the ends of the range: of a subnormal,
+// csqrt's half sum may round to zero and leave y / (2 t) infinite; of a value near the largest it
+// may overflow.  For what data decide: the adjoint of an evanescent water phase underflows
+// gradually.  (Apart from csqrt, whose chain is the latency of every prologue: scaled there too,
+// the 64 x 1024 gradient of 21 layers takes 75.8 us instead of 75.0.)
+KR_HD cd csqrt_any(cd z) {
+  const double m = fmax(fabs(z.x), fabs(z.y));
+  double s = 1.0, back = 1.0;
+  if (m < 0x1p-960) {
+    s = 0x1p120;
+    back = 0x1p-60;
+  } else if (m > 0x1p960) {
+    s = 0.25;
+    back = 2.0;
+  }
+  const cd r = csqrt(mk(z.x * s, z.y * s));
+  return mk(r.x * back, r.y * back);
 }
 
 KR_HD cd cexp_(cd z) {
