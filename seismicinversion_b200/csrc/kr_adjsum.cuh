@@ -54,7 +54,7 @@ __device__ __forceinline__ bool ray_lo_fill(const GridLine& g, int n_layers, con
                                             cd* lo) {
   bool ok = true;
   for (int e = threadIdx.x; e < 2 * (n_layers - 1) * kPhLo; e += blockDim.x) {
-    const cd v = cexp_(((double)(e % kPhLo) * g.d) * sweep_exponent<2>(lay, e / kPhLo));
+    const cd v = cexp_(((double)(e % kPhLo) * g.d) * sweep_exponent(lay, e / kPhLo));
     ok &= phase_usable(v);
     lo[e] = v;
   }
@@ -82,7 +82,7 @@ __device__ __forceinline__ bool ray_hm_fill(const double2* __restrict__ omega, i
   const double2 w = omega[min(kb & ~(kPhTile - 1), n_w - 1)];
   const cd mid = (double)((kb & (kPhTile - 1)) + kPhLo * (lane & 1)) * g.d;
   for (int e = lane; e < 4 * (n_layers - 1); e += 32) {
-    const cd c = sweep_exponent<2>(lay, e >> 1);
+    const cd c = sweep_exponent(lay, e >> 1);
     const cd v = cexp_sum(mk(w.x, w.y) * c, mid * c);
     bad |= !phase_usable(v);
     hm[e] = v;

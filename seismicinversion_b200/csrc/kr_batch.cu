@@ -228,9 +228,9 @@ __device__ __forceinline__ void forward_item(const ItemRec& item, const kr_model
     const int m0 = n_tiles > 1 ? 0 : (item.w0 % kPhTile) / kPhLo;
     const int m1 = n_tiles > 1 ? kPhMid : ((item.w0 + item.nw - 1) % kPhTile) / kPhLo + 1;
     const int per = kPhLo + m1 - m0;
-    for (int e = threadIdx.x; e < NPH * I * per; e += THREADS) {
-      const int id = e / per, j = e - id * per;
-      bad |= !sweep_table_entry<N>(g, lay, id, j < kPhLo ? j : j + m0, tab);
+    for (int e = threadIdx.x; e < I * per; e += THREADS) {
+      const int l = e / per, j = e - l * per;
+      bad |= !sweep_table_entry<N>(g, lay, l, j < kPhLo ? j : j + m0, tab);
     }
   }
   const bool ok = __syncthreads_or(bad) == 0;

@@ -49,9 +49,10 @@ sweep_kernel(const double* __restrict__ tab, int L, const double* __restrict__ p
     const GridLine line = grid_line(omega, n_w);
     sweep_tiles_check(omega, n_w, line, t0, t1 - t0, s_tiles);
     unsigned bad = 0u;
-    for (int e = threadIdx.x; e < ng * n_ent; e += 32 * W) {
-      const int g = e / n_ent, id = (e - g * n_ent) / kPhHead, j = e % kPhHead;
-      if (!sweep_table_entry<N>(line, s_lay + g * L, id, j, s_tab + (size_t)g * n_ent))
+    for (int e = threadIdx.x; e < ng * I * kPhHead; e += 32 * W) {
+      const int gl = e / kPhHead, g = gl / I;
+      if (!sweep_table_entry<N>(line, s_lay + g * L, gl - g * I, e - gl * kPhHead,
+                                s_tab + (size_t)g * n_ent))
         bad |= 1u << g;
     }
     if (bad) atomicOr(&s_bad, bad);

@@ -4,11 +4,14 @@
 //
 // What bounds it is the FP64 pipe: ~115 FP64 instructions per (omega, p, interface) in
 // kennett_step_x when the squared and mixed phase factors P = ea^2, Q = eb^2, S = ea eb come
-// from a table.  The table holds, per phase exponent c (2 i eta h, 2 i neta h, i (eta + neta) h
-// of every layer above the half-space), lo[j] = exp(j delta c), j < 16, and
-// mid[m] = exp(16 m delta c), m < 8; a warp forms hi = exp(omega_{128 u} c) of its tile u times
-// the mid entries of its own frequencies once per pass (hm), so a lookup is one complex product
-// of two shared-memory reads.  Models too deep for three phases per layer in shared memory
+// from a table.  The table holds, for the phases exp(omega c) with c = i eta h and i neta h of
+// every layer above the half-space, lo[j] = exp(j delta c), j < 16, and mid[m] = exp(16 m delta c),
+// m < 8, as their squares and product; a warp forms hi = exp(omega_{128 u} c) of its tile u (again
+// squares and product) times the mid entries of its own frequencies once per pass (hm), so a
+// lookup is one complex product of two shared-memory reads.  P, Q and S come from the same two
+// exponentials so that S^2 = P Q holds to a few roundings whatever the rounding of omega c: models
+// near a pole amplify a mismatch (exp of 2 c and of the sums instead: global-matrix R of the
+// 5-layer model off by 1.8 times as much at 0.7 to 1 s/km).  Models too deep for three phases per layer in shared memory
 // tabulate ea and eb alone (two lookups and three more products per step); models deeper still
 // evaluate exponentials directly, as do tiles that are off the grid's line (kr_phase.cuh).
 //
@@ -42,27 +45,29 @@ __host__ __device__ inline size_t sweep_warp_bytes(int n_layers, int nph, int F)
   return sizeof(cd) * 2 * F * nph * (size_t)(n_layers - 1);
 }
 
-// Exponent `id` (NPH l + k) of a model.
-template <int NPH>
+// Exponent `id` (2 l + k) of a model: i eta h of layer l, or i neta h.
 __device__ __forceinline__ cd sweep_exponent(const LayerP* lay, int id) {
-  const LayerP& lp = lay[id / NPH];
-  const int k = id % NPH;
-  if (NPH == 2) return k ? lp.cb : lp.ca;
-  return k == 0 ? 2.0 * lp.ca : k == 1 ? 2.0 * lp.cb : lp.ca + lp.cb;
+  const LayerP& lp = lay[id >> 1];
+  return id & 1 ? lp.cb : lp.ca;
 }
 
 __device__ __forceinline__ bool phase_usable(cd v) {
   return fabs(v.x) <= kPhMaxMag && fabs(v.y) <= kPhMaxMag;
 }
 
-// Entry j (lo, then mid) of phase `id` of a slowness's table; returns whether it is usable.
+// Entry j (lo, then mid) of every phase of layer l of a slowness's table; returns whether they are
+// usable.
 template <int NPH>
-__device__ __forceinline__ bool sweep_table_entry(const GridLine& g, const LayerP* lay, int id,
+__device__ __forceinline__ bool sweep_table_entry(const GridLine& g, const LayerP* lay, int l,
                                                   int j, cd* tab) {
   const cd z = (double)(j < kPhLo ? j : (j - kPhLo) * kPhLo) * g.d;
-  const cd v = cexp_(z * sweep_exponent<NPH>(lay, id));
-  tab[id * kPhHead + j] = v;
-  return phase_usable(v);
+  const cd a = cexp_(z * lay[l].ca), b = cexp_(z * lay[l].cb);
+  cd* t = tab + (size_t)NPH * l * kPhHead + j;
+  const cd u = NPH == 3 ? a * a : a, v = NPH == 3 ? b * b : b;
+  t[0] = u;
+  t[kPhHead] = v;
+  if (NPH == 3) t[2 * kPhHead] = a * b;
+  return phase_usable(u) && phase_usable(v);
 }
 
 // The prologue's two stages out of line: one compiled body per kernel file, called by every
@@ -228,18 +233,27 @@ __device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, do
                                            const cd* tab, bool use, cd* hm, bool fs, double2* __restrict__ Rp) {
   const int lane = threadIdx.x & 31;
   constexpr int N = NPH > 0 ? NPH : 1;
-  constexpr int kHi = NPH == 3 ? (3 * (kPqsLayers - 1) + 31) / 32 : (2 * (kPairLayers - 1) + 31) / 32;
-  const int n_phase = N * (n_layers - 1);
-  cd hi[kHi];
+  constexpr int kDeepest = NPH == 3 ? kPqsLayers : kPairLayers;
+  constexpr int kHi = (2 * (kDeepest - 1) + 31) / 32;
+  const int n_exp = 2 * (n_layers - 1);
+  // lanes take the exponents in turn; a layer's two lie in neighbouring lanes, which exchange them
+  // for the product (formed alike by both, which then share its hm entries)
+  cd hi[kHi], hs[NPH == 3 ? kHi : 1];
   if (NPH > 0 && use) {
     bool bad = false;
 #pragma unroll
     for (int r = 0; r < kHi; ++r) {
+      if (32 * r >= n_exp) break;
       const int id = 32 * r + lane;
-      if (id < n_phase) {
-        hi[r] = cexp_(mk(w0.x, w0.y) * sweep_exponent<N>(lay, id));
-        bad |= !phase_usable(hi[r]);
+      cd e = mk(0.0, 0.0);
+      if (id < n_exp) e = cexp_(mk(w0.x, w0.y) * sweep_exponent(lay, id));
+      if (NPH == 3) {
+        const cd o = mk(__shfl_xor_sync(0xffffffffu, e.x, 1), __shfl_xor_sync(0xffffffffu, e.y, 1));
+        hs[r] = (lane & 1) ? o * e : e * o;
+        e = e * e;
       }
+      hi[r] = e;
+      bad |= !phase_usable(e);
     }
     use = !__any_sync(0xffffffffu, bad);
   }
@@ -250,10 +264,20 @@ __device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, do
 #pragma unroll
       for (int r = 0; r < kHi; ++r) {
         const int id = 32 * r + lane;
-        if (id < n_phase) {
-          const cd* mid = tab + id * kPhHead + kPhLo + pass * 2 * F;
+        if (id < n_exp) {
+          const int ph = NPH == 3 ? 3 * (id >> 1) + (id & 1) : id;
+          const cd* mid = tab + ph * kPhHead + kPhLo + pass * 2 * F;
 #pragma unroll
-          for (int m = 0; m < 2 * F; ++m) hm[id * 2 * F + m] = hi[r] * mid[m];
+          for (int m = 0; m < 2 * F; ++m) hm[ph * 2 * F + m] = hi[r] * mid[m];
+          if (NPH == 3) {
+            const int ps = 3 * (id >> 1) + 2;
+            const cd* mids = tab + ps * kPhHead + kPhLo + pass * 2 * F;
+#pragma unroll
+            for (int m = 0; m < F; ++m) {
+              const int k = 2 * m + (id & 1);
+              hm[ps * 2 * F + k] = hs[r] * mids[k];
+            }
+          }
         }
       }
       __syncwarp();
