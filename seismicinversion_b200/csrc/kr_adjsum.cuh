@@ -24,8 +24,10 @@ namespace kr {
 // to 63 slownesses had errors of up to 1.3e-12 of the largest entry, instead of 3e-14.
 //
 // Models of up to kRayTabLayers layers tabulate: a 48-layer block of the batched gradient is
-// 107 KB, two per SM; above, the table would cost a resident block.  Every derivative kernel
-// applies the same rules, so they agree bit for bit.
+// 107 KB, two per SM; from 52 layers the table would cost a resident block.  Deeper models that the
+// forward sweep tabulates (to kPairLayers) evaluate exponentials with the same rounding of the
+// tile's first phase (PhaseLine); beyond, both sides take exp of omega c directly.  Every derivative
+// kernel applies the same rules, so they agree bit for bit.
 // ------------------------------------------------------------------------------------------
 constexpr int kRayTabLayers = 48;
 __host__ __device__ inline bool ray_table_model(int n_layers) { return n_layers <= kRayTabLayers; }
@@ -102,6 +104,35 @@ __device__ __forceinline__ RayTable ray_table(const cd* lo, const cd* hm) {
 __device__ __forceinline__ bool on_line(const GridLine& g, int k, double2 w) {
   return fabs(w.x - fma((double)k, g.d.x, g.w0.x)) <= g.tol &&
          fabs(w.y - fma((double)k, g.d.y, g.w0.y)) <= g.tol;
+}
+
+// Phases of one frequency by direct exponentials.  On a tile of the grid's line, for a model that
+// the forward sweep tabulates, exp(omega_k c) = exp(omega_{128 u} c + (k - 128 u) delta c) with the
+// first product rounded as there: without it, gradients of 49- to 66-layer models made from the
+// forward's R are off by 2.5e-14 of their largest component, with it by less than 1e-15.  Elsewhere
+// w0 is the frequency itself and dw zero.
+struct PhaseLine {
+  cd w0, dw;
+  const LayerP* lay;
+  __device__ __forceinline__ cd at(cd c) const {
+    // the remainder of the sum for |b| <= |a| (Dekker); otherwise, in the grid's first tile, the
+    // rounding it leaves is the frequency's own
+    const cd a = w0 * c, b = dw * c, s = a + b, r = b - (s - a);
+    const cd v = cexp_(s);
+    return cmac(v, v, r);
+  }
+  __device__ __forceinline__ cd a(int l) const { return at(lay[l].ca); }
+  __device__ __forceinline__ cd b(int l) const { return at(lay[l].cb); }
+  __device__ __forceinline__ bool cheap() const { return false; }
+};
+__device__ __forceinline__ bool ray_line_model(int n_layers) { return n_layers <= kPairLayers; }
+
+// The source of frequency k = w; `on`: its tile is on the line and the model is a ray_line_model.
+__device__ __forceinline__ PhaseLine phase_line(bool on, const double2* __restrict__ omega, int n_w,
+                                                int k, cd w, const LayerP* lay) {
+  if (!on) return PhaseLine{w, mk(0.0, 0.0), lay};
+  const double2 w0 = omega[k & ~(kPhTile - 1)];
+  return PhaseLine{mk(w0.x, w0.y), (double)(k & (kPhTile - 1)) * grid_line(omega, n_w).d, lay};
 }
 
 // Staging of the warp sums of 12 explicit values per lane (the dual adjoint of the

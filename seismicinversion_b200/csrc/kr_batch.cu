@@ -324,20 +324,20 @@ struct BatchGradSink {
 #define KR_FOR_PASSES(kb) \
   for (int kb = (item.w0 & ~31) + (int)(threadIdx.x & ~31u); kb < item.w0 + item.nw; kb += THREADS)
 
-// The lo entries and tile verdicts of a gradient item; returns whether the lo entries may be
-// used.  Contains block barriers; all threads call it.
+// The tile verdicts and (models that tabulate) lo entries of a gradient item; returns whether its
+// tiles on the line take the table, or PhaseLine.  Contains block barriers; all threads call it.
 __device__ __forceinline__ bool ray_item_tables(const ItemRec& item, const kr_model_desc& d,
                                                 const double2* om, const LayerP* lay, cd* lo,
                                                 SweepTiles& tiles) {
-  const bool table = ray_table_model(d.n_layers);
+  const bool line = ray_line_model(d.n_layers);
   const int u0 = item.w0 / kPhTile, n = (item.w0 + item.nw - 1) / kPhTile - u0 + 1;
-  if (table) sweep_tiles_clear(tiles, n);
+  if (line) sweep_tiles_clear(tiles, n);
   __syncthreads();
-  bool ok = table;
-  if (table) {
+  bool ok = line;
+  if (line) {
     const GridLine g = grid_line(om, d.n_w);
     sweep_tiles_check(om, d.n_w, g, u0, n, tiles);
-    ok = ray_lo_fill(g, d.n_layers, lay, lo);
+    if (ray_table_model(d.n_layers)) ok = ray_lo_fill(g, d.n_layers, lay, lo);
   }
   return __syncthreads_and(ok) != 0;
 }
@@ -408,12 +408,13 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
       const size_t e = (size_t)pr.j * d.n_w + (valid ? iw : 0);
       sink.obs = obs_all + d.obs_off + e;
       sink.R_out = (d.flags & KR_BATCH_STORE_R) ? R_all + d.R_off + e : nullptr;
-      const bool tab = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0 &&
-                       ray_hm_fill(om, d.n_w, kb, L, v.lay, hm);
+      const bool on = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0;
+      const bool tab = on && ray_table_model(L) && ray_hm_fill(om, d.n_w, kb, L, v.lay, hm);
       if (tab)
         jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan, ray_table(lo, hm), sink);
       else
-        jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan, PhaseDirect{w, v.lay}, sink);
+        jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan,
+                      phase_line(on && !ray_table_model(L), om, d.n_w, iw, w, v.lay), sink);
       __syncwarp();
       double c2 = valid ? (sink.res.x * sink.res.x + sink.res.y * sink.res.y) : 0.0;
       for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);
@@ -492,12 +493,13 @@ batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_al
       sink.acc = acc + (size_t)warp * sum_rows(L) * kRayRow;
       sink.stage = stage + warp * kRayStage;
       sink.I = I;
-      const bool tab = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0 &&
-                       ray_hm_fill(om, d.n_w, kb, L, sl, hm);
+      const bool on = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0;
+      const bool tab = on && ray_table_model(L) && ray_hm_fill(om, d.n_w, kb, L, sl, hm);
       if (tab)
         adjoint_rays(L, w, fs, seg, sc, ray_table(lo, hm), sink);
       else
-        adjoint_rays(L, w, fs, seg, sc, PhaseDirect{w, sl}, sink);
+        adjoint_rays(L, w, fs, seg, sc,
+                     phase_line(on && !ray_table_model(L), om, d.n_w, iw, w, sl), sink);
       __syncwarp();  // the hm entries are read before the next pass overwrites them
       if (valid) c2 += sink.res.x * sink.res.x + sink.res.y * sink.res.y;
     }

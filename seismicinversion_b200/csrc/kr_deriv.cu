@@ -190,15 +190,16 @@ deriv_sweep_kernel(int L, const double* __restrict__ p, int n_p,
   cd* s_lo = reinterpret_cast<cd*>(reinterpret_cast<unsigned char*>(s_wacc) + acc_bytes +
                                    pair_smem_bytes(L));
   cd* hm = s_lo + ray_lo_values(L) + (threadIdx.x >> 5) * ray_hm_values(L);
-  bool use_tab = table != 0;
-  if (use_tab) {
+  const bool tab = table != 0;
+  bool on = ray_line_model(L);  // the tile on the line (and, with a table, its lo entries usable)
+  if (on) {
     const GridLine g = grid_line(omega, n_w);
-    use_tab = ray_lo_fill(g, L, lay, s_lo);
-    if (valid) use_tab &= on_line(g, iw, make_double2(w.x, w.y));
-    use_tab = __syncthreads_and(use_tab) != 0;
-    if (use_tab)
-      use_tab = ray_hm_fill(omega, n_w, tile * kDerThreads + (threadIdx.x & ~31), L, lay, hm);
+    if (tab) on = ray_lo_fill(g, L, lay, s_lo);
+    if (valid) on &= on_line(g, iw, make_double2(w.x, w.y));
+    on = __syncthreads_and(on) != 0;
   }
+  const bool use_tab = tab && on && ray_hm_fill(omega, n_w, tile * kDerThreads + (threadIdx.x & ~31),
+                                                L, lay, hm);
   PairSink<MODE> sink;
   sink.L = L;
   sink.ip = ip;
@@ -212,7 +213,8 @@ deriv_sweep_kernel(int L, const double* __restrict__ p, int n_p,
   if (use_tab)
     jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan, ray_table(s_lo, hm), sink);
   else
-    jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan, PhaseDirect{w, lay}, sink);
+    jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan,
+                  phase_line(on && !tab, omega, n_w, iw, w, lay), sink);
   if (GRAD) {
     const cd res = sink.res;
     double c2 = valid ? (res.x * res.x + res.y * res.y) : 0.0;
@@ -297,15 +299,16 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
   __syncthreads();
   for (int i = threadIdx.x; i < I; i += kDerThreads)
     interface_store(pj, i, s_lay, s_root, s_if + i);
-  bool ok = table != 0;
+  const bool tab = table != 0;
+  bool on = ray_line_model(L);  // the tile on the line (and, with a table, its lo entries usable)
   cd* hm = s_lo + ray_lo_values(L) + warp * ray_hm_values(L);
-  if (ok) {
+  if (on) {
     const GridLine g = grid_line(omega, n_w);
-    ok = ray_lo_fill(g, L, s_lay, s_lo);
-    if (valid) ok &= on_line(g, iw, make_double2(w.x, w.y));
+    if (tab) on = ray_lo_fill(g, L, s_lay, s_lo);
+    if (valid) on &= on_line(g, iw, make_double2(w.x, w.y));
+    on = __syncthreads_and(on) != 0;
   }
-  ok = __syncthreads_and(ok) != 0;
-  if (ok) ok = ray_hm_fill(omega, n_w, tile * kDerThreads + 32 * warp, L, s_lay, hm);
+  const bool ok = tab && on && ray_hm_fill(omega, n_w, tile * kDerThreads + 32 * warp, L, s_lay, hm);
   __syncthreads();  // the layer terms are read before the staging rows overwrite them
   const size_t e = (size_t)ip * n_w + (valid ? iw : 0);
   RaySumSink sink;
@@ -321,8 +324,8 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
   } else {
     // direct exponentials read the layer terms of the preparation
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    adjoint_rays(L, w, free_surface != 0, seg, s_if, PhaseDirect{w, lay_all + (size_t)ip * L},
-                 sink);
+    adjoint_rays(L, w, free_surface != 0, seg, s_if,
+                 phase_line(on && !tab, omega, n_w, iw, w, lay_all + (size_t)ip * L), sink);
   }
   double c2 = valid ? (sink.res.x * sink.res.x + sink.res.y * sink.res.y) : 0.0;
   for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);

@@ -101,15 +101,17 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
     const double2 wv = omega[iw];
     w = mk(wv.x, wv.y);
   }
-  bool use_tab = table != 0;
+  const bool tab = table != 0;
+  bool on = ray_line_model(L);  // the tile on the line (and, with a table, its lo entries usable)
   cd* hm = s_lo + ray_lo_values(L) + warp * ray_hm_values(L);
-  if (use_tab) {
+  if (on) {
     const GridLine g = grid_line(omega, n_w);
-    use_tab = ray_lo_fill(g, L, sl, s_lo);
-    if (valid) use_tab &= on_line(g, iw, make_double2(w.x, w.y));
-    use_tab = __syncthreads_and(use_tab) != 0;
-    if (use_tab) use_tab = ray_hm_fill(omega, n_w, tile * kHessThreads + 32 * warp, L, sl, hm);
+    if (tab) on = ray_lo_fill(g, L, sl, s_lo);
+    if (valid) on &= on_line(g, iw, make_double2(w.x, w.y));
+    on = __syncthreads_and(on) != 0;
   }
+  const bool use_tab =
+      tab && on && ray_hm_fill(omega, n_w, tile * kHessThreads + 32 * warp, L, sl, hm);
   const size_t k = valid ? iw : 0;
   HessRaySink sink;
   sink.valid = valid;
@@ -126,7 +128,8 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
   if (use_tab)
     adjoint_rays(L, w, free_surface != 0, seg, sc, ray_table(s_lo, hm), sink);
   else
-    adjoint_rays(L, w, free_surface != 0, seg, sc, PhaseDirect{w, sl}, sink);
+    adjoint_rays(L, w, free_surface != 0, seg, sc, phase_line(on && !tab, omega, n_w, iw, w, sl),
+                 sink);
   __syncthreads();
   for (int e = threadIdx.x; e < nrow; e += kHessThreads) {
     double s = acc[e];
