@@ -170,6 +170,8 @@ size_t kr_misfit_hessian_workspace_bytes(int32_t n_layers, int32_t n_p, int32_t 
  * (p, w); block partials reduced in a fixed order (deterministic).
  *   R_obs : device complex [n_p][n_w];  H : device float64 [4N][4N] output
  *   workspace : >= kr_misfit_hessian_workspace_bytes(n_layers, n_p, n_w) bytes
+ * Frequencies with a negative real or imaginary part, whose phases grow with depth, are not taken:
+ * H is NaN (kr_misfit_hvp gives the Hessian).
  */
 kr_status kr_misfit_hessian(const double* layers, int32_t n_layers, const double* p, int32_t n_p,
                             const double* omega, int32_t n_w, uint32_t flags,

@@ -133,7 +133,7 @@ KR_HD void interface_tangents(double p, int iface, const LayerP& up, const Layer
 //     g^T dRd g + 2 x^T dTd g + x^T dRu x + 2 sum_a z_a x_a dlog(e_a) + g'^T dr g',
 // so g' is the next step's vector, every coefficient adjoint is a product of two components
 // of (g, x), and the phases' are 2 z_a x_a (times omega: the phases are exp(omega c)).  X is
-// all the step must keep from the forward sweep: 64 FP64 operations per step for (g, x, z, g')
+// all the step must keep from the forward sweep (ray_step_grown: the state r): 64 FP64 operations per step for (g, x, z, g')
 // where differentiating the step's arithmetic entry by entry took ~300.
 struct Ray {
   cd a, b;
@@ -146,6 +146,26 @@ KR_HD void ray_step(const S3& X, const F& f, const Ray& g, Ray& x, Ray& z) {
   x.b = cdot2(X.b, y1, X.d, y2);
   z.a = cmac(cmac(y1, f.ru11, x.a), f.ru12, x.b);
   z.b = cmac(cmac(y2, f.ru12, x.a), f.ru22, x.b);
+}
+
+// The same from the state r below the step, for phases that grow downwards (phases_grow).  With a
+// large M = E r E the sum y + Ru x = N^-1 y nearly cancels (X tends to -Ru^-1) and g' = E z enlarges
+// what is left: at |E|^2 ~ 1e8 it has no correct digit.  Here N^-1 = adj(N) / det N is formed
+// itself.  Keeping r instead of X costs the step's reciprocal again in the reverse sweep, so
+// decaying phases (every frequency of the first quadrant) keep X.
+KR_HD void ray_step_grown(const S3& r, cd ea, cd eb, const Iface& f, const Ray& g, Ray& x, Ray& z) {
+  const cd m11 = (ea * ea) * r.a, m12 = (ea * eb) * r.b, m22 = (eb * eb) * r.d;
+  S3 X;
+  const cd idet = step_x(m11, m12, m22, f, X.a, X.b, X.d);
+  const cd y1 = cdot2(f.td11, g.a, f.td12, g.b), y2 = cdot2(f.td21, g.a, f.td22, g.b);
+  x.a = cdot2(X.a, y1, X.b, y2);
+  x.b = cdot2(X.b, y1, X.d, y2);
+  const cd one = mk(1.0, 0.0);
+  const cd n11 = cmac(cmac(one, -f.ru11, m11), -f.ru12, m12);
+  const cd n22 = cmac(cmac(one, -f.ru12, m12), -f.ru22, m22);
+  const cd m_n12 = cdot2(f.ru11, m12, f.ru12, m22), m_n21 = cdot2(f.ru12, m11, f.ru22, m12);
+  z.a = cdot2(n22, y1, m_n12, y2) * idet;
+  z.b = cdot2(n11, y2, m_n21, y1) * idet;
 }
 
 // The 10 coefficient adjoints of a step (order of ScatTan) from its (g, x).
@@ -257,6 +277,7 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
   // tabulated phase factors are recomputed in the reverse sweep (two products each) instead of
   // kept on the tape, as in adjoint_pair_sums
   const bool keep_ph = !ph.cheap();
+  const bool grown = ph.grows();  // the tape holds the state below each step instead of its X
   M2 r = m2(coef[I - 1].rd11, coef[I - 1].rd12, coef[I - 1].rd12, coef[I - 1].rd22);
   for (int q = 0; q < ncp; ++q) {
     cp[q] = s3(r);
@@ -266,9 +287,10 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
       const int i = I - 2 - s;
       const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
       S3 x;
+      const S3 below = s3(r);
       r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
       if (top) {
-        sg[s - s0] = x;
+        sg[s - s0] = grown ? below : x;
         if (keep_ph) {
           sea[s - s0] = ea;
           seb[s - s0] = eb;
@@ -307,8 +329,9 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
         const int i = I - 2 - s;
         const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
         S3 X;
+        const S3 below = s3(x);
         x = kennett_step_x(x, ea * ea, eb * eb, ea * eb, coef[i], X.a, X.b, X.d);
-        sg[s - s0] = X;
+        sg[s - s0] = grown ? below : X;
         if (keep_ph) {
           sea[s - s0] = ea;
           seb[s - s0] = eb;
@@ -320,7 +343,10 @@ KR_HD void jacobian_pair(int L, cd w, bool free_surface, int seg, const LayerP* 
       const cd ea = keep_ph ? sea[s - s0] : ph.a(i + 1);
       const cd eb = keep_ph ? seb[s - s0] : ph.b(i + 1);
       Ray x, z;
-      ray_step(sg[s - s0], coef[i], g, x, z);
+      if (grown)
+        ray_step_grown(sg[s - s0], ea, eb, coef[i], g, x, z);
+      else
+        ray_step(sg[s - s0], coef[i], g, x, z);
       cd cbar[10];
       ray_adjoints(g, x, cbar);
       contract<10>(tan[i], cbar, cur, nxt);
@@ -371,7 +397,7 @@ KR_HD size_t sum_rows(int L) { return (size_t)L; }
 // sink gets once top(f0) (the ocean phase term of layer 0) and per step
 // ray(i, g, x, wz, X, ea, eb): g and x of ray_step at interface i and omega z, whose products
 // are the 12 adjoints (the 10 of ray_adjoints; fa = 2 wz_a x_a, fb = 2 wz_b x_b), and the step's
-// X and phases; the bottom interface comes with everything but g zero.
+// X (of decaying phases) and phase factors; the bottom interface comes with everything but g zero.
 #ifdef __CUDACC__
 #pragma nv_exec_check_disable
 #endif
@@ -387,6 +413,7 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
   // tabulated phase factors are recomputed in the reverse sweep (two products each) instead of
   // kept on the tape: 48 instead of 80 bytes of local memory per step
   const bool keep_ph = !ph.cheap();
+  const bool grown = ph.grows();  // the tape holds the state below each step instead of its X
   M2 r = m2(coef[I - 1].rd11, coef[I - 1].rd12, coef[I - 1].rd12, coef[I - 1].rd22);
   for (int q = 0; q < ncp; ++q) {
     cp[q] = s3(r);
@@ -396,9 +423,10 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
       const int i = I - 2 - s;
       const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
       S3 x;
+      const S3 below = s3(r);
       r = kennett_step_x(r, ea * ea, eb * eb, ea * eb, coef[i], x.a, x.b, x.d);
       if (top) {
-        sg[s - s0] = x;
+        sg[s - s0] = grown ? below : x;
         if (keep_ph) {
           sea[s - s0] = ea;
           seb[s - s0] = eb;
@@ -426,8 +454,9 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
         const int i = I - 2 - s;
         const cd ea = ph.a(i + 1), eb = ph.b(i + 1);
         S3 X;
+        const S3 below = s3(x);
         x = kennett_step_x(x, ea * ea, eb * eb, ea * eb, coef[i], X.a, X.b, X.d);
-        sg[s - s0] = X;
+        sg[s - s0] = grown ? below : X;
         if (keep_ph) {
           sea[s - s0] = ea;
           seb[s - s0] = eb;
@@ -439,7 +468,10 @@ KR_HD void adjoint_rays(int L, cd w, bool free_surface, int seg, const Iface* co
       const cd ea = keep_ph ? sea[s - s0] : ph.a(i + 1);
       const cd eb = keep_ph ? seb[s - s0] : ph.b(i + 1);
       Ray x, z;
-      ray_step(sg[s - s0], coef[i], g, x, z);
+      if (grown)
+        ray_step_grown(sg[s - s0], ea, eb, coef[i], g, x, z);
+      else
+        ray_step(sg[s - s0], coef[i], g, x, z);
       const Ray wz = {w * z.a, w * z.b};
       sink.ray(i, g, x, wz, sg[s - s0], ea, eb);
       g.a = ea * z.a;

@@ -40,6 +40,7 @@ struct RayTable {
     return hm[4 * l + 2] * lo[2 * kPhLo * l + kPhLo];
   }
   __device__ __forceinline__ bool cheap() const { return true; }
+  __device__ __forceinline__ bool grows() const { return false; }  // such warps do without a table
 };
 
 __host__ __device__ inline size_t ray_lo_values(int n_layers) {
@@ -124,10 +125,30 @@ struct PhaseLine {
   __device__ __forceinline__ cd a(int l) const { return at(lay[l].ca); }
   __device__ __forceinline__ cd b(int l) const { return at(lay[l].cb); }
   __device__ __forceinline__ bool cheap() const { return false; }
+  __device__ __forceinline__ bool grows() const { return false; }
+};
+// The same for a warp with growing phases: in the frequency sums a sweep of its own (as a flag of the
+// other's, the second way of the step cost deep models 5 to 8 %), in the per-step contraction, with
+// few registers to spare, a flag (a third sweep spills: 64 x 1024 Jacobian of 21 layers 108.5 us
+// against 106.6).
+struct PhaseGrown : PhaseLine {
+  __device__ __forceinline__ explicit PhaseGrown(const PhaseLine& p) : PhaseLine(p) {}
+  __device__ __forceinline__ bool grows() const { return true; }
+};
+struct PhaseEither : PhaseLine {
+  bool grow;
+  __device__ __forceinline__ PhaseEither(const PhaseLine& p, bool g) : PhaseLine(p), grow(g) {}
+  __device__ __forceinline__ bool grows() const { return grow; }
 };
 __device__ __forceinline__ bool ray_line_model(int n_layers) { return n_layers <= kPairLayers; }
 
-// The source of frequency k = w; `on`: its tile is on the line and the model is a ray_line_model.
+// Whether a frequency of the warp has growing phases.  All 32 lanes call it.
+__device__ __forceinline__ bool warp_grows(bool valid, cd w) {
+  return __any_sync(0xffffffffu, valid && phases_grow(w));
+}
+
+// The source of frequency k = w; `on`: its tile is on the line and the forward sweep's phases of it
+// come from a table.
 __device__ __forceinline__ PhaseLine phase_line(bool on, const double2* __restrict__ omega, int n_w,
                                                 int k, cd w, const LayerP* lay) {
   if (!on) return PhaseLine{w, mk(0.0, 0.0), lay};

@@ -409,12 +409,15 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
       sink.obs = obs_all + d.obs_off + e;
       sink.R_out = (d.flags & KR_BATCH_STORE_R) ? R_all + d.R_off + e : nullptr;
       const bool on = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0;
-      const bool tab = on && ray_table_model(L) && ray_hm_fill(om, d.n_w, kb, L, v.lay, hm);
+      const bool grow = warp_grows(valid, w);
+      const bool tab =
+          on && !grow && ray_table_model(L) && ray_hm_fill(om, d.n_w, kb, L, v.lay, hm);
       if (tab)
         jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan, ray_table(lo, hm), sink);
       else
         jacobian_pair(L, w, fs, seg, v.lay, v.dlay, v.coef, v.tan,
-                      phase_line(on && !ray_table_model(L), om, d.n_w, iw, w, v.lay), sink);
+                      PhaseEither(phase_line(on && (grow || !ray_table_model(L)), om, d.n_w, iw, w,
+                                             v.lay), grow), sink);
       __syncwarp();
       double c2 = valid ? (sink.res.x * sink.res.x + sink.res.y * sink.res.y) : 0.0;
       for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);
@@ -494,12 +497,16 @@ batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_al
       sink.stage = stage + warp * kRayStage;
       sink.I = I;
       const bool on = lo_ok && s_tiles.off[kb / kPhTile - item.w0 / kPhTile] == 0;
-      const bool tab = on && ray_table_model(L) && ray_hm_fill(om, d.n_w, kb, L, sl, hm);
+      const bool grow = warp_grows(valid, w);
+      const bool tab =
+          on && !grow && ray_table_model(L) && ray_hm_fill(om, d.n_w, kb, L, sl, hm);
       if (tab)
         adjoint_rays(L, w, fs, seg, sc, ray_table(lo, hm), sink);
-      else
+      else if (!grow)
         adjoint_rays(L, w, fs, seg, sc,
                      phase_line(on && !ray_table_model(L), om, d.n_w, iw, w, sl), sink);
+      else
+        adjoint_rays(L, w, fs, seg, sc, PhaseGrown(phase_line(on, om, d.n_w, iw, w, sl)), sink);
       __syncwarp();  // the hm entries are read before the next pass overwrites them
       if (valid) c2 += sink.res.x * sink.res.x + sink.res.y * sink.res.y;
     }

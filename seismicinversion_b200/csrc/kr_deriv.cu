@@ -198,8 +198,9 @@ deriv_sweep_kernel(int L, const double* __restrict__ p, int n_p,
     if (valid) on &= on_line(g, iw, make_double2(w.x, w.y));
     on = __syncthreads_and(on) != 0;
   }
-  const bool use_tab = tab && on && ray_hm_fill(omega, n_w, tile * kDerThreads + (threadIdx.x & ~31),
-                                                L, lay, hm);
+  const bool grow = warp_grows(valid, w);
+  const bool use_tab = tab && on && !grow &&
+                       ray_hm_fill(omega, n_w, tile * kDerThreads + (threadIdx.x & ~31), L, lay, hm);
   PairSink<MODE> sink;
   sink.L = L;
   sink.ip = ip;
@@ -214,7 +215,7 @@ deriv_sweep_kernel(int L, const double* __restrict__ p, int n_p,
     jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan, ray_table(s_lo, hm), sink);
   else
     jacobian_pair(L, w, free_surface != 0, seg, lay, dlay, coef, tan,
-                  phase_line(on && !tab, omega, n_w, iw, w, lay), sink);
+                  PhaseEither(phase_line(on && (!tab || grow), omega, n_w, iw, w, lay), grow), sink);
   if (GRAD) {
     const cd res = sink.res;
     double c2 = valid ? (res.x * res.x + res.y * res.y) : 0.0;
@@ -308,7 +309,9 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
     if (valid) on &= on_line(g, iw, make_double2(w.x, w.y));
     on = __syncthreads_and(on) != 0;
   }
-  const bool ok = tab && on && ray_hm_fill(omega, n_w, tile * kDerThreads + 32 * warp, L, s_lay, hm);
+  const bool grow = warp_grows(valid, w);
+  const bool ok = tab && on && !grow &&
+                  ray_hm_fill(omega, n_w, tile * kDerThreads + 32 * warp, L, s_lay, hm);
   __syncthreads();  // the layer terms are read before the staging rows overwrite them
   const size_t e = (size_t)ip * n_w + (valid ? iw : 0);
   RaySumSink sink;
@@ -324,8 +327,13 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
   } else {
     // direct exponentials read the layer terms of the preparation
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    adjoint_rays(L, w, free_surface != 0, seg, s_if,
-                 phase_line(on && !tab, omega, n_w, iw, w, lay_all + (size_t)ip * L), sink);
+    const LayerP* lay = lay_all + (size_t)ip * L;
+    if (!grow)
+      adjoint_rays(L, w, free_surface != 0, seg, s_if, phase_line(on && !tab, omega, n_w, iw, w, lay),
+                   sink);
+    else
+      adjoint_rays(L, w, free_surface != 0, seg, s_if,
+                   PhaseGrown(phase_line(on, omega, n_w, iw, w, lay)), sink);
   }
   double c2 = valid ? (sink.res.x * sink.res.x + sink.res.y * sink.res.y) : 0.0;
   for (int o = 16; o > 0; o >>= 1) c2 += __shfl_down_sync(0xffffffffu, c2, o);

@@ -33,7 +33,7 @@ constexpr size_t kStepBytes = (size_t)256 << 20;
 // Rays
 // ---------------------------------------------------------------------------------------
 struct HessRaySink {
-  bool valid, fs;
+  bool valid, fs, grow;
   const double2* obs;
   double2* out;   // step values of this (p, omega), value c of step i at out[(i kStepVals + c) n_w]
   double2* seeds; // seed and zeta of this (p, omega)
@@ -47,7 +47,8 @@ struct HessRaySink {
     sigma = mk(0.0, 0.0);
     if (valid) {
       const double2 o = *obs;
-      const cd seed = mk(2.0 * (R.x - o.x), -2.0 * (R.y - o.y));
+      cd seed = mk(2.0 * (R.x - o.x), -2.0 * (R.y - o.y));
+      if (grow) seed = mk(nan(""), nan(""));  // these formulas lose growing phases: no value
       // 1 + Y = 1 / (1 - R) with the free surface
       const cd zeta = fs ? (-2.0 * seed) * recip(1.0 - R) : mk(0.0, 0.0);
       seeds[0] = make_double2(seed.x, seed.y);
@@ -116,6 +117,7 @@ hess_rays_kernel(int L, const double2* __restrict__ omega, int n_w, int n_wtiles
   HessRaySink sink;
   sink.valid = valid;
   sink.fs = free_surface != 0;
+  sink.grow = phases_grow(w);
   sink.obs = obs + (size_t)ip * n_w + k;
   sink.out = steps + (size_t)jp * I * kStepVals * n_w + k;
   sink.seeds = seeds + 2 * ((size_t)jp * n_w + k);

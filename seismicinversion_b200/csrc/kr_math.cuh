@@ -164,6 +164,10 @@ struct LayerP {
   double pad;  // 96 bytes: arrays of LayerP are whole 16-byte units (vector copies)
 };
 
+// Whether |exp(omega i eta h)| may exceed 1: eta and neta lie in the first quadrant and h >= 0, so
+// only for frequencies with a negative real or imaginary part.
+KR_HD bool phases_grow(cd w) { return w.x < 0.0 || w.y < 0.0; }
+
 // Phase factors exp(omega * i eta h) and exp(omega * i neta h) of layer l, evaluated directly
 // (kernels on uniform frequency grids use a tabulated source with the same a(l) / b(l)).
 struct PhaseDirect {
@@ -173,6 +177,8 @@ struct PhaseDirect {
   KR_HD cd b(int l) const { return cexp_(w * lay[l].cb); }
   // whether a factor is cheaper to recompute than to keep (a tabulated source: two products)
   KR_HD bool cheap() const { return false; }
+  // whether a phase may grow downwards (phases_grow)
+  KR_HD bool grows() const { return phases_grow(w); }
 };
 
 // Layer table layout (device or host): 6 rows of n_layers doubles:
@@ -381,10 +387,8 @@ struct M2 {
   cd a, b, c, d;
 };
 
-// X = MT (I - Ru MT)^-1 of the step (entries 11, 12, 22) from the squared and mixed phase
-// factors P = ea^2, Q = eb^2, S = ea eb.
-KR_HD void step_x(const M2& r, cd P, cd Q, cd S, const Iface& f, cd& x11, cd& x12, cd& x22) {
-  const cd m11 = P * r.a, m12 = S * r.b, m22 = Q * r.d;
+// X = MT (I - Ru MT)^-1 of the step (entries 11, 12, 22) from MT's entries; returns 1 / det N.
+KR_HD cd step_x(cd m11, cd m12, cd m22, const Iface& f, cd& x11, cd& x12, cd& x22) {
   const cd dm = cdot2(m11, m22, -m12, m12);
   const cd one = mk(1.0, 0.0);
   const cd idet = recip_near(
@@ -392,6 +396,11 @@ KR_HD void step_x(const M2& r, cd P, cd Q, cd S, const Iface& f, cd& x11, cd& x1
   x11 = cmac(m11, -f.ru22, dm) * idet;
   x12 = cmac(m12, f.ru12, dm) * idet;
   x22 = cmac(m22, -f.ru11, dm) * idet;
+  return idet;
+}
+// The same from the squared and mixed phase factors P = ea^2, Q = eb^2, S = ea eb.
+KR_HD void step_x(const M2& r, cd P, cd Q, cd S, const Iface& f, cd& x11, cd& x12, cd& x22) {
+  step_x(P * r.a, S * r.b, Q * r.d, f, x11, x12, x22);
 }
 
 // The step, which also hands out X: the reverse sweep of the derivatives needs nothing else of

@@ -25,6 +25,7 @@ __all__ = [
     "vjp",
     "misfit_hvp",
     "misfit_hessian",
+    "misfit_hessian_by_axes",
     "jacobian_dot",
     "table_from_tensors",
     "stream_handle",
@@ -294,8 +295,9 @@ def misfit_hvp(layers: torch.Tensor, p, omega, R_obs, V, free_surface: bool = Fa
 def misfit_hessian(layers: torch.Tensor, p, omega, R_obs, free_surface: bool = False):
     """Exact Hessian of chi = sum |R - R_obs|^2 over the packed sub-ocean parameters
     [4N - 1, 4N - 1] (alpha, beta, rho of layers 1..N, h of layers 1..N-1), float64 on the
-    device: ``kr_misfit_hessian``, or ``kr_misfit_hvp`` along every axis for models too deep for
-    it."""
+    device: ``kr_misfit_hessian``, or ``misfit_hessian_by_axes`` for models too deep for it.
+    NaN where a frequency's real or imaginary part is negative (phases grow with depth, which
+    ``kr_misfit_hessian`` does not take): ``misfit_hessian_by_axes`` has a value there."""
     dev = layers.device
     L = layers.shape[1]
     n = 4 * (L - 1)
@@ -306,11 +308,7 @@ def misfit_hessian(layers: torch.Tensor, p, omega, R_obs, free_surface: bool = F
     h = _lib.lib()
     ws_bytes = h.kr_misfit_hessian_workspace_bytes(L, n_p, n_w)
     if ws_bytes == 0 and n_p > 0 and n_w > 0:
-        idx = torch.as_tensor([k * L + l for k in range(4) for l in range(1, L)][:n - 1], device=dev)
-        V = torch.zeros((n - 1, 4 * L), dtype=torch.float64, device=dev)
-        V[torch.arange(n - 1, device=dev), idx] = 1.0
-        H = misfit_hvp(layers, p_t, w_t, Ro, V, free_surface)[:, idx]
-        return 0.5 * (H + H.T)
+        return misfit_hessian_by_axes(layers, p_t, w_t, Ro, free_surface)
     ws = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dev)
     H = torch.empty((n, n), dtype=torch.float64, device=dev)
     flags = _lib.KR_FREE_SURFACE if free_surface else 0
@@ -319,6 +317,19 @@ def misfit_hessian(layers: torch.Tensor, p, omega, R_obs, free_surface: bool = F
                              stream_handle(dev))
     _lib.check(st, "kr_misfit_hessian")
     return H[:n - 1, :n - 1]
+
+
+def misfit_hessian_by_axes(layers: torch.Tensor, p, omega, R_obs, free_surface: bool = False):
+    """``misfit_hessian`` as ``kr_misfit_hvp`` along every axis, symmetrised: any depth and any
+    frequencies, at the cost of one dual adjoint sweep per parameter."""
+    dev = layers.device
+    L = layers.shape[1]
+    n = 4 * (L - 1)
+    idx = torch.as_tensor([k * L + l for k in range(4) for l in range(1, L)][:n - 1], device=dev)
+    V = torch.zeros((n - 1, 4 * L), dtype=torch.float64, device=dev)
+    V[torch.arange(n - 1, device=dev), idx] = 1.0
+    H = misfit_hvp(layers, p, omega, R_obs, V, free_surface)[:, idx]
+    return 0.5 * (H + H.T)
 
 
 def jacobian_dot(layers: torch.Tensor, p, omega, V, free_surface: bool = False):

@@ -113,9 +113,11 @@ class _Problem:
         return V
 
     def hessian_exact(self, phys: np.ndarray) -> np.ndarray:
-        """The exact Hessian over the packed parameters (kr_misfit_hessian)."""
-        return D.misfit_hessian(self.table(phys), self.p, self.omega, self.R_obs,
-                                self.fs).cpu().numpy()
+        """The exact Hessian over the packed parameters (kr_misfit_hessian; by directions where
+        that has no value, as for frequencies with a negative real or imaginary part)."""
+        args = (self.table(phys), self.p, self.omega, self.R_obs, self.fs)
+        H = D.misfit_hessian(*args).cpu().numpy()
+        return H if np.isfinite(H).all() else D.misfit_hessian_by_axes(*args).cpu().numpy()
 
     def hessian_fd(self, phys: np.ndarray, step: float = 1e-5, stencil: int = 2) -> np.ndarray:
         """Central differences of the exact adjoint gradient, all perturbed models in one
