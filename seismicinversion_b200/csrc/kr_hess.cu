@@ -493,13 +493,14 @@ extern "C" kr_status kr_misfit_hessian(const double* layers, int32_t n_layers, c
   const int L = n_layers, I = L - 1;
   if (n_p < 0 || n_w < 0 || (flags & ~KR_FREE_SURFACE) || !H) return KR_ERR_INVALID_ARGUMENT;
   if (L < 2) return KR_ERR_INVALID_MODEL;
-  if (L > kMaxLayers || !hess_fits(L)) return KR_ERR_TOO_LARGE;
+  if (L > kMaxLayers) return KR_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
-  if (n_p == 0 || n_w == 0) {
+  if (n_p == 0 || n_w == 0) {  // whatever the depth: the sum over nothing
     const cudaError_t e = cudaMemsetAsync(H, 0, sizeof(double) * 16 * (size_t)I * I, st);
     if (e != cudaSuccess) set_last_error("kr_misfit_hessian: memset", e);
     return cuda_status(e);
   }
+  if (!hess_fits(L)) return KR_ERR_TOO_LARGE;
   if (!layers || !p || !omega || !R_obs) return KR_ERR_INVALID_ARGUMENT;
   if (!aligned16(omega) || !aligned16(R_obs)) return KR_ERR_INVALID_ARGUMENT;
   const HessWs w = hess_ws(workspace, L, n_p, n_w);
