@@ -50,7 +50,10 @@ static __device__ __noinline__ void gmm_store(double p, int k, const LayerP* lay
   const cd d = 2.0 * (mul - u.rho * (u.betac * u.betac));
   const cd pd = (p * p) * d;
   const cd a = (l.rho - u.rho) - pd, b = l.rho - pd, c = u.rho + pd;
-  const cd ie = recip(u.eta), in = recip(u.neta);
+  // A fluid layer at p = 0 has neta = 0: its S amplitudes decouple from P there (every mixed entry has
+  // a factor p) and are left without their coupling to the layer below instead of dividing by zero.
+  const cd ie = recip(u.eta);
+  const cd in = (u.neta.x == 0.0 && u.neta.y == 0.0) ? mk(0.0, 0.0) : recip(u.neta);
   const cd cp = (c * l.eta) * ie, cs = (c * l.neta) * in;   // c eta2 / eta1, c neta2 / neta1
   const cd ap = p * (a * ie), as = p * (a * in);            // p a / eta1, p a / neta1
   const cd dn = p * (d * l.neta), de = p * (d * l.eta);     // p d neta2, p d eta2
