@@ -343,12 +343,13 @@ __device__ __forceinline__ bool ray_item_tables(const ItemRec& item, const kr_mo
 }
 
 // Gradient items of models whose frequency sums exceed shared memory (more than ~118 layers in
-// the batch): the contraction per (omega, p), as deriv_sweep_kernel.
+// the batch; all of them with KR_DERIV_SUMS=0): the contraction per (omega, p), as
+// deriv_sweep_kernel.  `deep`: the class of the work list.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
 batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all,
                       const double2* __restrict__ obs_all, double2* __restrict__ R_all,
-                      double* __restrict__ chi_grad, int stage) {
+                      double* __restrict__ chi_grad, int stage, int deep) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // [THREADS / 32][4L + 1] accumulators (padded to 16 bytes), then (models that tabulate) the
   // phase table, then, if `stage`, the item's slowness data
@@ -357,10 +358,11 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
   PlanHeader* h = reinterpret_cast<PlanHeader*>(plan);
   const kr_model_desc* models = reinterpret_cast<const kr_model_desc*>(plan + h->off_models);
   const PairRec* pairs = reinterpret_cast<const PairRec*>(plan + h->off_pairs);
-  const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_grad);
-  const int n_items = h->n_grad_deep;
+  const ItemRec* items = reinterpret_cast<const ItemRec*>(plan + h->off_grad) +
+                         (deep ? 0 : h->n_grad_deep);
+  const int n_items = deep ? h->n_grad_deep : h->n_grad - h->n_grad_deep;
   __shared__ int s_item;
-  ItemFeed feed(&h->counters[2], &s_item);
+  ItemFeed feed(&h->counters[deep ? 2 : 3], &s_item);
   for (;;) {
     const int it = feed.next();
     if (it >= n_items) break;
@@ -784,6 +786,13 @@ static kr_status launch_batch_forward(unsigned char* pl, int max_layers, const d
   return KR_OK;
 }
 
+// batch_gradient_kernel's shared-memory limit, one for both classes that launch it.
+template <int THREADS>
+static SmemLimit& gradient_limit() {
+  static SmemLimit lim;
+  return lim;
+}
+
 // One class of the gradient items on a resident grid.  `after`: as the programmatic dependent of
 // the class launched before it.
 template <int THREADS, bool DEEP>
@@ -791,17 +800,17 @@ static kr_status launch_batch_gradient(unsigned char* pl, int max_layers, const 
                                        const double2* obs, double2* R, double* chi_grad, bool after,
                                        cudaStream_t st) {
   const int L = DEEP ? max_layers : std::min(max_layers, kPqsLayers);
-  const size_t sums = (DEEP && !batch_sums_enabled()) ? 0 : sums_smem(THREADS, L);
-  static SmemLimit slim, glim;
+  const size_t sums = batch_sums_enabled() ? sums_smem(THREADS, L) : 0;
+  static SmemLimit slim;
   if (!sums) {
     int stage = 0;
     const size_t smem = grad_smem(THREADS, L, &stage);
     const void* fn = (const void*)batch_gradient_kernel<THREADS>;
     if (smem > 46 * 1024 &&
-        raise_smem_limit(fn, smem, glim, "kr_batch_launch: gradient smem") != KR_OK)
+        raise_smem_limit(fn, smem, gradient_limit<THREADS>(), "kr_batch_launch: gradient smem") != KR_OK)
       return KR_ERR_CUDA;
     batch_gradient_kernel<THREADS><<<occupancy_grid(fn, THREADS, smem), THREADS, smem, st>>>(
-        pl, w, obs, R, chi_grad, stage);
+        pl, w, obs, R, chi_grad, stage, DEEP ? 1 : 0);
     return check_launch("kr_batch_launch: gradient");
   }
   const void* fn = (const void*)batch_grad_sums_kernel<THREADS, DEEP>;
