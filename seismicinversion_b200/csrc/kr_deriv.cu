@@ -253,21 +253,21 @@ reduce_partials_kernel(const double* __restrict__ partial, int n_blocks, int str
 }
 
 // GRAD / VJP with the contraction moved out of the frequency loop (kr_adjsum.cuh): block =
-// one slowness x 128 frequencies.  The block forms its own layer terms, coefficients and phase
-// table (the stages of the forward kernel's prologue), so nothing but the contraction waits for
-// deriv_prep_kernel, whose programmatic dependent it is.  Dynamic smem: per-warp sum rows and
-// staging rows (first the layer terms and roots, which only the prologue reads), the interface
-// coefficients, then (table models) the phase table: 52 KB for 21 layers, four blocks per SM, so
-// that the 512 blocks of a 64 x 1024 gradient are one wave.  Writes the block's [4L] contributions and chi to
-// partial[block][4L + 1].
+// one slowness x 128 frequencies.  With `own` (sum_kernel_own) the block forms its own layer terms
+// and coefficients (the stages of the forward kernel's prologue), so nothing but the contraction
+// waits for deriv_prep_kernel, whose programmatic dependent it is; otherwise it waits for them and
+// copies them.  Dynamic smem: per-warp sum rows and staging rows (first the layer terms and roots,
+// which only the prologue reads), the interface coefficients, then (table models) the phase table:
+// 52 KB for 21 layers, four blocks per SM, so that the 512 blocks of a 64 x 1024 gradient are one
+// wave.  Writes the block's [4L] contributions and chi to partial[block][4L + 1].
 template <int MINB>
 __global__ void __launch_bounds__(kDerThreads, MINB)
 deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restrict__ p,
                  const double2* __restrict__ omega, int n_w, int n_wtiles, int free_surface,
-                 int vjp, int seg, int table, const LayerP* __restrict__ lay_all,
-                 const LayerD* __restrict__ dlay_all, const ScatTan* __restrict__ tan_all,
-                 const double2* __restrict__ obs, double2* __restrict__ R_out,
-                 double* __restrict__ partial) {
+                 int vjp, int seg, int table, int own, const LayerP* __restrict__ lay_all,
+                 const LayerD* __restrict__ dlay_all, const Iface* __restrict__ coef_all,
+                 const ScatTan* __restrict__ tan_all, const double2* __restrict__ obs,
+                 double2* __restrict__ R_out, double* __restrict__ partial) {
   // the reduction after this kernel may launch as soon as every block of it has started
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int W = kDerThreads / 32;
@@ -288,18 +288,25 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
   cd* s_lo = reinterpret_cast<cd*>(s_if + I);
   const double pj = p[ip];
   sums_zero(acc, L, W);
-  for (int t = threadIdx.x; t < 2 * L; t += kDerThreads) {
-    const int half = t >= L ? 1 : 0, l = t - half * L;
-    layer_store(tab6, L, l, half, pj, s_lay + l, s_root + l);
-  }
   cd w = mk(0.0, 0.0);
   if (valid) {
     const double2 wv = omega[iw];
     w = mk(wv.x, wv.y);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < I; i += kDerThreads)
-    interface_store(pj, i, s_lay, s_root, s_if + i);
+  if (own) {
+    for (int t = threadIdx.x; t < 2 * L; t += kDerThreads) {
+      const int half = t >= L ? 1 : 0, l = t - half * L;
+      layer_store(tab6, L, l, half, pj, s_lay + l, s_root + l);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < I; i += kDerThreads)
+      interface_store(pj, i, s_lay, s_root, s_if + i);
+  } else {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    copy16(s_lay, lay_all + (size_t)ip * L, sizeof(LayerP) * L);
+    copy16(s_if, coef_all + (size_t)ip * I, sizeof(Iface) * I);
+    __syncthreads();
+  }
   const bool tab = table != 0;
   bool on = ray_line_model(L);  // the tile on the line (and, with a table, its lo entries usable)
   cd* hm = s_lo + ray_lo_values(L) + warp * ray_hm_values(L);
@@ -412,6 +419,23 @@ static size_t sum_kernel_smem(int L, int table) {
   return smem <= kStageSmemMax ? smem : 0;
 }
 
+// Blocks of deriv_sum_kernel that an SM holds (4 up to 23 layers, 3 up to 31, 2 up to 48 with the
+// table; 128 registers allow no more than 4).
+static int sum_kernel_blocks(size_t smem) {
+  const int n = (int)((227 * 1024) / (smem + 1024 + 64));
+  return n > 4 ? 4 : n;
+}
+
+// Whether the sweep forms its own terms and coefficients beside deriv_prep_kernel: where its blocks
+// leave a third of a wave for that kernel's.  Beyond, the own prologue only lengthens every block
+// (64 x 1024, 512 blocks: 5 layers 42 us against 36.5 with the prepared coefficients, 21 layers 78.7
+// against 74.7; 513 x 257 of 3 layers 74.8 against 64.7); below, it saves the wait (48 x 1024: 29.4
+// against 37.9 for 5 layers; 32 x 1024: 62.5 against 72.7 for 21).  Models without a table wait
+// anyway, for the layer terms of their exponentials.
+static bool sum_kernel_own(size_t n_blocks, size_t smem, int table) {
+  return table && 3 * n_blocks <= 2 * 148 * (size_t)sum_kernel_blocks(smem);
+}
+
 // KR_DERIV_SUMS=0 keeps the per-step contraction for GRAD / VJP (comparison runs).
 static bool deriv_sums_enabled() {
   static int v = -1;
@@ -425,9 +449,8 @@ static bool deriv_sums_enabled() {
 template <int MINB>
 static kr_status launch_sum_v(unsigned blocks, size_t smem, cudaStream_t st, const double* layers,
                               int L, const double* p, const double2* omega, int n_w, int n_wtiles,
-                              int fs, int vjp, int seg, int table, const LayerP* lay,
-                              const LayerD* dlay, const ScatTan* tan, const double2* obs,
-                              double2* R, double* partial) {
+                              int fs, int vjp, int seg, int table, int own, const DerivWs& w,
+                              const double2* obs, double2* R) {
   static SmemLimit lim;
   if (smem > 47 * 1024) {  // with the static arrays above the 48 KB default
     const kr_status a = raise_smem_limit((const void*)deriv_sum_kernel<MINB>, smem, lim,
@@ -446,9 +469,10 @@ static kr_status launch_sum_v(unsigned blocks, size_t smem, cudaStream_t st, con
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, deriv_sum_kernel<MINB>, layers, L, p, omega, n_w,
-                                           n_wtiles, fs, vjp, seg, table, lay, dlay, tan, obs, R,
-                                           partial);
+  const cudaError_t e = cudaLaunchKernelEx(
+      &cfg, deriv_sum_kernel<MINB>, layers, L, p, omega, n_w, n_wtiles, fs, vjp, seg,
+      table, own, (const LayerP*)w.lay, (const LayerD*)w.dlay, (const Iface*)w.coef,
+      (const ScatTan*)w.tan, obs, R, w.partial);
   if (e != cudaSuccess) {
     set_last_error("kr_deriv: sweep launch", e);
     return KR_ERR_CUDA;
@@ -480,11 +504,10 @@ static kr_status launch_deriv(const double* layers, int L, const double* p, int 
     const double2* o = reinterpret_cast<const double2*>(R_obs);
     const double2* w2 = reinterpret_cast<const double2*>(omega);
     double2* R2 = reinterpret_cast<double2*>(R);
-    s = sum_minb() == 3
-            ? launch_sum_v<3>((unsigned)n_blocks, sum_smem, st, layers, L, p, w2, n_w, n_wtiles,
-                              fs, vjp, seg, sum_table, w.lay, w.dlay, w.tan, o, R2, w.partial)
-            : launch_sum_v<4>((unsigned)n_blocks, sum_smem, st, layers, L, p, w2, n_w, n_wtiles,
-                              fs, vjp, seg, sum_table, w.lay, w.dlay, w.tan, o, R2, w.partial);
+    const int own = sum_kernel_own(n_blocks, sum_smem, sum_table) ? 1 : 0;
+    auto* launch = sum_minb() == 3 ? launch_sum_v<3> : launch_sum_v<4>;
+    s = launch((unsigned)n_blocks, sum_smem, st, layers, L, p, w2, n_w, n_wtiles, fs, vjp, seg,
+               sum_table, own, w, o, R2);
     if (s != KR_OK) return s;
     s = check_launch("kr_deriv: sweep");
     if (s != KR_OK) return s;
