@@ -31,6 +31,9 @@
 
 namespace kr {
 
+// deriv_sum_kernel keeps the layer terms of an off-line block in the table's room
+static_assert(sizeof(LayerP) * 2 <= sizeof(cd) * 2 * kPhLo, "layer terms fit the lo entries");
+
 constexpr int kDerThreads = 128;
 static_assert((kMaxLayers - 2 + kSegMax - 1) / kSegMax <= kCpMax,
               "checkpoints must cover the deepest model");
@@ -319,6 +322,10 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
   const bool grow = warp_grows(valid, w);
   const bool ok = tab && on && !grow &&
                   ray_hm_fill(omega, n_w, tile * kDerThreads + 32 * warp, L, s_lay, hm);
+  // a block off the line needs no table: its layer terms go there, and the sweep need not wait for
+  // the prepared ones
+  const bool keep_lay = tab && !on;
+  if (keep_lay) copy16(s_lo, s_lay, sizeof(LayerP) * L);
   __syncthreads();  // the layer terms are read before the staging rows overwrite them
   const size_t e = (size_t)ip * n_w + (valid ? iw : 0);
   RaySumSink sink;
@@ -332,9 +339,11 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
   if (ok) {
     adjoint_rays(L, w, free_surface != 0, seg, s_if, ray_table(s_lo, hm), sink);
   } else {
-    // direct exponentials read the layer terms of the preparation
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const LayerP* lay = lay_all + (size_t)ip * L;
+    const LayerP* lay = reinterpret_cast<const LayerP*>(s_lo);
+    if (!keep_lay) {  // the layer terms of the preparation
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      lay = lay_all + (size_t)ip * L;
+    }
     if (!grow)
       adjoint_rays(L, w, free_surface != 0, seg, s_if, phase_line(on && !tab, omega, n_w, iw, w, lay),
                    sink);
