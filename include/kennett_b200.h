@@ -91,7 +91,8 @@ kr_status kr_reflectivity(const double* layers, int32_t n_layers, const double* 
  * (GlobalMatrix/global_matrix.py:297-348) and the forward of gmm_reflectivity_torch
  * (GlobalMatrix/gmm_torch.py:229-305, riccati_solver.py:200-330).  Arguments and errors as
  * kr_reflectivity; with KR_FREE_SURFACE the result is R / (1 + R).  One thread per
- * (omega, p); per interface a 4x4 complex solve with partial pivoting.
+ * (omega, p); the interfaces' 4x4 systems are solved once per slowness in closed form, which leaves
+ * one 2x2 quotient per (omega, p, interface).
  */
 kr_status kr_gmm_reflectivity(const double* layers, int32_t n_layers, const double* p,
                               int32_t n_p, const double* omega, int32_t n_w, uint32_t flags,
@@ -356,7 +357,8 @@ kr_status kr_batch_plan_host(const kr_model_desc* descs_host, int32_t n_models,
  * Runs a planned batch: reset -> per-(model, slowness) coefficient prep -> persistent
  * forward kernel -> persistent gradient kernel, all enqueued on `stream` with no host
  * synchronisation or allocation (capturable in a CUDA graph).  `cfg` must be the plan's
- * schedule and `max_layers` the largest n_layers of the batch.
+ * schedule and `max_layers` the largest n_layers of the batch.  R_obs may be NULL only for a batch
+ * without gradient models (none is launched).
  */
 kr_status kr_batch_launch(void* plan, const kr_batch_config* cfg, int32_t max_layers,
                           const double* layers, const double* p, const double* omega,
@@ -364,17 +366,17 @@ kr_status kr_batch_launch(void* plan, const kr_batch_config* cfg, int32_t max_la
 
 /*
  * Tuning knob (no counterpart in the reference): register budget of the kr_reflectivity
- * kernel as the number of 128-thread blocks each SM must fit (4 -> 128 registers per thread,
- * 5 -> 96, 6 -> 80; other values restore the automatic choice: 5 for models whose phases
- * come from the frequency-grid table, 4 otherwise).  Process-wide; results are identical for
- * every setting, only speed changes.
+ * kernel for models of up to 30 layers as the number of 128-thread blocks each SM must fit
+ * (4 -> 128 registers per thread, 5 -> 96, 6 -> 80; other values restore the automatic choice, 4).
+ * Process-wide; results are identical for every setting, only speed changes.
  */
 void kr_set_forward_variant(int32_t min_blocks_per_sm);
 
 /*
  * Tuning knob (no counterpart in the reference): register budget of the kr_jacobian /
  * kr_misfit_gradient / kr_vjp sweep kernels as 128-thread blocks per SM (2 -> up to 255
- * registers, 3 -> 168; other values select 2).  Process-wide; results do not depend on it.
+ * registers, 3 -> 168; the frequency sums of gradients take 168 either way; other values restore
+ * the automatic choice by depth).  Process-wide; results do not depend on it.
  */
 void kr_set_deriv_variant(int32_t min_blocks_per_sm);
 

@@ -370,10 +370,12 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
 // Shared memory the sweep may use for staging one slowness's data (per block).
 constexpr size_t kStageSmemMax = 160 * 1024;
 
-// Register budget of the sweep kernels: blocks of 128 threads per SM (2 -> up to 255
-// registers, 3 -> 168).  KR_DERIV_MINB or kr_set_deriv_variant; by default 3 for the per-step
-// sweeps (64 x 1024 x 21-layer Jacobian 106 us against 111 at 2) and 4 (128 registers) for the
-// frequency-sum sweep (gradient 75 us against 88 at 3, where 512 blocks are more than one wave).
+// Register budget of the sweep kernels as blocks of 128 threads per SM (2 -> up to 255 registers,
+// 3 -> 168, 4 -> 128), set by KR_DERIV_MINB or kr_set_deriv_variant or chosen by depth.
+// Per-step sweeps: 3 (64 x 1024 x 21-layer Jacobian 107 us against 112 at 2), but 2 beyond 108
+// layers, whose data is not staged (7 x 100 of 130 layers 479 us against 562 at 3).  Frequency
+// sums: 4 where shared memory holds four blocks (up to 23 layers: 64 x 1024 of 23 layers 84 us
+// against 100 at 3), else 3 (24 to 100 layers equal or up to 1 % faster than at 4).
 static int g_deriv_minb = -1;
 
 static int deriv_minb_setting() {
@@ -384,8 +386,11 @@ static int deriv_minb_setting() {
   }
   return g_deriv_minb;
 }
-static int deriv_minb() { return deriv_minb_setting() == 2 ? 2 : 3; }
-static int sum_minb() { return deriv_minb_setting() == 3 ? 3 : 4; }
+static int deriv_minb(bool staged) {
+  const int v = deriv_minb_setting();
+  return v ? v : staged ? 3 : 2;
+}
+static int sum_minb(int blocks) { return deriv_minb_setting() || blocks < 4 ? 3 : 4; }
 
 template <int MODE, int MINB>
 static kr_status launch_sweep_v(unsigned blocks, size_t smem, cudaStream_t st, int L,
@@ -514,7 +519,7 @@ static kr_status launch_deriv(const double* layers, int L, const double* p, int 
     const double2* w2 = reinterpret_cast<const double2*>(omega);
     double2* R2 = reinterpret_cast<double2*>(R);
     const int own = sum_kernel_own(n_blocks, sum_smem, sum_table) ? 1 : 0;
-    auto* launch = sum_minb() == 3 ? launch_sum_v<3> : launch_sum_v<4>;
+    auto* launch = sum_minb(sum_kernel_blocks(sum_smem)) == 3 ? launch_sum_v<3> : launch_sum_v<4>;
     s = launch((unsigned)n_blocks, sum_smem, st, layers, L, p, w2, n_w, n_wtiles, fs, vjp, seg,
                sum_table, own, w, o, R2);
     if (s != KR_OK) return s;
@@ -546,7 +551,7 @@ static kr_status launch_deriv(const double* layers, int L, const double* p, int 
   // kr_reflectivity, so R here is bit-identical to the forward kernel's)
   const int table = (stage && ray_table_model(L)) ? 1 : 0;
   const size_t smem = acc + (stage ? pair : 0) + (table ? ray_table_bytes(L, kDerThreads / 32) : 0);
-  s = launch_sweep<MODE>(deriv_minb(), (unsigned)n_blocks, smem, st, L, p, n_p,
+  s = launch_sweep<MODE>(deriv_minb(stage != 0), (unsigned)n_blocks, smem, st, L, p, n_p,
                          reinterpret_cast<const double2*>(omega), n_w, n_wtiles,
                          (flags & KR_FREE_SURFACE) ? 1 : 0, seg, stage, table, w.lay, w.dlay, w.coef,
                          w.tan, reinterpret_cast<const double2*>(R_obs),
