@@ -23,13 +23,14 @@ namespace kr {
 // cancels.  With direct exps the water layer's alpha and h gradients of 5- to 31-layer models on 4
 // to 63 slownesses had errors of up to 1.3e-12 of the largest entry, instead of 3e-14.
 //
-// Models of up to kRayTabLayers layers tabulate: a 48-layer block of the batched gradient is
-// 107 KB, two per SM; from 52 layers the table would cost a resident block.  Deeper models that the
+// Models of up to kRayTabLayers layers tabulate: a 51-layer block of the batched gradient is
+// 113 KB (110.4 KB and static arrays), two per SM; from 52 layers the table would cost a resident
+// block.  Deeper models that the
 // forward sweep tabulates (to kPairLayers) evaluate exponentials with the same rounding of the
 // tile's first phase (PhaseLine); beyond, both sides take exp of omega c directly.  Every derivative
 // kernel applies the same rules, so they agree bit for bit.
 // ------------------------------------------------------------------------------------------
-constexpr int kRayTabLayers = 48;
+constexpr int kRayTabLayers = 51;
 __host__ __device__ inline bool ray_table_model(int n_layers) { return n_layers <= kRayTabLayers; }
 
 struct RayTable {

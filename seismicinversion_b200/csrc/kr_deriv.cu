@@ -433,7 +433,7 @@ static size_t sum_kernel_smem(int L, int table) {
   return smem <= kStageSmemMax ? smem : 0;
 }
 
-// Blocks of deriv_sum_kernel that an SM holds (4 up to 23 layers, 3 up to 31, 2 up to 48 with the
+// Blocks of deriv_sum_kernel that an SM holds (4 up to 23 layers, 3 up to 31, 2 up to 51 with the
 // table; 128 registers allow no more than 4).
 static int sum_kernel_blocks(size_t smem) {
   const int n = (int)((227 * 1024) / (smem + 1024 + 64));
