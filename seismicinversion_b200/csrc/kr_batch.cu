@@ -218,12 +218,11 @@ __device__ __forceinline__ void forward_item(const ItemRec& item, const kr_model
   const int u0 = item.w0 / kPhTile, n_tiles = (item.w0 + item.nw - 1) / kPhTile - u0 + 1;
   copy16(lay, v.lay, sizeof(LayerP) * L);
   copy16(coef, v.coef, sizeof(Iface) * I);
-  if (NPH > 0) sweep_tiles_clear(tiles, n_tiles);
-  __syncthreads();
+  const GridLine g = grid_line(om, d.n_w);
+  bool on = NPH > 0 && sweep_tiles_check(om, d.n_w, g, u0, n_tiles, tiles);
+  on = __syncthreads_or(on) != 0;
   bool bad = false;
-  if (NPH > 0) {
-    const GridLine g = grid_line(om, d.n_w);
-    sweep_tiles_check(om, d.n_w, g, u0, n_tiles, tiles);
+  if (NPH > 0 && on) {
     // an item within one tile needs only the mid entries of its own frequencies
     const int m0 = n_tiles > 1 ? 0 : (item.w0 % kPhTile) / kPhLo;
     const int m1 = n_tiles > 1 ? kPhMid : ((item.w0 + item.nw - 1) % kPhTile) / kPhLo + 1;
@@ -325,21 +324,17 @@ struct BatchGradSink {
   for (int kb = (item.w0 & ~31) + (int)(threadIdx.x & ~31u); kb < item.w0 + item.nw; kb += THREADS)
 
 // The tile verdicts and (models that tabulate) lo entries of a gradient item; returns whether its
-// tiles on the line take the table, or PhaseLine.  Contains block barriers; all threads call it.
+// tiles on the line take the table, or PhaseLine.  `lay` may still be on its way from other threads:
+// contains block barriers; all threads call it.
 __device__ __forceinline__ bool ray_item_tables(const ItemRec& item, const kr_model_desc& d,
                                                 const double2* om, const LayerP* lay, cd* lo,
                                                 SweepTiles& tiles) {
-  const bool line = ray_line_model(d.n_layers);
   const int u0 = item.w0 / kPhTile, n = (item.w0 + item.nw - 1) / kPhTile - u0 + 1;
-  if (line) sweep_tiles_clear(tiles, n);
-  __syncthreads();
-  bool ok = line;
-  if (line) {
-    const GridLine g = grid_line(om, d.n_w);
-    sweep_tiles_check(om, d.n_w, g, u0, n, tiles);
-    if (ray_table_model(d.n_layers)) ok = ray_lo_fill(g, d.n_layers, lay, lo);
-  }
-  return __syncthreads_and(ok) != 0;
+  const GridLine g = grid_line(om, d.n_w);
+  bool on = ray_line_model(d.n_layers) && sweep_tiles_check(om, d.n_w, g, u0, n, tiles);
+  on = __syncthreads_or(on) != 0;
+  if (!on || !ray_table_model(d.n_layers)) return on;
+  return __syncthreads_and(ray_lo_fill(g, d.n_layers, lay, lo)) != 0;
 }
 
 // Gradient items of models whose frequency sums exceed shared memory (more than ~118 layers in
@@ -391,7 +386,6 @@ batch_gradient_kernel(unsigned char* plan, const double2* __restrict__ omega_all
       v.lay = sl;
       v.dlay = sd;
     }
-    __syncthreads();
     const double2* om = omega_all + d.omega_off;
     const bool lo_ok = ray_item_tables(item, d, om, v.lay, lo, s_tiles);
     cd* hm = lo + ray_lo_values(L) + (threadIdx.x >> 5) * ray_hm_values(L);
@@ -478,7 +472,6 @@ batch_grad_sums_kernel(unsigned char* plan, const double2* __restrict__ omega_al
     sums_zero(acc, L, W);
     copy16(sc, v.coef, sizeof(Iface) * I);
     copy16(sl, v.lay, sizeof(LayerP) * L);
-    __syncthreads();
     const double2* om = omega_all + d.omega_off;
     const bool lo_ok = ray_item_tables(item, d, om, sl, lo, s_tiles);
     const int seg = checkpoint_spacing(L - 2 > 0 ? L - 2 : 1);

@@ -35,19 +35,18 @@ sweep_kernel(const double* __restrict__ tab, int L, const double* __restrict__ p
   const int n_ent = NPH * I * kPhHead;  // table entries of one slowness
   cd* s_hm = s_tab + (size_t)G * n_ent;
   if (threadIdx.x == 0) s_bad = 0u;
-  if (NPH > 0) sweep_tiles_clear(s_tiles, t1 - t0);
   for (int e = threadIdx.x; e < 2 * ng * L; e += 32 * W) {
     const int half = e >= ng * L ? 1 : 0, j = e - half * ng * L;
     layer_store(tab, L, j % L, half, p[ip0 + j / L], s_lay + j, s_root + j);
   }
-  __syncthreads();
+  const GridLine line = grid_line(omega, n_w);
+  bool on = NPH > 0 && sweep_tiles_check(omega, n_w, line, t0, t1 - t0, s_tiles);
+  on = __syncthreads_or(on) != 0;
   for (int e = threadIdx.x; e < ng * I; e += 32 * W) {
     const int g = e / I, i = e - g * I;
     Form::store(p[ip0 + g], i, s_lay + g * L, s_root + g * L, s_coef + e);
   }
-  if (NPH > 0) {
-    const GridLine line = grid_line(omega, n_w);
-    sweep_tiles_check(omega, n_w, line, t0, t1 - t0, s_tiles);
+  if (NPH > 0 && on) {
     unsigned bad = 0u;
     for (int e = threadIdx.x; e < ng * I * kPhHead; e += 32 * W) {
       const int gl = e / kPhHead, g = gl / I;

@@ -204,22 +204,30 @@ struct SweepTiles {
   unsigned char off[kSweepTiles]; // 1: the tile leaves the grid's line
 };
 
-// Block-cooperative: starts and verdicts of tiles [u0, u0 + n).  The caller synchronises before
-// (off[] cleared by sweep_tiles_clear) and after.
-__device__ __forceinline__ void sweep_tiles_clear(SweepTiles& t, int n) {
-  for (int e = threadIdx.x; e < n; e += blockDim.x) t.off[e] = 0;
-}
-__device__ __forceinline__ void sweep_tiles_check(const double2* __restrict__ omega, int n_w,
+// Starts and verdicts of tiles [u0, u0 + n), the block's warps taking tiles in turn; returns whether
+// one of this warp's is on the line.  All threads call it; the caller synchronises.  Where no tile of
+// the block is, no table is built.
+__device__ __forceinline__ bool sweep_tiles_check(const double2* __restrict__ omega, int n_w,
                                                   const GridLine& g, int u0, int n,
                                                   SweepTiles& t) {
-  const int k_end = min(n_w, (u0 + n) * kPhTile);
-  for (int k = u0 * kPhTile + threadIdx.x; k < k_end; k += blockDim.x) {
-    const double2 w = omega[k];
-    const double m = (double)k;
-    if (k % kPhTile == 0) t.w0[k / kPhTile - u0] = w;
-    if (!(fabs(w.x - fma(m, g.d.x, g.w0.x)) <= g.tol && fabs(w.y - fma(m, g.d.y, g.w0.y)) <= g.tol))
-      t.off[k / kPhTile - u0] = 1;
+  const int lane = threadIdx.x & 31;
+  bool any = false;
+  for (int v = threadIdx.x >> 5; v < n; v += blockDim.x >> 5) {
+    bool off = false;
+#pragma unroll
+    for (int q = 0; q < kPhTile / 32; ++q) {
+      const int k = (u0 + v) * kPhTile + 32 * q + lane;
+      if (k >= n_w) continue;
+      const double2 w = omega[k];
+      const double m = (double)k;
+      if (q == 0 && lane == 0) t.w0[v] = w;
+      off |= !(fabs(w.x - fma(m, g.d.x, g.w0.x)) <= g.tol && fabs(w.y - fma(m, g.d.y, g.w0.y)) <= g.tol);
+    }
+    off = __any_sync(0xffffffffu, off);
+    if (lane == 0) t.off[v] = off ? 1 : 0;
+    any |= !off;
   }
+  return any;
 }
 
 // One warp: passes [pass0, pass1) of tile u (pass q: the 32 F consecutive frequencies from
