@@ -344,7 +344,10 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
       }
     } else {
       // slownesses off the progression, falling or below zero, a negative or extreme omega r: each
-      // term by itself
+      // term by itself, cos and sin by rotation where the tile is on the progression
+      const bool turn = s_line[t & 1] && regular;
+      double s = 0.0, c = 1.0;
+      if (turn) sincos(x_first, &s, &c);
 #pragma unroll 1
       for (int k = 0; k < m; ++k) {
         const double2 pf = pf_p[k];
@@ -354,9 +357,13 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
         if (x < kJ0X0) {
           jv = x > -kJ0X0 ? j0_table(s_j0, fabs(x)) : j0(x);
         } else {
-          double s, c;
-          sincos(x, &s, &c);
+          if (!turn) sincos(x, &s, &c);
           jv = j0_asymptotic(x, c, s);
+        }
+        if (turn) {
+          const double c2 = fma(c, cdl, -s * sd);
+          s = fma(s, cdl, c * sd);
+          c = c2;
         }
         const double t = jv * pf.y;
         bx = fma(t, rv.x, bx);
