@@ -53,8 +53,8 @@ extern "C" kr_status kr_reflectivity(const double* layers, int32_t n_layers, con
   cudaStream_t st = (cudaStream_t)stream;
   constexpr const char* kWhat = "kr_reflectivity";
   switch (sweep_phases(n_layers)) {
-    case 0:
-      return launch_forward<KennettForm, 0, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
+    case 0:  // eight warps a block: above 246 layers an SM's shared memory holds one block
+      return launch_forward<KennettForm, 0, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
     case 2:
       return launch_forward<KennettForm, 2, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
     default:

@@ -169,7 +169,7 @@ extern "C" kr_status kr_gmm_reflectivity(const double* layers, int32_t n_layers,
   constexpr const char* kWhat = "kr_gmm_reflectivity";
   switch (sweep_phases(n_layers)) {
     case 0:
-      return launch_forward<GmmForm, 0, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
+      return launch_forward<GmmForm, 0, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
                                                  R, st);
     case 2:
       return launch_forward<GmmForm, 2, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
