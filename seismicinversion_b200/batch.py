@@ -220,11 +220,22 @@ class ModelBatch:
         self.graph = None
         self.schedule = None
         self.plan = None
-        # short grids leave a wide block's warps without frequencies: 12 x 64 of 4096 5-layer
-        # models take 361 us with one warp per item, 401 with two and 530 with four; of 1500
-        # 12-layer models (12 x 50) 395, 321 and 392, their table being larger than their sweep
-        few = 128 if len(w) > 256 else 64 if L > 8 or len(w) > 128 else 32
-        self.set_schedule(schedule or (few, 128))
+        # Short grids leave a wide block's warps without frequencies, deep models make a narrow
+        # block's table larger than its sweep, and an item of one tile pays the prologue for 128
+        # frequencies.  Microseconds with 32 / 64 / 128 threads: 4000 x 12 x 64 of 8 layers
+        # 466 / 509 / 706, of 12 layers 871 / 730 / 922, of 30 layers - / 2379 / 2475; 500 x 12 x 160
+        # of 5 layers 77 / 91 / 124, of 12 layers 195 / 187 / 194; 500 x 12 x 100 of 20 layers
+        # - / 261 / 237, of 48 layers - / 769 / 662; 200 x 12 x 512 of 5 layers - / 77 / 81, of 30
+        # layers - / - / 435.  Items of 128 frequencies instead of 512: 20 x 32 x 2047 of 3 layers
+        # 89 instead of 52, of 30 layers 538 instead of 443.  Fewer than 16 items per SM are a matter of
+        # one item's latency: 50 x 16 x 1024 of 12 layers 163 with 64 threads, 120 with 128.
+        if L <= 8 and len(w) <= 192:
+            few = 32
+        elif len(w) > 192 and n * len(p) * -(-len(w) // 512) < 148 * 16:
+            few = 128
+        else:
+            few = 64 if L <= 12 or len(w) <= 64 else 128
+        self.set_schedule(schedule or (few, 512))
         return self
 
     # -- planning ------------------------------------------------------------------------
