@@ -204,11 +204,6 @@ KR_HD void set_zero(cd& x) { x = mk(0.0, 0.0); }
 KR_HD void set_zero(double& x) { x = 0.0; }
 KR_HD void acc_zero(Acc& z) { z.a = z.b = z.r = z.h = mk(0.0, 0.0); }
 KR_HD void acc_zero(AccR& z) { z.a = z.b = z.r = z.h = 0.0; }
-KR_HD Acc acc_zero() {
-  Acc z;
-  acc_zero(z);
-  return z;
-}
 // s += x y (complex), or s += Re(x y) (real: 2 FP64 operations instead of 4)
 KR_HD void acc_add(cd& s, cd x, cd y) { s = cmac(s, x, y); }
 KR_HD void acc_add(double& s, cd x, cd y) { s = fma(x.x, y.x, fma(-x.y, y.y, s)); }

@@ -547,8 +547,7 @@ static kr_status launch_deriv(const double* layers, int L, const double* p, int 
   const size_t acc = GRAD ? sizeof(double) * (((size_t)(kDerThreads / 32) * (4 * L + 1) + 1) / 2 * 2) : 0;
   const size_t pair = pair_smem_bytes(L);
   const int stage = (acc + pair <= kStageSmemMax) ? 1 : 0;
-  // phase table of the block's tile after the staged slowness data (models that tabulate in
-  // kr_reflectivity, so R here is bit-identical to the forward kernel's)
+  // phase table of the block's tile after the staged slowness data
   const int table = (stage && ray_table_model(L)) ? 1 : 0;
   const size_t smem = acc + (stage ? pair : 0) + (table ? ray_table_bytes(L, kDerThreads / 32) : 0);
   s = launch_sweep<MODE>(deriv_minb(stage != 0), (unsigned)n_blocks, smem, st, L, p, n_p,

@@ -53,7 +53,6 @@ KR_HD cd cdot2(cd a, cd b, cd c, cd d) {
   return mk(fma(a.x, b.x, fma(-a.y, b.y, fma(c.x, d.x, -(c.y * d.y)))),
             fma(a.x, b.y, fma(a.y, b.x, fma(c.x, d.y, c.y * d.x))));
 }
-KR_HD cd cmac2(cd s, cd a, cd b, cd c, cd d) { return cmac(cmac(s, c, d), a, b); }
 KR_HD double abs2(cd a) { return fma(a.x, a.x, a.y * a.y); }
 
 // 1/z via the conjugate over |z|^2, with a prescale by 1e-150 or 1e150 so that |z|^2 neither
@@ -103,8 +102,7 @@ KR_HD cd csqrt(cd z) {
 // csqrt of any magnitude, scaled by a power of four near the ends of the range: of a subnormal,
 // csqrt's half sum may round to zero and leave y / (2 t) infinite; of a value near the largest it
 // may overflow.  For what data decide: the adjoint of an evanescent water phase underflows
-// gradually.  (Apart from csqrt, whose chain is the latency of every prologue: scaled there too,
-// the 64 x 1024 gradient of 21 layers takes 75.8 us instead of 75.0.)
+// gradually.
 KR_HD cd csqrt_any(cd z) {
   const double m = fmax(fabs(z.x), fabs(z.y));
   double s = 1.0, back = 1.0;

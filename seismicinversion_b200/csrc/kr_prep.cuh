@@ -13,7 +13,7 @@ namespace kr {
 // coefficients and the workspace copy of its upper layer (and of the half-space, for the last
 // interface), so no lane of a warp waits on another's extra work.  The coefficients read the
 // layer terms back from shared memory after a barrier, as the forward kernel's prologue
-// does, so they round exactly as there (R bit-identical across entry points).  Blocks of 128 threads:
+// does, so they round exactly as there.  Blocks of 128 threads:
 // with 64, twice as many SMs are busy with 250 registers a thread while the frequency-sum sweep
 // runs beside this kernel (64 x 32 gradient 65 us against 56), and kernels that wait for it gain
 // nothing (64 x 1024 Jacobian 106.4 against 106.2).

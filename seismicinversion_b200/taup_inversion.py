@@ -105,13 +105,6 @@ class _Problem:
     _STENCILS = {2: ((1, -1), (0.5, -0.5)),
                  4: ((2, 1, -1, -2), (-1.0 / 12, 8.0 / 12, -8.0 / 12, 1.0 / 12))}
 
-    def basis(self) -> torch.Tensor:
-        """Unit directions of the packed parameters in the full [4L] parameter space."""
-        P = len(self.idx)
-        V = torch.zeros((P, 4 * self.L), dtype=_FDTYPE, device=self.dev)
-        V[torch.arange(P), torch.as_tensor(self.idx)] = 1.0
-        return V
-
     def hessian_exact(self, phys: np.ndarray) -> np.ndarray:
         """The exact Hessian over the packed parameters (kr_misfit_hessian; by directions where
         that has no value, as for frequencies with a negative real or imaginary part)."""
