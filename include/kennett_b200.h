@@ -109,7 +109,7 @@ size_t kr_jacobian_workspace_bytes(int32_t n_layers, int32_t n_p, int32_t n_w);
  * tape of up to 64 steps (deeper models checkpoint and recompute segments); interface-
  * coefficient tangents by forward-mode dual numbers once per (p, interface).
  *   layers, p, omega, flags : as kr_reflectivity
- *   R : device complex [n_p][n_w] output, or NULL
+ *   R : device complex [n_p][n_w] output, or NULL (kr_reflectivity's to rounding)
  *   J : device complex [n_p][4*n_layers][n_w] output, J[j][k*L + l][w] = dR(p_j, w)/d theta,
  *       theta = alpha_l (k=0), beta_l (1), rho_l (2), h_l (3).  Derivatives through the
  *       ocean's S quantities, layers with beta = 0 and the half-space phase are zero.

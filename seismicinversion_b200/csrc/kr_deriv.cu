@@ -4,9 +4,9 @@
 // Kernels (stream-ordered, no host synchronisation):
 //   deriv_prep_kernel  : per (p, interface, tangent column or coefficients): layer terms and
 //                        derivative factors, interface coefficients and their 10 x 6 tangents
-//                        -> workspace (kr_prep.cuh).  The frequency-sum sweep forms its own
-//                        coefficients, is launched as this kernel's programmatic dependent and
-//                        waits for it only before its contraction
+//                        -> workspace (kr_prep.cuh).  The frequency-sum sweep is launched as
+//                        this kernel's programmatic dependent; on small grids it forms its own
+//                        coefficients and waits only before its contraction
 //   deriv_sum_kernel   : GRAD / VJP, per (omega, p): forward sweep with a tape of up to 64
 //                        steps (deeper models checkpoint and recompute segments), seed
 //                        2 conj(R - R_obs) (GRAD) or conj(gR) (VJP), reverse sweep; the per-step

@@ -7,10 +7,16 @@
 //     exp(omega_k c) = (hi[u] * mid[t / 16]) * lo[t % 16],
 //     lo[j] = exp(j delta c) (j < 16),  mid[m] = exp(16 m delta c) (m < 8),
 //     hi[u] = exp(omega_{128 u} c)       (the tile's own first frequency)
-// in the forward kernels (kr_sweep.cuh); the derivative kernels (kr_adjsum.cuh) keep hi mid as
-// one entry of the same rounding.  Each entry is one direct exp of an exactly formed argument,
-// and a product of table reads replaces an exp and a sincos per layer, phase and frequency.  A tile whose frequencies leave the line, or whose entries exceed 1e100 in
-// magnitude (so that no product can overflow), evaluates its phases directly.
+// in the forward kernels (kr_sweep.cuh: as squares and products of a layer's two where it tabulates
+// three phases); the derivative kernels (kr_adjsum.cuh) keep hi mid as one entry of the same
+// rounding.  Each exponential is one direct exp of an exactly formed argument, and a product of
+// table reads replaces an exp and a sincos per layer, phase and frequency.  A tile whose frequencies
+// leave the line, or whose entries exceed 1e100 in magnitude (so that no product can overflow),
+// evaluates its phases directly.
+//
+// R of kr_reflectivity and of the batch's forward items is the same bit for bit, and so is R of all
+// derivative kernels; between the two families it agrees to rounding
+// (tests/test_adjoint_from_forward_gpu.py bounds what that does to a gradient).
 #pragma once
 
 #include "kr_internal.cuh"
