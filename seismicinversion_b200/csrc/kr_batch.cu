@@ -126,7 +126,7 @@ batch_prep_kernel(unsigned char* plan, const double* __restrict__ layers,
       layer_store(tab, L, l, half, pj, lay + l, roots + l);
     }
     if (gs > 32) __syncthreads(); else __syncwarp();
-    for (int i = t0; i < I; i += gs) interface_store(pj, i, lay, roots, coef + i);
+    for (int i = t0; i < I; i += gs) interface_store(pj, i, lay, roots + i, roots + i + 1, coef + i);
     if (grad)
       for (int l = t0; l < L; l += gs) dlay[l] = layer_derivs(tab, L, l, pj, lay[l]);
     if (gs > 32) __syncthreads(); else __syncwarp();  // the roots are read before the next pair's

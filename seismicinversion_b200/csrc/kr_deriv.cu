@@ -303,7 +303,7 @@ deriv_sum_kernel(const double* __restrict__ tab6, int L, const double* __restric
     }
     __syncthreads();
     for (int i = threadIdx.x; i < I; i += kDerThreads)
-      interface_store(pj, i, s_lay, s_root, s_if + i);
+      interface_store(pj, i, s_lay, s_root + i, s_root + i + 1, s_if + i);
   } else {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     copy16(s_lay, lay_all + (size_t)ip * L, sizeof(LayerP) * L);

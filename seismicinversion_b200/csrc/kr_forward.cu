@@ -52,20 +52,14 @@ extern "C" kr_status kr_reflectivity(const double* layers, int32_t n_layers, con
   if (!aligned16(omega) || !aligned16(R)) return KR_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   constexpr const char* kWhat = "kr_reflectivity";
-  switch (sweep_phases(n_layers)) {
-    case 0:  // eight warps a block: above 246 layers an SM's shared memory holds one block (64 x 1024
-             // of 256 layers 604 us with four warps, 410 with eight)
-      return launch_forward<KennettForm, 0, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
-    case 2:
-      return launch_forward<KennettForm, 2, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
+  if (n_layers > kPqsLayers)
+    return launch_forward_deep<KennettForm>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
+  switch (forward_minb()) {
+    case 6:
+      return launch_forward<KennettForm, 3, 1, 4, 6>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
+    case 5:
+      return launch_forward<KennettForm, 3, 1, 4, 5>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
     default:
-      switch (forward_minb()) {
-        case 6:
-          return launch_forward<KennettForm, 3, 1, 4, 6>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
-        case 5:
-          return launch_forward<KennettForm, 3, 1, 4, 5>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
-        default:
-          return launch_forward<KennettForm, 3, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
-      }
+      return launch_forward<KennettForm, 3, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
   }
 }

@@ -83,7 +83,7 @@ __device__ __forceinline__ void div22(const cd a[4], const cd b[4], cd y[4]) {
 struct GmmForm {
   typedef GmmCoef Coef;
   static __device__ __forceinline__ void store(double p, int i, const LayerP* lay,
-                                               const LayerRoots*, Coef* out) {
+                                               const LayerRoots*, const LayerRoots*, Coef* out) {
     gmm_store(p, i, lay, out);
   }
   template <int F, class Ph>
@@ -167,15 +167,8 @@ extern "C" kr_status kr_gmm_reflectivity(const double* layers, int32_t n_layers,
   if (!aligned16(omega) || !aligned16(R)) return KR_ERR_INVALID_ARGUMENT;
   cudaStream_t st = (cudaStream_t)stream;
   constexpr const char* kWhat = "kr_gmm_reflectivity";
-  switch (sweep_phases(n_layers)) {
-    case 0:
-      return launch_forward<GmmForm, 0, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
-                                                 R, st);
-    case 2:
-      return launch_forward<GmmForm, 2, 1, 8, 2>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
-                                                 R, st);
-    default:
-      return launch_forward<GmmForm, 3, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags,
-                                                 R, st);
-  }
+  if (n_layers > kPqsLayers)
+    return launch_forward_deep<GmmForm>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R, st);
+  return launch_forward<GmmForm, 3, 1, 4, 4>(kWhat, layers, n_layers, p, n_p, omega, n_w, flags, R,
+                                             st);
 }

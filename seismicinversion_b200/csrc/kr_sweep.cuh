@@ -24,7 +24,7 @@
 namespace kr {
 
 // Phases per layer of a tabulating model: 3 (P, Q, S) up to kPqsLayers layers, where a block of
-// four warps (56 KB at 30 layers) fits four times on an SM; 2 (ea, eb) up to kPairLayers, where
+// four warps (58 KB at 30 layers, 50 KB for one with a pass) fits three or four times on an SM; 2 (ea, eb) up to kPairLayers, where
 // a block of eight warps (113 KB at 66) fits twice: 193 x 1501 of a 64-layer model takes 253 us
 // against 348 with direct exponentials; 0 beyond.  Every forward kernel applies this rule to
 // the model, so a model's phases round alike everywhere.
@@ -33,16 +33,20 @@ constexpr int kPairLayers = 66;
 __host__ __device__ inline int sweep_phases(int n_layers) {
   return n_layers <= kPqsLayers ? 3 : n_layers <= kPairLayers ? 2 : 0;
 }
+// The same two phases' values without a table: the lanes of a warp form its entries step by step
+// (SweepLanes).
+constexpr int kLanePhases = 1;
 
 // Shared memory of one slowness (layer terms and roots, interface coefficients, lo / mid
 // entries) and of
-// one warp (its hm products) for NPH phases per layer and F frequencies per lane.
+// one warp (its hm products) for NPH phases per layer and F frequencies per lane.  Without a table
+// the roots lie where the coefficients come to lie, but for the last layer's.
 __host__ __device__ inline size_t sweep_slowness_bytes(int n_layers, int nph) {
-  return prologue_smem_bytes(n_layers) + sizeof(LayerRoots) * n_layers +
-         sizeof(cd) * kPhHead * nph * (size_t)(n_layers - 1);
+  return prologue_smem_bytes(n_layers) + sizeof(LayerRoots) * (nph > 1 ? n_layers : 1) +
+         (nph > 1 ? sizeof(cd) * kPhHead * nph * (size_t)(n_layers - 1) : 0);
 }
 __host__ __device__ inline size_t sweep_warp_bytes(int n_layers, int nph, int F) {
-  return sizeof(cd) * 2 * F * nph * (size_t)(n_layers - 1);
+  return sizeof(cd) * 2 * F * (nph == kLanePhases ? 2 : nph) * (size_t)(n_layers - 1);
 }
 
 // Exponent `id` (2 l + k) of a model: i eta h of layer l, or i neta h.
@@ -85,8 +89,9 @@ static __device__ __noinline__ void layer_store(const double* tab, int L, int l,
   }
 }
 static __device__ __noinline__ void interface_store(double p, int i, const LayerP* lay,
-                                                    const LayerRoots* roots, Iface* out) {
-  *out = interface_coeffs(p, i, lay[i], lay[i + 1], roots[i], roots[i + 1]);
+                                                    const LayerRoots* up, const LayerRoots* lo,
+                                                    Iface* out) {
+  *out = interface_coeffs(p, i, lay[i], lay[i + 1], *up, *lo);
 }
 
 // Phase factors of F frequencies of one lane from the table.
@@ -137,13 +142,52 @@ struct SweepDirect {
   }
 };
 
+// Phase factors ea, eb of the table, bit for bit, without its lo entries in memory: lane 16 q + j forms
+// entry j of phase q (P, S) of the layer at hand, and shuffles hand the entries round.  One exponential
+// a lane and step (SweepDirect: two), and of shared memory only the warp's hm products: where a
+// slowness has few passes, its table (three times the rest of its data) would keep other slownesses
+// off the SM (forward_plan).
+struct SweepLanes {
+  cd zlo;        // the lane's lo entry's exponent over c
+  const cd* hm;  // the lane's first hm product of phase 0
+  const LayerP* lay;
+  static __device__ __forceinline__ cd from(cd v, int lane) {
+    return mk(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane));
+  }
+  __device__ __forceinline__ SweepLanes(cd d, const cd* h, const LayerP* l)
+      : zlo((double)(threadIdx.x & 15) * d), hm(h), lay(l) {}
+  __device__ __forceinline__ void pqs(int l, cd P[1], cd Q[1], cd S[1]) const {
+    const int lane = threadIdx.x & 31;
+    const cd lo = cexp_(zlo * ((lane & 16) ? lay[l].cb : lay[l].ca));
+    const cd u = hm[4 * l] * from(lo, lane & 15), v = hm[4 * l + 2] * from(lo, 16 + (lane & 15));
+    P[0] = u * u;
+    Q[0] = v * v;
+    S[0] = u * v;
+  }
+  __device__ __forceinline__ void ocean(cd E[1]) const {
+    const cd u = hm[0] * cexp_(zlo * lay[0].ca);
+    E[0] = u * u;
+  }
+};
+
+// Whether all lo and mid entries of a phase are usable: the exponentials themselves only where their
+// size is not plain (below e^200, 1e87).
+__device__ __forceinline__ bool phase_table_usable(const GridLine& g, cd c) {
+  if ((double)((kPhMid - 1) * kPhLo) * (g.d * c).x <= 200.0) return true;
+  bool ok = true;
+  for (int j = 0; j < kPhHead; ++j)
+    ok &= phase_usable(cexp_(((double)(j < kPhLo ? j : (j - kPhLo) * kPhLo) * g.d) * c));
+  return ok;
+}
+
 // The Kennett recursion as a form of the sweep: its interface coefficients, formed once per
 // (slowness, interface), and the upward sweep of F frequencies, giving R at the surface.
 struct KennettForm {
   typedef Iface Coef;
   static __device__ __forceinline__ void store(double p, int i, const LayerP* lay,
-                                               const LayerRoots* roots, Coef* out) {
-    interface_store(p, i, lay, roots, out);
+                                               const LayerRoots* up, const LayerRoots* lo,
+                                               Coef* out) {
+    interface_store(p, i, lay, up, lo, out);
   }
   template <int F, class Ph>
   static __device__ __forceinline__ void sweep(int n_layers, const Coef* coef, const Ph& ph,
@@ -188,6 +232,13 @@ __device__ __noinline__ SweepOut<F> sweep_table(int n_layers, const typename For
   SweepOut<F> o;
   Form::template sweep<F>(n_layers, coef, SweepTable<NPH, F>{lo, hm}, fs, o.R);
   return o;
+}
+template <class Form>
+__device__ __noinline__ cd sweep_lanes(int n_layers, const typename Form::Coef* coef, cd d,
+                                       const cd* hm, const LayerP* lay, bool fs) {
+  cd R[1];
+  Form::template sweep<1>(n_layers, coef, SweepLanes(d, hm, lay), fs, R);
+  return R[0];
 }
 template <class Form>
 __device__ __noinline__ cd sweep_direct(int n_layers, const typename Form::Coef* coef,
@@ -306,6 +357,54 @@ __device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, do
       const cd R = sweep_direct<Form>(n_layers, coef, lay, mk(wv.x, wv.y), fs);
       Rp[k] = make_double2(R.x, R.y);
     }
+  }
+}
+
+// The same for phases formed by the lanes: passes [pass0, pass1) of 32 frequencies; hm: the warp's
+// scratch.
+template <class Form>
+__device__ __forceinline__ void sweep_tile_lanes(const double2* __restrict__ omega, const GridLine& g,
+                                                 double2 w0, int u, int pass0, int pass1, int n_w,
+                                                 int n_layers, const LayerP* lay,
+                                                 const typename Form::Coef* coef, bool use, cd* hm,
+                                                 bool fs, double2* __restrict__ Rp) {
+  const int lane = threadIdx.x & 31;
+  constexpr int kHi = (2 * (kPairLayers - 1) + 31) / 32;
+  const int n_exp = 2 * (n_layers - 1);
+  cd hi[kHi];
+  if (use) {
+    bool ok = true;
+#pragma unroll
+    for (int r = 0; r < kHi; ++r) {
+      const int id = 32 * r + lane;
+      if (id >= n_exp) break;
+      hi[r] = cexp_(mk(w0.x, w0.y) * sweep_exponent(lay, id));
+      ok &= phase_usable(hi[r]);
+    }
+    use = __all_sync(0xffffffffu, ok);
+  }
+  for (int pass = pass0; pass < pass1; ++pass) {
+    const int k = u * kPhTile + pass * 32 + lane;
+    if (k - lane >= n_w) break;
+    cd R;
+    if (use) {
+#pragma unroll
+      for (int r = 0; r < kHi; ++r) {
+        const int id = 32 * r + lane;
+        if (id >= n_exp) break;
+        const cd c = sweep_exponent(lay, id);
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+          hm[2 * id + m] = hi[r] * cexp_(((double)((2 * pass + m) * kPhLo) * g.d) * c);
+      }
+      __syncwarp();
+      R = sweep_lanes<Form>(n_layers, coef, g.d, hm + (lane >> 4), lay, fs);
+      __syncwarp();  // hm is read before the next pass overwrites it
+    } else if (k < n_w) {
+      const double2 wv = omega[k];
+      R = sweep_direct<Form>(n_layers, coef, lay, mk(wv.x, wv.y), fs);
+    }
+    if (k < n_w) Rp[k] = make_double2(R.x, R.y);
   }
 }
 
