@@ -220,23 +220,39 @@ class ModelBatch:
         self.graph = None
         self.schedule = None
         self.plan = None
-        # Short grids leave a wide block's warps without frequencies, deep models make a narrow
-        # block's table larger than its sweep, and an item of one tile pays the prologue for 128
-        # frequencies.  Microseconds with 32 / 64 / 128 threads: 4000 x 12 x 64 of 8 layers
-        # 466 / 509 / 706, of 12 layers 871 / 730 / 922, of 30 layers - / 2379 / 2475; 500 x 12 x 160
-        # of 5 layers 77 / 91 / 124, of 12 layers 195 / 187 / 194; 500 x 12 x 100 of 20 layers
-        # - / 261 / 237, of 48 layers - / 769 / 662; 200 x 12 x 512 of 5 layers - / 77 / 81, of 30
-        # layers - / - / 435.  Items of 128 frequencies instead of 512: 20 x 32 x 2047 of 3 layers
-        # 89 instead of 52, of 30 layers 538 instead of 443.  Fewer than 16 items per SM are a matter of
-        # one item's latency: 50 x 16 x 1024 of 12 layers 163 with 64 threads, 120 with 128.
-        if L <= 8 and len(w) <= 192:
-            few = 32
-        elif len(w) > 192 and n * len(p) * -(-len(w) // 512) < 148 * 16:
-            few = 128
-        else:
-            few = 64 if L <= 12 or len(w) <= 64 else 128
-        self.set_schedule(schedule or (few, 512))
+        self.set_schedule(schedule or self._table_schedule(L, n * len(p), len(w)))
         return self
+
+    @staticmethod
+    def _table_schedule(L: int, pairs: int, nw: int) -> tuple[int, int]:
+        """The default schedule of ``pairs`` (model, slowness) pairs of L layers and nw frequencies.
+
+        Short grids leave a wide block's warps without frequencies, deep models make a narrow block's
+        table larger than its sweep, and an item of one tile pays the prologue for 128 frequencies.
+        Microseconds with 32 / 64 / 128 threads: 4000 x 12 x 64 of 8 layers 460 / 505 / 699, of 12
+        layers 865 / 725 / 918; 300 x 12 x 200 of 5 layers 67 / 68 / 68, of 12 layers 155 / 152 / 143,
+        of 30 layers 615 / 430 / 356.
+
+        With fewer than 16 items of 512 frequencies per SM one item's latency counts: 128 threads, and
+        items as short as it takes to have 8 per SM; one up to 66 layers, whose blocks are two per SM
+        and whose tables cost most; 14 beyond, without tables.  With items of 128 / 256 / 512: 10 x 8
+        x 512 of 21 layers 41 / 56 / 71, of 48 layers 75 / 69 / 108, of 100 layers 165 / 295 / 473;
+        30 x 12 x 1024 of 21 layers 117 / 107 / 150, of 48 layers 293 / 258 / 238, of 100 layers
+        654 / 653 / 1094; 100 x 12 x 160 of 12 layers 62 / 60 / -, and 80 with 64 threads and 512.
+
+        Items of at most 64 frequencies have the deep class form its phases without a table: 500 x 12
+        x 64 of 48 layers 395 with 64 threads, 531 with a table.
+        """
+        def items(tile):
+            return pairs * -(-nw // tile)
+
+        short = 64 if L > 30 and nw <= 64 else None
+        if items(512) < 148 * 16 and not (L <= 4 and nw <= 192):
+            need = 148 * (8 if L <= 30 else 1 if L <= 66 else 14)
+            return 128, short or next((t for t in (512, 256) if items(t) >= need), 128)
+        if L <= 8 and nw <= 192:
+            return 32, 512
+        return 64 if L <= 12 or nw <= 64 else 128, short or 512
 
     # -- planning ------------------------------------------------------------------------
     def _cfg(self, schedule):

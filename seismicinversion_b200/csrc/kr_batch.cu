@@ -201,20 +201,29 @@ struct ItemFeed {
 // Forward items: one (model, slowness) pair and a frequency range [w0, w0 + nw).  The block
 // copies the pair's layer terms and coefficients from the plan, builds its phase table and its
 // warps take the passes of the range in turn (kr_sweep.cuh: the code of kr_reflectivity, so the
-// results are bit-identical to a per-model call).  DEEP selects the class of the work list:
+// results are bit-identical to a per-model call).  CLASS selects the class of the work list:
 // models of up to kPqsLayers layers, whose blocks are small, or deeper ones; each class is one
 // persistent launch with the shared memory and registers of its own models, so that a batch's
-// shallow models do not run at the occupancy of its deepest.
+// shallow models do not run at the occupancy of its deepest.  The deep class has two kernels that give
+// the same bits: with phase tables (98 KB for 66 layers and 128 threads, two blocks per SM) and with
+// phases formed by the lanes (45 KB, four), which direct exponentials beyond 66 layers share.  Items
+// of one or two passes, and batches with models beyond 66 layers, take the second: 500 x 12 x 64 of
+// 48 layers 531 us with tables, 395 without; 64 x 12 x 31 of 80 layers 184 with the tables' two blocks
+// per SM, 144 without; 96 uneven models of up to 64 layers 10.70 ms with tables, 11.32 without.
+enum ForwardClass { kShallow, kDeepTable, kDeepLanes };
+
 template <int NPH, int F, int THREADS>
 __device__ __forceinline__ void forward_item(const ItemRec& item, const kr_model_desc& d, int j,
                                              const PairView& v, const double2* om, double2* Rp,
                                              unsigned char* smem, SweepTiles& tiles) {
-  constexpr int N = NPH > 0 ? NPH : 1;
+  constexpr bool kTable = NPH > 1, kLanes = NPH == kLanePhases;
+  constexpr int N = kTable ? NPH : 2;
   const int L = d.n_layers, I = L - 1;
   LayerP* lay = reinterpret_cast<LayerP*>(smem);
   Iface* coef = reinterpret_cast<Iface*>(lay + L);
   cd* tab = reinterpret_cast<cd*>(coef + I);
-  cd* hm = tab + (size_t)NPH * I * kPhHead + (size_t)(threadIdx.x >> 5) * 2 * F * NPH * I;
+  cd* hm = tab + (kTable ? (size_t)NPH * I * kPhHead : 0) +
+           (size_t)(threadIdx.x >> 5) * 2 * F * (kLanes ? 2 : NPH) * I;
   const int u0 = item.w0 / kPhTile, n_tiles = (item.w0 + item.nw - 1) / kPhTile - u0 + 1;
   copy16(lay, v.lay, sizeof(LayerP) * L);
   copy16(coef, v.coef, sizeof(Iface) * I);
@@ -222,7 +231,9 @@ __device__ __forceinline__ void forward_item(const ItemRec& item, const kr_model
   bool on = NPH > 0 && sweep_tiles_check(om, d.n_w, g, u0, n_tiles, tiles);
   on = __syncthreads_or(on) != 0;
   bool bad = false;
-  if (NPH > 0 && on) {
+  if (kLanes && on)
+    for (int e = threadIdx.x; e < 2 * I; e += THREADS) bad |= !phase_table_usable(g, sweep_exponent(lay, e));
+  if (kTable && on) {
     // an item within one tile needs only the mid entries of its own frequencies
     const int m0 = n_tiles > 1 ? 0 : (item.w0 % kPhTile) / kPhLo;
     const int m1 = n_tiles > 1 ? kPhMid : ((item.w0 + item.nw - 1) % kPhTile) / kPhLo + 1;
@@ -238,19 +249,24 @@ __device__ __forceinline__ void forward_item(const ItemRec& item, const kr_model
   const int passes = n_tiles >= 2 * (THREADS / 32) ? kPasses : 1, parts = kPasses / passes;
   for (int t = threadIdx.x >> 5; t < n_tiles * parts; t += THREADS / 32) {
     const int q = t / parts, pass = (t - q * parts) * passes;
-    sweep_tile<KennettForm, NPH, F>(om, NPH > 0 ? tiles.w0[q] : make_double2(0.0, 0.0), u0 + q, pass,
-                       pass + passes, item.w0, item.w0 + item.nw, L, lay, coef, tab,
-                       NPH > 0 && ok && tiles.off[q] == 0, hm, (d.flags & KR_FREE_SURFACE) != 0,
-                       Rp);
+    const double2 w0 = NPH > 0 ? tiles.w0[q] : make_double2(0.0, 0.0);
+    const bool use = NPH > 0 && ok && tiles.off[q] == 0, fs = (d.flags & KR_FREE_SURFACE) != 0;
+    if (kLanes)
+      sweep_tile_lanes<KennettForm>(om, g, w0, u0 + q, pass, pass + passes, item.w0, item.w0 + item.nw,
+                                    L, lay, coef, use, hm, fs, Rp);
+    else
+      sweep_tile<KennettForm, kTable ? NPH : 0, F>(om, w0, u0 + q, pass, pass + passes, item.w0,
+                                                   item.w0 + item.nw, L, lay, coef, tab, use, hm, fs, Rp);
   }
 }
 
-template <int THREADS, bool DEEP>
-__global__ void __launch_bounds__(THREADS, (DEEP ? 256 : 512) / THREADS)
+template <int THREADS, ForwardClass CLASS>
+__global__ void __launch_bounds__(THREADS, (CLASS == kDeepTable ? 256 : 512) / THREADS)
 batch_forward_kernel(unsigned char* plan, const double2* __restrict__ omega_all,
                      double2* __restrict__ R_all) {
   // the next launch on the stream that allows it may fill in as this one's blocks finish
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  constexpr bool DEEP = CLASS != kShallow;
   extern __shared__ __align__(16) unsigned char s_pair[];
   __shared__ SweepTiles s_tiles;
   PlanHeader* h = reinterpret_cast<PlanHeader*>(plan);
@@ -272,8 +288,10 @@ batch_forward_kernel(unsigned char* plan, const double2* __restrict__ omega_all,
     double2* Rp = R_all + d.R_off + (size_t)pr.j * d.n_w;
     if (!DEEP)
       forward_item<3, 1, THREADS>(item, d, pr.j, v, om, Rp, s_pair, s_tiles);
-    else if (sweep_phases(d.n_layers) == 2)
+    else if (CLASS == kDeepTable)
       forward_item<2, 1, THREADS>(item, d, pr.j, v, om, Rp, s_pair, s_tiles);
+    else if (sweep_phases(d.n_layers) == 2)
+      forward_item<kLanePhases, 1, THREADS>(item, d, pr.j, v, om, Rp, s_pair, s_tiles);
     else
       forward_item<0, 1, THREADS>(item, d, pr.j, v, om, Rp, s_pair, s_tiles);
   }
@@ -592,15 +610,14 @@ static kr_status layout(const kr_model_desc* descs, int n_models, const kr_batch
 
 constexpr size_t kBatchStageMax = 160 * 1024;
 
-// Shared memory of the forward kernel's two classes for models of up to max_layers.
-static size_t fwd_smem(int threads, int max_layers, bool deep) {
-  const int w = threads / 32;
-  if (!deep) {
-    const int L = std::min(max_layers, kPqsLayers);
-    return sweep_slowness_bytes(L, 3) + w * sweep_warp_bytes(L, 3, 1);
+// Shared memory of a class of the forward kernel for models of up to max_layers.
+static size_t fwd_smem(int threads, int max_layers, ForwardClass c) {
+  const int w = threads / 32, L = std::min(max_layers, c == kShallow ? kPqsLayers : kPairLayers);
+  if (c != kDeepLanes) {
+    const int nph = c == kShallow ? 3 : 2;
+    return sweep_slowness_bytes(L, nph) + w * sweep_warp_bytes(L, nph, 1);
   }
-  const int L = std::min(max_layers, kPairLayers);
-  return std::max(sweep_slowness_bytes(L, 2) + w * sweep_warp_bytes(L, 2, 1),
+  return std::max(prologue_smem_bytes(L) + w * sweep_warp_bytes(L, kLanePhases, 1),
                   prologue_smem_bytes(max_layers));
 }
 
@@ -752,11 +769,11 @@ namespace kr {
 
 // One class of the forward items on a resident grid.  `after`: as the programmatic dependent of
 // the launch before it (the tangents, or the deep class).
-template <int THREADS, bool DEEP>
+template <int THREADS, ForwardClass CLASS>
 static kr_status launch_batch_forward(unsigned char* pl, int max_layers, const double2* w,
                                       double2* R, bool after, cudaStream_t st) {
-  const void* fn = (const void*)batch_forward_kernel<THREADS, DEEP>;
-  const size_t smem = fwd_smem(THREADS, max_layers, DEEP);
+  const void* fn = (const void*)batch_forward_kernel<THREADS, CLASS>;
+  const size_t smem = fwd_smem(THREADS, max_layers, CLASS);
   static SmemLimit lim;
   if (smem > 46 * 1024 &&  // with the static arrays above the 48 KB default
       raise_smem_limit(fn, smem, lim, "kr_batch_launch: forward smem") != KR_OK)
@@ -771,7 +788,7 @@ static kr_status launch_batch_forward(unsigned char* pl, int max_layers, const d
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   lc.attrs = attr;
   lc.numAttrs = after ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&lc, batch_forward_kernel<THREADS, DEEP>, pl, w, R);
+  const cudaError_t e = cudaLaunchKernelEx(&lc, batch_forward_kernel<THREADS, CLASS>, pl, w, R);
   if (e != cudaSuccess) {
     set_last_error("kr_batch_launch: forward", e);
     return KR_ERR_CUDA;
@@ -837,7 +854,6 @@ static kr_status launch_batch(unsigned char* pl, const kr_batch_config* cfg, int
                               const double* layers, const double* p, const double* omega,
                               const double* R_obs, double* R, double* chi_grad,
                               cudaStream_t st) {
-  (void)cfg;
   batch_reset_kernel<<<148, 128, 0, st>>>(pl, chi_grad);
   kr_status s = check_launch("kr_batch_launch: reset");
   if (s != KR_OK) return s;
@@ -859,10 +875,12 @@ static kr_status launch_batch(unsigned char* pl, const kr_batch_config* cfg, int
   const double2* obs = reinterpret_cast<const double2*>(R_obs);
   double2* R2 = reinterpret_cast<double2*>(R);
   if (deep) {
-    s = launch_batch_forward<THREADS, true>(pl, max_layers, w, R2, grads, st);
+    const bool lanes = max_layers > kPairLayers || cfg->tile_w <= 64;
+    s = lanes ? launch_batch_forward<THREADS, kDeepLanes>(pl, max_layers, w, R2, grads, st)
+              : launch_batch_forward<THREADS, kDeepTable>(pl, max_layers, w, R2, grads, st);
     if (s != KR_OK) return s;
   }
-  s = launch_batch_forward<THREADS, false>(pl, max_layers, w, R2, grads || deep, st);
+  s = launch_batch_forward<THREADS, kShallow>(pl, max_layers, w, R2, grads || deep, st);
   if (s != KR_OK || !grads) return s;
   if (deep) {
     s = launch_batch_gradient<THREADS, true>(pl, max_layers, w, obs, R2, chi_grad, false, st);

@@ -103,8 +103,8 @@ sweep_kernel(const double* __restrict__ tab, int L, const double* __restrict__ p
     const double2 w0 = NPH > 0 ? s_tiles.w0[v] : make_double2(0.0, 0.0);
     double2* Rp = R + (size_t)(ip0 + g) * n_w;
     if (NPH == kLanePhases)
-      sweep_tile_lanes<Form>(omega, line, w0, t0 + v, pass, pass + passes, n_w, L, s_lay + g * L,
-                             s_coef + g * I, use, hm, free_surface != 0, Rp);
+      sweep_tile_lanes<Form>(omega, line, w0, t0 + v, pass, pass + passes, 0, n_w, L,
+                             s_lay + g * L, s_coef + g * I, use, hm, free_surface != 0, Rp);
     else
       sweep_tile<Form, kTable ? NPH : 0, F>(omega, w0, t0 + v, pass, pass + passes, 0, n_w, L,
                                             s_lay + g * L, s_coef + g * I, s_tab + (size_t)g * n_ent,

@@ -360,12 +360,11 @@ __device__ __forceinline__ void sweep_tile(const double2* __restrict__ omega, do
   }
 }
 
-// The same for phases formed by the lanes: passes [pass0, pass1) of 32 frequencies; hm: the warp's
-// scratch.
+// The same for phases formed by the lanes (passes of 32 frequencies).
 template <class Form>
 __device__ __forceinline__ void sweep_tile_lanes(const double2* __restrict__ omega, const GridLine& g,
-                                                 double2 w0, int u, int pass0, int pass1, int n_w,
-                                                 int n_layers, const LayerP* lay,
+                                                 double2 w0, int u, int pass0, int pass1, int k_lo,
+                                                 int k_hi, int n_layers, const LayerP* lay,
                                                  const typename Form::Coef* coef, bool use, cd* hm,
                                                  bool fs, double2* __restrict__ Rp) {
   const int lane = threadIdx.x & 31;
@@ -384,8 +383,9 @@ __device__ __forceinline__ void sweep_tile_lanes(const double2* __restrict__ ome
     use = __all_sync(0xffffffffu, ok);
   }
   for (int pass = pass0; pass < pass1; ++pass) {
-    const int k = u * kPhTile + pass * 32 + lane;
-    if (k - lane >= n_w) break;
+    const int kb = u * kPhTile + pass * 32, k = kb + lane;
+    if (kb >= k_hi || kb + 32 <= k_lo) continue;
+    const bool valid = k >= k_lo && k < k_hi;
     cd R;
     if (use) {
 #pragma unroll
@@ -400,11 +400,11 @@ __device__ __forceinline__ void sweep_tile_lanes(const double2* __restrict__ ome
       __syncwarp();
       R = sweep_lanes<Form>(n_layers, coef, g.d, hm + (lane >> 4), lay, fs);
       __syncwarp();  // hm is read before the next pass overwrites it
-    } else if (k < n_w) {
+    } else if (valid) {
       const double2 wv = omega[k];
       R = sweep_direct<Form>(n_layers, coef, lay, mk(wv.x, wv.y), fs);
     }
-    if (k < n_w) Rp[k] = make_double2(R.x, R.y);
+    if (valid) Rp[k] = make_double2(R.x, R.y);
   }
 }
 
