@@ -9,7 +9,7 @@
 // 8192 x 2047 grid runs at 12.9e12 (119 FP64 instructions per update, 3.1 ms; the form with
 // two phases per step, a correctly rounded division and a block per slowness took 132 and
 // 3.3 ms).  4096 x 2047 slownesses of a 5-layer model: 389 -> 322 us; 2048 x 511: 137 -> 58 us
-// (several slownesses share a prologue); 193 x 1501 of a 64-layer model: 348 -> 253 us (table
+// (several slownesses share a prologue); 193 x 1501 of a 64-layer model: 351 -> 230 us (table
 // instead of direct exponentials).  Two frequencies per lane (half the coefficient loads, two
 // chains) measured the same on 21 layers and 7 % slower on 5: registers, not loads, bound it.
 #include <stdlib.h>

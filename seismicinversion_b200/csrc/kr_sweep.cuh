@@ -25,8 +25,8 @@ namespace kr {
 
 // Phases per layer of a tabulating model: 3 (P, Q, S) up to kPqsLayers layers, where a block of
 // four warps (58 KB at 30 layers, 50 KB for one with a pass) fits three or four times on an SM; 2 (ea, eb) up to kPairLayers, where
-// a block of eight warps (113 KB at 66) fits twice: 193 x 1501 of a 64-layer model takes 253 us
-// against 348 with direct exponentials; 0 beyond.  Every forward kernel applies this rule to
+// a block of eight warps (113 KB at 66) fits twice: 193 x 1501 of a 64-layer model takes 230 us
+// against 351 with direct exponentials; 0 beyond.  Every forward kernel applies this rule to
 // the model, so a model's phases round alike everywhere.
 constexpr int kPqsLayers = 30;
 constexpr int kPairLayers = 66;
