@@ -233,7 +233,8 @@ class ModelBatch:
         layers 865 / 725 / 918; 300 x 12 x 200 of 5 layers 67 / 68 / 68, of 12 layers 155 / 152 / 143,
         of 30 layers 615 / 430 / 356.
 
-        With fewer than 16 items of 512 frequencies per SM one item's latency counts: 128 threads, and
+        With fewer than 16 items of 512 frequencies per SM one item's latency counts: 128 threads (64 on
+        short grids of 10 and more pairs per SM: 190 x 12 x 50 of 6 layers 49 / 38 / 42), and
         items as short as it takes to have 8 per SM; one up to 66 layers, whose blocks are two per SM
         and whose tables cost most; 14 beyond, without tables.  With items of 128 / 256 / 512: 10 x 8
         x 512 of 21 layers 41 / 56 / 71, of 48 layers 75 / 69 / 108, of 100 layers 165 / 295 / 473;
@@ -247,7 +248,9 @@ class ModelBatch:
             return pairs * -(-nw // tile)
 
         short = 64 if L > 30 and nw <= 64 else None
-        if items(512) < 148 * 16 and not (L <= 4 and nw <= 192):
+        if items(512) < 148 * 16:
+            if nw <= 192 and (L <= 4 or (pairs >= 148 * 10 and (L <= 8 or nw <= 64))):
+                return 64, short or 256
             need = 148 * (8 if L <= 30 else 1 if L <= 66 else 14)
             return 128, short or next((t for t in (512, 256) if items(t) >= need), 128)
         if L <= 8 and nw <= 192:
