@@ -282,18 +282,19 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
     const double2 *pf_p = s_pf[t & 1], *w_p = s_w[t & 1];
     const double* q_p = s_q[t & 1];
     const int m = min(kSub, n - t * kSub);
-    const bool rising = rising_tile(s_line[t & 1] != 0, step, pf_p[0].x, regular);
-    // Fast tile: slownesses in arithmetic progression with x increasing from >= 25 in every
-    // lane, so every term takes the asymptotic branch with the anchor / rotation scheme (no
-    // data-dependent branches in the inner loop).  The number of expansion terms follows
-    // from the warp's smallest argument.
-    const double x_first = (om * pf_p[0].x) * r;
-    const int nt = x_first >= 3000.0 ? 2 : x_first >= 300.0 ? 3 : x_first >= 100.0 ? 4
-                 : x_first >= 60.0 ? 5 : x_first >= kJ0X0 ? 7 : 8;
-    const int terms = __reduce_max_sync(0xffffffffu, rising ? nt : 8);
+    // A falling tile is a rising one from its other end: its least argument is the last one's.
+    const double p_low = pf_p[step > 0.0 ? 0 : m - 1].x, x_low = (om * p_low) * r;
+    const bool steady = rising_tile(s_line[t & 1] != 0, fabs(step), p_low, regular);
+    // Fast tile: slownesses in arithmetic progression with x >= 25 in every lane, so every term
+    // takes the asymptotic branch with the anchor / rotation scheme (no data-dependent branches
+    // in the inner loop).  The number of expansion terms follows from the warp's smallest
+    // argument.
+    const int nt = x_low >= 3000.0 ? 2 : x_low >= 300.0 ? 3 : x_low >= 100.0 ? 4
+                 : x_low >= 60.0 ? 5 : x_low >= kJ0X0 ? 7 : 8;
+    const int terms = __reduce_max_sync(0xffffffffu, steady ? nt : 8);
     if (terms < 8) {
       double s, c;
-      sincos(x_first, &s, &c);
+      sincos((om * pf_p[0].x) * r, &s, &c);
       const TileTurn d = {half_tan * omr, sd * z, cdl, sd * omr};
       const double u = c + s, v = (c - s) * z, z2 = z * z;
       switch (terms) {
@@ -305,7 +306,7 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
       }
       continue;
     }
-    if (rising && __all_sync(0xffffffffu, (om * pf_p[m - 1].x) * r < kJ0X0)) {
+    if (steady && __all_sync(0xffffffffu, (om * pf_p[step > 0.0 ? m - 1 : 0].x) * r < kJ0X0)) {
       // every term from the table
 #pragma unroll 2
       for (int k = 0; k < m; ++k) {
@@ -315,10 +316,10 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
         bx = fma(t, rv.x, bx);
         by = fma(t, rv.y, by);
       }
-    } else if (rising) {
+    } else if (steady) {
       // the tile crosses x = 25
       double s, c;
-      sincos(x_first, &s, &c);
+      sincos((om * pf_p[0].x) * r, &s, &c);
       const double sn = sd * z, s1 = sd * omr, z2 = z * z;
       double u = c + s, v = (c - s) * z;
 #pragma unroll 1
@@ -343,11 +344,9 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
         u = u2;
       }
     } else {
-      // slownesses off the progression, falling or below zero, a negative or extreme omega r: each
-      // term by itself, cos and sin by rotation where the tile is on the progression
-      const bool turn = s_line[t & 1] && regular;
-      double s = 0.0, c = 1.0;
-      if (turn) sincos(x_first, &s, &c);
+      // slownesses off the progression or below zero, a negative or extreme omega r: each term by
+      // itself (a rotation here for falling tiles costs the others registers: 6000 x 1000 x 10 173 us
+      // against 167)
 #pragma unroll 1
       for (int k = 0; k < m; ++k) {
         const double2 pf = pf_p[k];
@@ -357,13 +356,9 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
         if (x < kJ0X0) {
           jv = x > -kJ0X0 ? j0_table(s_j0, fabs(x)) : j0(x);
         } else {
-          if (!turn) sincos(x, &s, &c);
+          double s, c;
+          sincos(x, &s, &c);
           jv = j0_asymptotic(x, c, s);
-        }
-        if (turn) {
-          const double c2 = fma(c, cdl, -s * sd);
-          s = fma(s, cdl, c * sd);
-          c = c2;
         }
         const double t = jv * pf.y;
         bx = fma(t, rv.x, bx);
