@@ -282,15 +282,15 @@ bessel_partial_kernel(const double2* __restrict__ R, const double* __restrict__ 
     const double2 *pf_p = s_pf[t & 1], *w_p = s_w[t & 1];
     const double* q_p = s_q[t & 1];
     const int m = min(kSub, n - t * kSub);
-    // A falling tile is a rising one from its other end: its least argument is the last one's.
-    const double p_low = pf_p[step > 0.0 ? 0 : m - 1].x, x_low = (om * p_low) * r;
-    const bool steady = rising_tile(s_line[t & 1] != 0, fabs(step), p_low, regular);
+    // A falling tile is a rising one from its other end, where its first (least) argument is then.
+    const double p_first = pf_p[step > 0.0 ? 0 : m - 1].x, x_first = (om * p_first) * r;
+    const bool steady = rising_tile(s_line[t & 1] != 0, fabs(step), p_first, regular);
     // Fast tile: slownesses in arithmetic progression with x >= 25 in every lane, so every term
     // takes the asymptotic branch with the anchor / rotation scheme (no data-dependent branches
     // in the inner loop).  The number of expansion terms follows from the warp's smallest
     // argument.
-    const int nt = x_low >= 3000.0 ? 2 : x_low >= 300.0 ? 3 : x_low >= 100.0 ? 4
-                 : x_low >= 60.0 ? 5 : x_low >= kJ0X0 ? 7 : 8;
+    const int nt = x_first >= 3000.0 ? 2 : x_first >= 300.0 ? 3 : x_first >= 100.0 ? 4
+                 : x_first >= 60.0 ? 5 : x_first >= kJ0X0 ? 7 : 8;
     const int terms = __reduce_max_sync(0xffffffffu, steady ? nt : 8);
     if (terms < 8) {
       double s, c;
